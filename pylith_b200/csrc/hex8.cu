@@ -1,0 +1,79 @@
+// Q1 hexahedra, one thread per cell (hex8.cuh): residual, FP64 and FP32 Jacobian action.
+//
+// Bound: FP64 arithmetic, about 1,350 operations per cell (65 % of the FP64 pipe busy at 8 warps per
+// multiprocessor, DRAM 13 %); FP32, instruction issue and latency. One thread per cell takes the
+// whole sweep into registers (254 in FP64), where 8 lanes per cell staged every contraction through
+// shared memory: on the 96x96x72 box (663,552 cells) the FP64 residual went from 293 to 84 us, the
+// FP64 action from 277 to 79 us and the FP32 action from 207 to 55 us. The reductions alone, 16 M
+// on that box, take 58 us in FP64 when each cell adds its own 24 sums and 31 us when consecutive
+// cells hand on their shared face (hex8_scatter). FP32 with 6 blocks of 64 threads per
+// multiprocessor (145 registers, no spills) measured 62 us against 55 us with 8 (128 registers, 36
+// bytes spilled).
+#include <algorithm>
+
+#include "hex8.cuh"
+#include "internal.hpp"
+#include "launch.hpp"
+
+namespace plb {
+
+template <int RHEO, bool BF, int OP, typename T>
+__global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 4) k_hex8(DomainParams p) {
+    hex8_cell<RHEO, BF, OP, T>(p, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+}
+
+template <int RHEO, bool BF, int OP, typename T>
+static void launch_t(const DomainParams& p, cudaStream_t s) {
+    // warps spread over the multiprocessors while there are fewer than two per multiprocessor
+    const int th = p.ncells <= (int64_t)sm_count() * 64 ? 32 : 64;
+    k_hex8<RHEO, BF, OP, T><<<(unsigned)((p.ncells + th - 1) / th), th, 0, s>>>(p);
+    count_launch();
+}
+
+template <int RHEO>
+static void launch_r(const DomainParams& p, bool bf, int op, cudaStream_t s) {
+    if (op != OP_RESIDUAL) launch_t<RHEO, false, OP_JACOBIAN_ACTION, double>(p, s);
+    else if (bf) launch_t<RHEO, true, OP_RESIDUAL, double>(p, s);
+    else launch_t<RHEO, false, OP_RESIDUAL, double>(p, s);
+}
+
+void launch_hex8(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s) {
+    if (rheo == RHEO_ILE) launch_r<RHEO_ILE>(p, bf, op, s);
+    else launch_r<RHEO_GENMAXWELL>(p, bf, op, s);
+}
+
+void launch_hex8_jv32(const DomainParams& p, int rheo, cudaStream_t s) {
+    if (rheo == RHEO_ILE) launch_t<RHEO_ILE, false, OP_JACOBIAN_ACTION, float>(p, s);
+    else launch_t<RHEO_GENMAXWELL, false, OP_JACOBIAN_ACTION, float>(p, s);
+}
+
+// FP32 Jacobian action over the cells of many meshes in one launch (the ragged batch of solvers,
+// ragged.cu): member m's cells form warp chunks chunk0[m] .. chunk0[m + 1] - 1 of one index space
+// (kHex8ChunkCells cells per chunk), so a warp never mixes members; ops[m] holds member m's operator
+// arguments (its own cells, coordinates, cached per-cell tangent, input and output). Members must
+// have the cached isotropic tangent (lm32).
+static_assert(kHex8ChunkCells == 32, "one cell per lane");
+__global__ void __launch_bounds__(64, 8)
+    k_hex8_jv32_ragged(const DomainParams* __restrict__ ops, const int64_t* __restrict__ chunk0,
+                       const int* __restrict__ active, const int* __restrict__ nmembers) {
+    const int M = *nmembers;
+    const int64_t total = chunk0[M];
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < total; w += warps) {
+        int lo = 0, hi = M;  // the member of chunk w: largest m with chunk0[m] <= w
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (chunk0[mid] <= w) lo = mid;
+            else hi = mid;
+        }
+        if (!active[lo]) continue;  // the whole warp shares w
+        hex8_cell<RHEO_ILE, false, OP_JACOBIAN_ACTION, float>(ops[lo], (w - chunk0[lo]) * kHex8ChunkCells + (threadIdx.x & 31));
+    }
+}
+
+void launch_hex8_jv32_ragged(const DomainParams* ops, const int64_t* chunk0, const int* active, const int* nmembers,
+                             cudaStream_t s) {
+    k_hex8_jv32_ragged<<<sm_count() * 8, 64, 0, s>>>(ops, chunk0, active, nmembers);
+}
+
+}  // namespace plb

@@ -1,18 +1,17 @@
-// Hexahedral cells with a group of lanes per cell: the residual and Jacobian action of Q1 (8
-// quadrature points) and Q2 (27 quadrature points) hexahedra.
+// Hexahedral cells with a group of lanes per cell: the residual and Jacobian action of Q2
+// hexahedra (27 quadrature points), and the dispatch of all hexahedral kernels (Q1: hex8.cu).
 //
 // The thread-per-cell kernel (domain.cu) keeps a whole Q2 cell in one thread (81 accumulators,
-// 27 quadrature points in a loop) and spills. Here a group of lanes shares one cell: a full warp
-// for Q2 (27 lanes busy), 8 lanes for Q1 (four cells per warp). Lane q owns quadrature point q:
-// it forms the trilinear geometry, the solution gradient from the cell's node values staged in
-// shared memory, calls the registered pointwise kernel and stages its test-function weights
-// wdetJ f1 J^{-T} (and wdetJ f0). Lane n then owns node n: it contracts the staged weights with
-// the reference basis gradients of node n over all quadrature points and adds the result into
-// the output (FP64 reductions; nodes are shared with neighbouring cells). The reference basis
-// tables (gradients and values at the quadrature points, and the trilinear geometry gradients)
-// are built once per block in shared memory. The FP32 variant (inner iterations of the refined
-// solver) keeps the geometry and the tangent in FP64 and stages the field, the weights and the
-// sums in FP32.
+// 27 quadrature points in a loop) and spills. Here a warp shares one cell (27 lanes busy). Lane q
+// owns quadrature point q: it forms the trilinear geometry, the solution gradient from the cell's
+// node values staged in shared memory, calls the registered pointwise kernel and stages its
+// test-function weights wdetJ f1 J^{-T} (and wdetJ f0). Lane n then owns node n: it contracts the
+// staged weights with the reference basis gradients of node n over all quadrature points and adds
+// the result into the output (FP64 reductions; nodes are shared with neighbouring cells). The
+// reference basis tables (gradients and values at the quadrature points, and the trilinear
+// geometry gradients) are built once per block in shared memory. The FP32 variant (inner
+// iterations of the refined solver) keeps the geometry and the tangent in FP64 and stages the
+// field, the weights and the sums in FP32.
 #include "domain_kernels.cuh"
 #include "internal.hpp"
 #include "launch.hpp"
@@ -53,15 +52,11 @@ PL_D void fill_tables(double* t64, T* tt) {
     for (int i = threadIdx.x; i < H::NQ * H::NEN; i += blockDim.x) {
         const int q = i / H::NEN, n = i % H::NEN;
         double d[3];
-        if (CELL == HEX8) {
-            hex_corner_dN<2>(n, q & 1, (q >> 1) & 1, q >> 2, d);
-        } else {
-            const double x = gauss3_x(q % 3), y = gauss3_x((q / 3) % 3), z = gauss3_x(q / 9);
-            const int a = n % 3, b = (n / 3) % 3, c = n / 9;
-            d[0] = quad_d(a, x) * quad_v(b, y) * quad_v(c, z);
-            d[1] = quad_v(a, x) * quad_d(b, y) * quad_v(c, z);
-            d[2] = quad_v(a, x) * quad_v(b, y) * quad_d(c, z);
-        }
+        const double x = gauss3_x(q % 3), y = gauss3_x((q / 3) % 3), z = gauss3_x(q / 9);
+        const int a = n % 3, b = (n / 3) % 3, c = n / 9;
+        d[0] = quad_d(a, x) * quad_v(b, y) * quad_v(c, z);
+        d[1] = quad_v(a, x) * quad_d(b, y) * quad_v(c, z);
+        d[2] = quad_v(a, x) * quad_v(b, y) * quad_d(c, z);
 #pragma unroll
         for (int k = 0; k < 3; ++k) tt[q * H::LDB + n * 3 + k] = (T)d[k];
         tt[H::T_PHI + q * H::NEN + n] = (T)Elem<CELL>::phi(q, n);
@@ -69,13 +64,12 @@ PL_D void fill_tables(double* t64, T* tt) {
     for (int i = threadIdx.x; i < H::NQ * 8; i += blockDim.x) {
         const int q = i / 8, c = i % 8;
         double d[3];
-        if (CELL == HEX8) hex_corner_dN<2>(c, q & 1, (q >> 1) & 1, q >> 2, d);
-        else hex_corner_dN<3>(c, q % 3, (q / 3) % 3, q / 9, d);
+        hex_corner_dN<3>(c, q % 3, (q / 3) % 3, q / 9, d);
 #pragma unroll
         for (int k = 0; k < 3; ++k) t64[q * 25 + c * 3 + k] = d[k];
     }
     for (int q = threadIdx.x; q < H::NQ; q += blockDim.x)
-        t64[H::T_W + q] = CELL == HEX8 ? 1.0 : gauss3_w(q % 3) * gauss3_w((q / 3) % 3) * gauss3_w(q / 9);
+        t64[H::T_W + q] = gauss3_w(q % 3) * gauss3_w((q / 3) % 3) * gauss3_w(q / 9);
 }
 
 // Per-block tables and per-group staging of the group-of-lanes hexahedral kernels.
@@ -154,23 +148,7 @@ PL_D void hex_group_cells(const DomainParams& p, int64_t base, const HexGroupSme
             const int q = l;
             T inv[3][3];
             T wdetJ;
-            if constexpr (sizeof(T) == 4 && CELL == HEX8) {
-                // FP32 Jacobian action: FP32 geometry from the corners relative to corner 0 (the
-                // basis gradients sum to zero, so J is unchanged and no large coordinates cancel),
-                // with the field-basis gradient table (the Q1 field basis is the geometry basis)
-                float J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-#pragma unroll
-                for (int k = 1; k < 8; ++k)
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) {
-                        const float dx = (float)(sX[k * 3 + i] - sX[i]);
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) J[i][j] += dx * tB[q * H::LDB + k * 3 + j];
-                    }
-                const float detJ = invert3(J, inv);
-                if (!(detJ > 0.f)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
-                wdetJ = (float)tW[q] * detJ;
-            } else {
+            {
                 double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
@@ -294,50 +272,6 @@ __global__ void __launch_bounds__(HexGroup<CELL, T>::WARPS * 32) k_hex_group(Dom
     // every lane of a warp runs the same number of passes (the __syncwarp calls need them all)
     for (int64_t base = ((int64_t)blockIdx.x * H::WARPS + warp) * H::CPW; base < p.ncells; base += cells_per_pass)
         hex_group_cells<CELL, RHEO, BF, OP, T>(p, base, g);
-}
-
-// FP32 Jacobian action of Q1 hexahedra over the cells of many meshes in one launch (the ragged
-// batch of solvers, ragged.cu): member m's cells form warp chunks chunk0[m] .. chunk0[m + 1] - 1
-// of one index space (4 cells per chunk), so a warp never mixes members; ops[m] holds member m's
-// operator arguments (its own cells, coordinates, cached per-cell tangent, input and output).
-// Members must have the cached isotropic tangent (lm32).
-__global__ void __launch_bounds__(HexGroup<HEX8, float>::WARPS * 32)
-    k_hex8_jv32_ragged(const DomainParams* __restrict__ ops, const int64_t* __restrict__ chunk0,
-                       const int* __restrict__ active, const int* __restrict__ nmembers) {
-    using H = HexGroup<HEX8, float>;
-    extern __shared__ __align__(16) double hsm[];
-    fill_tables<HEX8, float>(hsm, reinterpret_cast<float*>(hsm + H::T_END64 + H::GROUPS * H::PER_GROUP_X));
-    __syncthreads();
-    const HexGroupSmem<HEX8, float> g = hex_group_smem<HEX8, float>(hsm);
-    const int M = *nmembers;
-    const int64_t total = chunk0[M];
-    const int warp = threadIdx.x >> 5;
-    for (int64_t w = (int64_t)blockIdx.x * H::WARPS + warp; w < total; w += (int64_t)gridDim.x * H::WARPS) {
-        int lo = 0, hi = M;  // the member of chunk w: largest m with chunk0[m] <= w
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (chunk0[mid] <= w) lo = mid;
-            else hi = mid;
-        }
-        if (!active[lo]) continue;  // the whole warp shares w
-        hex_group_cells<HEX8, RHEO_ILE, false, OP_JACOBIAN_ACTION, float>(ops[lo], (w - chunk0[lo]) * H::CPW, g);
-    }
-}
-
-void launch_hex8_jv32_ragged(const DomainParams* ops, const int64_t* chunk0, const int* active, const int* nmembers,
-                             cudaStream_t s) {
-    using H = HexGroup<HEX8, float>;
-    const size_t smem = H::smem_bytes();
-    static int per_sm = 0, nsm = 0;
-    if (!per_sm) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        ensure_kernel_smem((const void*)k_hex8_jv32_ragged, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hex8_jv32_ragged, H::WARPS * 32, smem);
-        per_sm = std::max(per_sm, 1);
-    }
-    k_hex8_jv32_ragged<<<nsm * per_sm, H::WARPS * 32, smem, s>>>(ops, chunk0, active, nmembers);
 }
 
 // ---- Q2 hexahedra by sum factorisation --------------------------------------------------------
@@ -968,7 +902,7 @@ static void launch_sumfact(const DomainParams& p, int rheo, bool bf, int op, cud
 
 bool launch_domain_apply_hexgroup(const DomainParams& p, int cell, int rheo, bool bf, int op, cudaStream_t s) {
     if (p.ncells == 0) return true;
-    if (cell == HEX8) launch_group_cell<HEX8>(p, rheo, bf, op, s);
+    if (cell == HEX8) launch_hex8(p, rheo, bf, op, s);
     else if (cell == HEX27 && PLB_Q2_LINES) launch_lines(p, rheo, bf, op, s);
     else if (cell == HEX27 && PLB_Q2_SUMFACT) launch_sumfact(p, rheo, bf, op, s);
     else if (cell == HEX27) launch_group_cell<HEX27>(p, rheo, bf, op, s);
@@ -1009,8 +943,7 @@ bool launch_domain_jv32_hexgroup(const DomainParams& p, int cell, int rheo, cuda
     if (p.ncells == 0) return true;
     const bool gm = rheo == RHEO_GENMAXWELL;
     if (cell == HEX8) {
-        if (gm) launch_group_t<HEX8, RHEO_GENMAXWELL, false, OP_JACOBIAN_ACTION, float>(p, s);
-        else launch_group_t<HEX8, RHEO_ILE, false, OP_JACOBIAN_ACTION, float>(p, s);
+        launch_hex8_jv32(p, rheo, s);
     } else if (cell == HEX27) {
         if (gm) launch_group_t<HEX27, RHEO_GENMAXWELL, false, OP_JACOBIAN_ACTION, float>(p, s);
         else launch_group_t<HEX27, RHEO_ILE, false, OP_JACOBIAN_ACTION, float>(p, s);

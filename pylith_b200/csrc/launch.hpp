@@ -31,6 +31,9 @@ void launch_domain_jv_f32_atomic(const DomainParams& p, int cell, int rheo, cuda
 // Hexahedra (Q1, Q2) with a group of lanes per cell (FP64 residual / Jacobian action, FP64
 // reductions into the output); returns false for other cell types.
 bool launch_domain_apply_hexgroup(const DomainParams& p, int cell, int rheo, bool bf, int op, cudaStream_t s);
+// Q1 hexahedra, one thread per cell (hex8.cu).
+void launch_hex8(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
+void launch_hex8_jv32(const DomainParams& p, int rheo, cudaStream_t s);
 // FP32 Jacobian action of hexahedra with a group of lanes per cell (FP64 geometry and tangent).
 bool launch_domain_jv32_hexgroup(const DomainParams& p, int cell, int rheo, cudaStream_t s);
 void launch_domain_jacobian(const DomainParams& p, int cell, int rheo, const int32_t* pos,
@@ -73,6 +76,7 @@ int prepare_jv32_tangent(pl_integrator_s* ig, double t, double dt);
 
 // FP32 Q1 Jacobian action over many members' cells in one launch (the ragged batch; device
 // tables: per-member operator arguments, warp-chunk prefix, active flags, member count).
+constexpr int kHex8ChunkCells = 32;  // cells per warp chunk
 void launch_hex8_jv32_ragged(const DomainParams* ops, const int64_t* chunk0, const int* active, const int* nmembers,
                              cudaStream_t s);
 // Step-by-step FP32 reliable-update PCG of one solver for an outside iteration loop (solver.cu).

@@ -272,7 +272,7 @@ int upload_tables(pl_ragged R) {
         ops[i] = p;
         vec[i] = RgVec{S->f_x, S->f_r, S->f_p, S->f_q, S->f_z, S->d_pinv32, S->d_mask, S->d_pair_neg, S->d_pair_pos,
                        S->nnodes, S->npairs, S->d_scal};
-        cell0[i + 1] = cell0[i] + (ig->ncells + 3) / 4;  // warp chunks of 4 Q1 cells
+        cell0[i + 1] = cell0[i] + (ig->ncells + kHex8ChunkCells - 1) / kHex8ChunkCells;  // warp chunks of Q1 cells
         node0[i + 1] = node0[i] + (S->nnodes + kRgChunk - 1) / kRgChunk;
         pair0[i + 1] = pair0[i] + S->npairs;
         active[i] = mb.active ? 1 : 0;

@@ -582,3 +582,55 @@ def test_reference_compiled_kernels_drive_the_device_path(oracle_lib, torch_cuda
     if_ref.compute_lhs_residual(0.0, 0.0, fu, fr[1])
     ctx.synchronize()
     assert torch.equal(fr[0], fr[1])
+
+
+def _hex8_variant(mesh, order):
+    """The box with jittered nodes, its cells in the given order: 'x' (as built: consecutive cells
+    share a face), 'morton', or 'shuffled' (neighbouring lanes share nothing or single nodes)."""
+    rng = np.random.default_rng(8)
+    h = (mesh.coords.max(axis=0) - mesh.coords.min(axis=0)) / 16
+    mesh.coords += rng.uniform(-0.05, 0.05, mesh.coords.shape) * np.minimum(h, 300.0)
+    if order == "morton":
+        return M.reorder_for_locality(mesh)
+    if order == "shuffled":
+        mesh.cells = np.ascontiguousarray(mesh.cells[rng.permutation(mesh.num_cells)])
+    return mesh
+
+
+# one cell; less than, exactly and one more than a warp; a 64-cell block and a partial one; the
+# first size with 64-cell blocks (more than 148 * 64 cells)
+@pytest.mark.parametrize("n", [(1, 1, 1), (31, 1, 1), (8, 4, 1), (33, 1, 1), (13, 5, 1), (7, 5, 3), (24, 21, 19)])
+@pytest.mark.parametrize("order", ["x", "morton", "shuffled"])
+def test_hex8_cell_kernel_sizes(oracle_lib, torch_cuda, ctx, n, order):
+    """The Q1 kernels against the oracle at warp and block edges, for cell orders with and without
+    faces shared by consecutive cells: residual with body force, action, FP32 action, a cell subset."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh = _hex8_variant(M.box_hex(*n), order)
+    mat = elastic_setup(mesh, seed=6, body_force=True)
+    aux = oracle_aux(O, mat)
+    u = np.random.default_rng(7).standard_normal(mesh.num_nodes * 3)
+    plain = O.AuxFields([aux_field for aux_field in [(mat.density[:, None], "cell"), (mat.shear_modulus[:, None], "cell"),
+                                                     (mat.bulk_modulus[:, None], "cell")]])
+    r_ref = O.residual(mesh, u, aux, f0="Elasticity::g0v_bodyforce", f1=F1_ILE)
+    jv_ref = O.jacobian_action(mesh, u, plain, g3=JF3_ILE)
+    dm = FA.DeviceMesh(ctx, mesh)
+    ig = mat.create_integrator(dm)
+    du = dev(torch, u)
+    dr, djv, d32 = torch.full_like(du, np.nan), torch.full_like(du, np.nan), torch.full_like(du.float(), np.nan)
+    ig.compute_lhs_residual(0.0, 0.0, du, dr)
+    ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, djv)
+    ig.compute_lhs_jacobian_action_f32(0.0, 0.0, du.float(), d32)
+    # every second cell as an integrator of its own, then the others on top
+    parts = [np.arange(s, mesh.num_cells, 2, dtype=np.int32) for s in (0, 1)]
+    dsum = torch.zeros_like(du)
+    for ids in parts:
+        sub = elastic_setup(mesh, seed=6)
+        part = MAT.IsotropicLinearElasticity(sub.density[ids], sub.shear_modulus[ids], sub.bulk_modulus[ids])
+        part.create_integrator(dm, ids).compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, dsum, mode=FA.ADD)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), r_ref) <= TOL64
+    assert rel_l2(djv.cpu().numpy(), jv_ref) <= TOL64
+    assert rel_l2(dsum.cpu().numpy(), jv_ref) <= TOL64
+    assert rel_l2(d32.double().cpu().numpy(), jv_ref) <= 1e-5
