@@ -173,65 +173,6 @@ __global__ void __launch_bounds__(128) k_domain_jv_f32(DomainParams p) {
     }
 }
 
-// Element Jacobians from the pointwise Jf3 (g3) contraction, added into a 3x3-block CSR
-// matrix at precomputed block positions (DMPlexComputeJacobianByKey + MatSetClosure).
-template <int CELL, int RHEO>
-__global__ void __launch_bounds__(128) k_domain_jacobian(DomainParams p, const int32_t* pos,
-                                                         double* vals) {
-    using E = Elem<CELL>;
-    using L = AuxLayout<RHEO, false>;
-    const AuxOffsets<RHEO, false> aoff;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < p.ncells;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t mc = p.cell_ids ? p.cell_ids[c] : c;
-        const int32_t* cn = p.cells + mc * E::nen;
-        double X[E::ngeom][3];
-#pragma unroll
-        for (int k = 0; k < E::ngeom; ++k)
-#pragma unroll
-            for (int i = 0; i < 3; ++i) X[k][i] = p.coords[3 * (int64_t)cn[E::corner(k)] + i];
-        double a[L::size] = {};
-        L::load_cell(p, c, a);
-        const int32_t* cpos = pos + mc * E::nen * E::nen;
-#pragma unroll 1
-        for (int q = 0; q < E::nq; ++q) {
-            Geom g;
-            E::geom(X, q, &g);
-            if (!(g.detJ > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
-            // the tangents (Jf3vu of both rheologies) read no per-point state
-            double x[3] = {0, 0, 0};
-            double Jf3[81];
-#pragma unroll
-            for (int i = 0; i < 81; ++i) Jf3[i] = 0.0;
-            call_jf3<RHEO>(L::numA, aoff.v, a, p, x, Jf3);
-#pragma unroll 1
-            for (int an = 0; an < E::nen; ++an) {
-                double ga[3];
-                E::grad(g, q, an, ga);
-                // t[g][dg] = sum_df ga[df] Jf3[f][g][df][dg], per f
-#pragma unroll 1
-                for (int bn = 0; bn < E::nen; ++bn) {
-                    double gb[3];
-                    E::grad(g, q, bn, gb);
-                    double* blk = vals + 9 * (int64_t)cpos[an * E::nen + bn];
-#pragma unroll
-                    for (int f = 0; f < 3; ++f)
-#pragma unroll
-                        for (int gg = 0; gg < 3; ++gg) {
-                            double v = 0.0;
-#pragma unroll
-                            for (int df = 0; df < 3; ++df)
-#pragma unroll
-                                for (int dg = 0; dg < 3; ++dg)
-                                    v += ga[df] * Jf3[((f * 3 + gg) * 3 + df) * 3 + dg] * gb[dg];
-                            red_add(&blk[f * 3 + gg], g.wdetJ * v);
-                        }
-                }
-            }
-        }
-    }
-}
-
 // DMProjectFieldLocal at quadrature points for the generalized Maxwell state: new viscous
 // strain from the previous viscous and total strain, then the new total strain; both kernels
 // see the previous state (IntegratorDomain.cc:555-590), written back in place.
@@ -388,19 +329,6 @@ void launch_domain_jv_f32_atomic(const DomainParams& p, int cell, int rheo, cuda
     else if (cell == HEX8) { if (rheo == RHEO_ILE) PLB_F32(HEX8, RHEO_ILE); else PLB_F32(HEX8, RHEO_GENMAXWELL); }
     else { if (rheo == RHEO_ILE) PLB_F32(HEX27, RHEO_ILE); else PLB_F32(HEX27, RHEO_GENMAXWELL); }
 #undef PLB_F32
-    count_launch();
-}
-
-void launch_domain_jacobian(const DomainParams& p, int cell, int rheo, const int32_t* pos,
-                            double* vals, cudaStream_t s) {
-    if (p.ncells == 0) return;
-    const int th = 128;
-    const int gr = grid_for(p.ncells, th);
-#define PLB_JAC(C, R) k_domain_jacobian<C, R><<<gr, th, 0, s>>>(p, pos, vals)
-    if (cell == TET4) { if (rheo == RHEO_ILE) PLB_JAC(TET4, RHEO_ILE); else PLB_JAC(TET4, RHEO_GENMAXWELL); }
-    else if (cell == HEX8) { if (rheo == RHEO_ILE) PLB_JAC(HEX8, RHEO_ILE); else PLB_JAC(HEX8, RHEO_GENMAXWELL); }
-    else { if (rheo == RHEO_ILE) PLB_JAC(HEX27, RHEO_ILE); else PLB_JAC(HEX27, RHEO_GENMAXWELL); }
-#undef PLB_JAC
     count_launch();
 }
 

@@ -634,3 +634,53 @@ def test_hex8_cell_kernel_sizes(oracle_lib, torch_cuda, ctx, n, order):
     assert rel_l2(djv.cpu().numpy(), jv_ref) <= TOL64
     assert rel_l2(dsum.cpu().numpy(), jv_ref) <= TOL64
     assert rel_l2(d32.double().cpu().numpy(), jv_ref) <= 1e-5
+
+
+# cells that do not fill a warp's 4 hexahedra or 8 tetrahedra, and rows of 1 to 125 blocks
+ASSEMBLY = {
+    "hex8_1": lambda: M.box_hex(1, 1, 1),
+    "hex8_5": lambda: M.box_hex(5, 1, 1),
+    "hex8_54": lambda: M.box_hex(3, 6, 3),
+    "hex27_1": lambda: M.box_hex27(1, 1, 1),
+    "hex27_12": lambda: M.box_hex27(2, 3, 2),
+    "tet_6": lambda: M.box_tet_kuhn(1, 1, 1),
+    "tet_510": lambda: M.box_tet_kuhn(5, 17, 1),
+}
+
+
+@pytest.mark.parametrize("kind", list(ASSEMBLY))
+@pytest.mark.parametrize("genmaxwell", [False, True])
+def test_assembly_and_product_sizes(oracle_lib, torch_cuda, ctx, kind, genmaxwell):
+    """The assembled Jacobian of two integrators on complementary cell subsets added into one
+    matrix, and its product with a vector, against the oracle's element matrices."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh = ASSEMBLY[kind]()
+    nc, nq = mesh.num_cells, M.QUAD_POINTS[mesh.cell_type]
+    rho, mu, K = MAT.lognormal_elastic(nc, seed=12)
+    ids = [np.arange(0, nc, 3, dtype=np.int32), np.array([c for c in range(nc) if c % 3], dtype=np.int32)]
+    dm = FA.DeviceMesh(ctx, mesh)
+    A = FA.Matrix(dm)
+    if genmaxwell:
+        tau = MAT.genmaxwell_times(rho, np.sqrt(mu / rho), [1e18, 1e19, 1e20], [0.3, 0.2, 0.1])
+        ratio = np.tile([0.3, 0.2, 0.1], (nc, 1))
+        state = [np.zeros((nc, nq, 18)), np.zeros((nc, nq, 6))]
+        aux = O.AuxFields([(a, "cell") for a in (rho[:, None], mu[:, None], K[:, None], tau, ratio)] + [(a, "qp") for a in state])
+        J = O.assemble(mesh, O.jacobian_elements(mesh, aux, g3=JF3_GM, constants=[MAT.YEAR]))
+        for i in ids:
+            MAT.IsotropicLinearGenMaxwell(rho[i], mu[i], K[i], tau[i], ratio[i], state[0][i], state[1][i]).create_integrator(
+                dm, MAT.YEAR, i).compute_lhs_jacobian(0.0, MAT.YEAR, 0.0, None, A)
+    else:
+        aux = O.AuxFields([(a[:, None], "cell") for a in (rho, mu, K)])
+        J = O.assemble(mesh, O.jacobian_elements(mesh, aux, g3=JF3_ILE))
+        for i in ids:
+            MAT.IsotropicLinearElasticity(rho[i], mu[i], K[i]).create_integrator(dm, i).compute_lhs_jacobian(0.0, 0.0, 0.0, None, A)
+    ctx.synchronize()
+    assert abs(A.to_scipy().tocsr() - J).max() <= TOL64 * abs(J).max()
+    x = np.random.default_rng(13).standard_normal(3 * mesh.num_nodes)
+    dx = dev(torch, x)
+    dy = torch.full_like(dx, np.nan)
+    A.spmv(dx, dy)
+    ctx.synchronize()
+    assert rel_l2(dy.cpu().numpy(), J @ x) <= TOL64
