@@ -13,32 +13,39 @@ using namespace plb;
 
 namespace {
 
-// y = A x for 3x3 blocks, one warp per block row.
-__global__ void k_bsr_spmv(int64_t nrows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                           const double* __restrict__ val, const double* __restrict__ x, double* __restrict__ y) {
+// y = A x for 3x3 blocks, one warp per block row. Lanes 0 .. 26 read the 27 consecutive doubles of
+// three blocks at a time, each lane always the same entry (f, g) of its block, so the values
+// stream in whole sectors; a block per lane puts 72 bytes between lanes (L1 pipe 81 % busy against
+// 42 %). The load chain row, column, x is hidden by taking 27 blocks at once (three at a time
+// without unrolling measured 22.7 us against 17.3 on 27,225 rows of a 32x32x24 Q1 box, cold).
+__global__ void __launch_bounds__(256) k_bsr_spmv(int64_t nrows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                                  const double* __restrict__ val, const double* __restrict__ x,
+                                                  double* __restrict__ y) {
     const int lane = threadIdx.x & 31;
+    const int blk = lane / 9, e = lane - 9 * blk, f = e / 3, g = e - 3 * f;  // lanes 27 .. 31 idle
     for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < nrows;
          r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-        for (int k = rp[r] + lane; k < rp[r + 1]; k += 32) {
-            const double* b = val + 9 * (int64_t)k;
-            const int64_t c = ci[k];
-            const double x0 = x[3 * c], x1 = x[3 * c + 1], x2 = x[3 * c + 2];
-            a0 += b[0] * x0 + b[1] * x1 + b[2] * x2;
-            a1 += b[3] * x0 + b[4] * x1 + b[5] * x2;
-            a2 += b[6] * x0 + b[7] * x1 + b[8] * x2;
-        }
+        const int k1 = rp[r + 1];
+        double s = 0.0;
+        for (int k0 = rp[r]; k0 < k1; k0 += 27) {
+            // all loads of 27 blocks (an interior row of Q1 hexahedra) in flight at once
+            int col[9];
+            double v[9];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += __shfl_down_sync(0xffffffffu, a0, o);
-            a1 += __shfl_down_sync(0xffffffffu, a1, o);
-            a2 += __shfl_down_sync(0xffffffffu, a2, o);
+            for (int i = 0; i < 9; ++i) {
+                const int k = k0 + 3 * i + blk;
+                const bool on = lane < 27 && k < k1;
+                col[i] = on ? ci[k] : -1;
+                v[i] = on ? val[9 * (int64_t)k + e] : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 9; ++i)
+                if (col[i] >= 0) s += v[i] * x[3 * (int64_t)col[i] + g];
         }
-        if (lane == 0) {
-            y[3 * r] = a0;
-            y[3 * r + 1] = a1;
-            y[3 * r + 2] = a2;
-        }
+        // rows f: the entries g, then the three blocks
+        s += __shfl_down_sync(0xffffffffu, s, 1) + __shfl_down_sync(0xffffffffu, s, 2);
+        s += __shfl_down_sync(0xffffffffu, s, 9) + __shfl_down_sync(0xffffffffu, s, 18);
+        if (lane < 9 && g == 0) y[3 * r + f] = s;
     }
 }
 
