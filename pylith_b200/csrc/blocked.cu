@@ -155,8 +155,6 @@ PL_D void load_slot_ids(const BlockArrays& A, int64_t b, uint32_t nd[kMaxSlotsPe
 #define PLB_PREFETCH_CELLS 1
 #endif
 
-PL_D void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr)); }
-
 #ifndef PLB_TET_MIN_BLOCKS
 #define PLB_TET_MIN_BLOCKS 4
 #endif

@@ -32,6 +32,8 @@ PL_D float safe_step_f32(double rz, double pq) {
     return isfinite(a) ? a : 0.0f;
 }
 
+PL_D void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr)); }
+
 PL_D void red_add(double* p, double v) { atomicAdd(p, v); }
 PL_D void red_add(float* p, float v) { atomicAdd(p, v); }
 

@@ -584,12 +584,12 @@ def test_reference_compiled_kernels_drive_the_device_path(oracle_lib, torch_cuda
     assert torch.equal(fr[0], fr[1])
 
 
-def _hex8_variant(mesh, order):
+def _hex_variant(mesh, order):
     """The box with jittered nodes, its cells in the given order: 'x' (as built: consecutive cells
     share a face), 'morton', or 'shuffled' (neighbouring lanes share nothing or single nodes)."""
     rng = np.random.default_rng(8)
     h = (mesh.coords.max(axis=0) - mesh.coords.min(axis=0)) / 16
-    mesh.coords += rng.uniform(-0.05, 0.05, mesh.coords.shape) * np.minimum(h, 300.0)
+    mesh.coords += rng.uniform(-0.05, 0.05, mesh.coords.shape) * np.minimum(h, 300.0)  # (Q2: corners count)
     if order == "morton":
         return M.reorder_for_locality(mesh)
     if order == "shuffled":
@@ -597,22 +597,27 @@ def _hex8_variant(mesh, order):
     return mesh
 
 
-# one cell; less than, exactly and one more than a warp; a 64-cell block and a partial one; the
-# first size with 64-cell blocks (more than 148 * 64 cells)
-@pytest.mark.parametrize("n", [(1, 1, 1), (31, 1, 1), (8, 4, 1), (33, 1, 1), (13, 5, 1), (7, 5, 3), (24, 21, 19)])
+# Q1: one cell; less than, exactly and one more than a warp; a 64-cell block and a partial one; the
+# first size with 64-cell blocks (more than 148 * 64 cells). Q2: one cell; one less than, exactly and
+# one more than a warp's ten cells; two warps and three.
+HEX_SIZES = [("hex8", n) for n in [(1, 1, 1), (31, 1, 1), (8, 4, 1), (33, 1, 1), (13, 5, 1), (7, 5, 3), (24, 21, 19)]]
+HEX_SIZES += [("hex27", n) for n in [(1, 1, 1), (9, 1, 1), (10, 1, 1), (11, 1, 1), (5, 2, 2), (7, 3, 2)]]
+
+
+@pytest.mark.parametrize("kind,n", HEX_SIZES)
 @pytest.mark.parametrize("order", ["x", "morton", "shuffled"])
-def test_hex8_cell_kernel_sizes(oracle_lib, torch_cuda, ctx, n, order):
-    """The Q1 kernels against the oracle at warp and block edges, for cell orders with and without
-    faces shared by consecutive cells: residual with body force, action, FP32 action, a cell subset."""
+def test_hex_cell_kernel_sizes(oracle_lib, torch_cuda, ctx, kind, n, order):
+    """The hexahedral kernels against the oracle at warp and block edges, for cell orders with and
+    without faces shared by consecutive cells: residual with body force, action, FP32 action, cell
+    subsets."""
     from pylith_b200 import feassemble as FA
 
     O, torch = oracle_lib, torch_cuda
-    mesh = _hex8_variant(M.box_hex(*n), order)
+    mesh = _hex_variant(M.box_hex(*n) if kind == "hex8" else M.box_hex27(*n), order)
     mat = elastic_setup(mesh, seed=6, body_force=True)
     aux = oracle_aux(O, mat)
     u = np.random.default_rng(7).standard_normal(mesh.num_nodes * 3)
-    plain = O.AuxFields([aux_field for aux_field in [(mat.density[:, None], "cell"), (mat.shear_modulus[:, None], "cell"),
-                                                     (mat.bulk_modulus[:, None], "cell")]])
+    plain = O.AuxFields([(a[:, None], "cell") for a in (mat.density, mat.shear_modulus, mat.bulk_modulus)])
     r_ref = O.residual(mesh, u, aux, f0="Elasticity::g0v_bodyforce", f1=F1_ILE)
     jv_ref = O.jacobian_action(mesh, u, plain, g3=JF3_ILE)
     dm = FA.DeviceMesh(ctx, mesh)
@@ -623,11 +628,9 @@ def test_hex8_cell_kernel_sizes(oracle_lib, torch_cuda, ctx, n, order):
     ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, djv)
     ig.compute_lhs_jacobian_action_f32(0.0, 0.0, du.float(), d32)
     # every second cell as an integrator of its own, then the others on top
-    parts = [np.arange(s, mesh.num_cells, 2, dtype=np.int32) for s in (0, 1)]
     dsum = torch.zeros_like(du)
-    for ids in parts:
-        sub = elastic_setup(mesh, seed=6)
-        part = MAT.IsotropicLinearElasticity(sub.density[ids], sub.shear_modulus[ids], sub.bulk_modulus[ids])
+    for ids in [np.arange(s, mesh.num_cells, 2, dtype=np.int32) for s in (0, 1)]:
+        part = MAT.IsotropicLinearElasticity(mat.density[ids], mat.shear_modulus[ids], mat.bulk_modulus[ids])
         part.create_integrator(dm, ids).compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, dsum, mode=FA.ADD)
     ctx.synchronize()
     assert rel_l2(dr.cpu().numpy(), r_ref) <= TOL64
