@@ -336,8 +336,11 @@ void launch_domain_update_state(const DomainParams& p, int cell, cudaStream_t s)
     if (p.ncells == 0) return;
     const int th = 128;
     const int gr = grid_for(p.ncells, th);
+    if (cell == HEX8) {
+        launch_hex8_update_state(p, s);
+        return;
+    }
     if (cell == TET4) k_domain_update_state<TET4><<<gr, th, 0, s>>>(p);
-    else if (cell == HEX8) k_domain_update_state<HEX8><<<gr, th, 0, s>>>(p);
     else k_domain_update_state<HEX27><<<gr, th, 0, s>>>(p);
     count_launch();
 }

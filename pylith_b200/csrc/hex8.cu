@@ -19,14 +19,67 @@ namespace plb {
 
 template <int RHEO, bool BF, int OP, typename T>
 __global__ void __launch_bounds__(64, sizeof(T) == 4 ? 8 : 4) k_hex8(DomainParams p) {
-    hex8_cell<RHEO, BF, OP, T>(p, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+    extern __shared__ __align__(16) double h8_smem[];
+    hex8_cell<RHEO, BF, OP, T>(p, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, h8_smem);
 }
+
+// State update of generalized-Maxwell cells (domain.cu, k_domain_update_state) with the gradient by
+// edge differences and the state copied ahead; written back in place. Bound: HBM (4.5 TB/s of state
+// read and written). 48x48x36 cells: 60 us with a thread per cell in a loop over the points, 56 us
+// this way; 12 or 16 warps per multiprocessor (456 bytes of spills and more) measured 66 and 73 us.
+__global__ void __launch_bounds__(64, 4) k_hex8_update_state(DomainParams p) {
+    using L = AuxLayout<RHEO_GENMAXWELL, false>;
+    extern __shared__ __align__(16) double h8_smem[];
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= p.ncells) return;
+    Hex8State state(h8_smem, p, c);
+    int nodes[8];
+    hex8_nodes(p, c, nodes);
+    Hex8Nodes<double> h;
+    hex8_load(p.coords, p.u, nodes, h);
+    double a[L::size] = {}, g[8][3];
+    L::load_cell(p, c, a);
+    const pw::MaxwellFactors<double> mf = pw::maxwell_factors(a + L::base + 2, p.constants[0]);
+    hex8_sweep<false, false, double>(
+        h, nullptr, g, [&](int q, const double(&G)[3][3], const double(&C)[3][3], double det, double(&)[3][3], double(&)[3]) {
+            const double rdet = 1.0 / det;
+            double s_x[9], visc[18];
+#pragma unroll
+            for (int f = 0; f < 3; ++f)
+#pragma unroll
+                for (int e = 0; e < 3; ++e)
+                    s_x[f * 3 + e] = (G[f][0] * C[0][e] + G[f][1] * C[1][e] + G[f][2] * C[2][e]) * rdet;
+            const double* st = state.take(q);
+            const pw::Sym<double> e = pw::strain(s_x);
+            pw::genmaxwell_viscous_strain(st, pw::sym_from_vector(st + 18), mf, e, visc);
+            double* pv = p.visc + q * p.ncells + c;
+            double* pt = p.total + q * p.ncells + c;
+#pragma unroll
+            for (int k = 0; k < 18; ++k) pv[(int64_t)k * 8 * p.ncells] = visc[k];
+            const double tot[6] = {e.xx, e.yy, e.zz, e.xy, e.yz, e.xz};
+#pragma unroll
+            for (int k = 0; k < 6; ++k) pt[(int64_t)k * 8 * p.ncells] = tot[k];
+        });
+}
+
+// Threads per block: warps spread over the multiprocessors while there are fewer than two per
+// multiprocessor.
+static int hex8_threads(int64_t ncells) { return ncells <= (int64_t)sm_count() * 64 ? 32 : 64; }
 
 template <int RHEO, bool BF, int OP, typename T>
 static void launch_t(const DomainParams& p, cudaStream_t s) {
-    // warps spread over the multiprocessors while there are fewer than two per multiprocessor
-    const int th = p.ncells <= (int64_t)sm_count() * 64 ? 32 : 64;
-    k_hex8<RHEO, BF, OP, T><<<(unsigned)((p.ncells + th - 1) / th), th, 0, s>>>(p);
+    const int th = hex8_threads(p.ncells);
+    auto kern = k_hex8<RHEO, BF, OP, T>;
+    const size_t smem = RHEO == RHEO_GENMAXWELL && OP == OP_RESIDUAL ? hex8_state_bytes(th) : 0;
+    if (smem) ensure_kernel_smem((const void*)kern, smem);
+    kern<<<(unsigned)((p.ncells + th - 1) / th), th, smem, s>>>(p);
+    count_launch();
+}
+
+void launch_hex8_update_state(const DomainParams& p, cudaStream_t s) {
+    const int th = hex8_threads(p.ncells);
+    ensure_kernel_smem((const void*)k_hex8_update_state, hex8_state_bytes(th));
+    k_hex8_update_state<<<(unsigned)((p.ncells + th - 1) / th), th, hex8_state_bytes(th), s>>>(p);
     count_launch();
 }
 

@@ -11,6 +11,10 @@
 // [0, 1]^3 a Gauss weight is 1/8, applied to the node sums at the end.
 #pragma once
 
+#include <cuda_pipeline.h>
+
+#include <type_traits>
+
 #include "domain_kernels.cuh"
 
 namespace plb {
@@ -31,6 +35,13 @@ template <typename T>
 struct Hex8Nodes {
     T V0[4][6], Dz[4][6];
 };
+
+PL_D void hex8_nodes(const DomainParams& p, int64_t c, int (&nodes)[8]) {
+    const int4* cn = reinterpret_cast<const int4*>(p.cells + 8 * (p.cell_ids ? (int64_t)p.cell_ids[c] : c));
+    const int4 lo = cn[0], hi = cn[1];
+    nodes[0] = lo.x, nodes[1] = lo.y, nodes[2] = lo.z, nodes[3] = lo.w;
+    nodes[4] = hi.x, nodes[5] = hi.y, nodes[6] = hi.z, nodes[7] = hi.w;
+}
 
 template <typename T, typename F>
 PL_D void hex8_load(const double* __restrict__ coords, const F* __restrict__ field, const int (&nodes)[8], Hex8Nodes<T>& h) {
@@ -63,7 +74,8 @@ PL_D void hex8_load(const double* __restrict__ coords, const F* __restrict__ fie
 // the node sums, before the factor 1/8.
 template <bool REVERSE, bool VALUE, typename T, typename Point>
 PL_D void hex8_sweep(const Hex8Nodes<T>& h, unsigned int* err, T (&g)[8][3], Point pt) {
-    T g0[4][3], gz[4][3], az[2][2][3];  // d/dP summed over the planes, its w_k-weighted sum, d/dzeta weights
+    // d/dP summed over the planes, its w_k-weighted sum, d/dzeta weights
+    T g0[4][3], gz[4][3], az[2][2][3];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const T wk = hex8_w<T>(k);
@@ -199,10 +211,48 @@ PL_D void hex8_scatter(const int (&nodes)[8], T (&g)[8][3], T* out) {
             for (int d = 0; d < 3; ++d) red_add(out + 3 * (int64_t)nodes[c] + d, g[c][d]);
 }
 
+// The generalized-Maxwell state of a thread's own cell, point by point (18 viscous strains, 6 total
+// strains), copied three points ahead into the thread's row of shared memory: 192 doubles per cell
+// are the bulk of what these kernels read, and at 8 warps per multiprocessor only copies that hold
+// no registers keep enough of them in flight. A slot is filled again one point after it was read.
+constexpr int kHex8Slots = 4, kHex8Row = 25;  // odd: a warp's accesses fall on distinct banks
+constexpr size_t hex8_state_bytes(int threads) { return sizeof(double) * kHex8Row * kHex8Slots * threads; }
+struct Hex8State {
+    double* row;  // [kHex8Slots][blockDim.x][kHex8Row], this thread's row
+    const DomainParams& p;
+    int64_t c;
+    PL_D Hex8State(double* smem, const DomainParams& params, int64_t cell) : row(smem + threadIdx.x * kHex8Row), p(params), c(cell) {
+#pragma unroll
+        for (int q = 0; q < kHex8Slots - 1; ++q) fetch(q);
+    }
+    PL_D double* slot(int q) { return row + (q % kHex8Slots) * blockDim.x * kHex8Row; }
+    PL_D void fetch(int q) {
+        if (q < 8) {
+            double* dst = slot(q);
+            const double* v = p.visc + q * p.ncells + c;
+            const double* t = p.total + q * p.ncells + c;
+#pragma unroll
+            for (int k = 0; k < 18; ++k) __pipeline_memcpy_async(dst + k, v + (int64_t)k * 8 * p.ncells, sizeof(double));
+#pragma unroll
+            for (int k = 0; k < 6; ++k) __pipeline_memcpy_async(dst + 18 + k, t + (int64_t)k * 8 * p.ncells, sizeof(double));
+        }
+        __pipeline_commit();  // (empty at the end: the wait counts groups)
+    }
+    // The state of point q, visited in order 0 .. 7.
+    PL_D const double* take(int q) {
+        fetch(q + kHex8Slots - 1);
+        __pipeline_wait_prior(kHex8Slots - 1);
+        return slot(q);
+    }
+};
+struct Hex8NoState {
+    PL_D Hex8NoState(double*, const DomainParams&, int64_t) {}
+};
+
 // Residual or Jacobian action of cell c (p.ncells <= c: no cell) into p.out / p.out32; every lane
-// of the warp calls it.
+// of the warp calls it. stage: shared memory of hex8_state_bytes (generalized-Maxwell residual).
 template <int RHEO, bool BF, int OP, typename T>
-PL_D void hex8_cell(const DomainParams& p, int64_t c) {
+PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
     using L = AuxLayout<RHEO, BF>;
     constexpr bool F32 = sizeof(T) == 4;
     const AuxOffsets<RHEO, BF> aoff;
@@ -212,11 +262,9 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c) {
 #pragma unroll
     for (int n = 0; n < 8; ++n) nodes[n] = -1;
     if (live) {
-        const int64_t mc = p.cell_ids ? p.cell_ids[c] : c;
-        const int4* cn = reinterpret_cast<const int4*>(p.cells + 8 * mc);
-        const int4 lo = cn[0], hi = cn[1];
-        nodes[0] = lo.x, nodes[1] = lo.y, nodes[2] = lo.z, nodes[3] = lo.w;
-        nodes[4] = hi.x, nodes[5] = hi.y, nodes[6] = hi.z, nodes[7] = hi.w;
+        constexpr bool STATE = RHEO == RHEO_GENMAXWELL && OP == OP_RESIDUAL;  // the tangents read no state
+        [[maybe_unused]] std::conditional_t<STATE, Hex8State, Hex8NoState> state(stage, p, c);
+        hex8_nodes(p, c, nodes);
         Hex8Nodes<T> h;
         if constexpr (F32) hex8_load(p.coords, p.v32, nodes, h);
         else hex8_load(p.coords, OP == OP_RESIDUAL ? p.u : p.v, nodes, h);
@@ -237,6 +285,10 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c) {
                 mu = (T)(-Jf3[((0 * 3 + 1) * 3 + 1) * 3 + 0]);
             }
         }
+        [[maybe_unused]] pw::MaxwellFactors<double> mf;
+        // once per cell: evaluated at each point, the exponentials made the unrolled code overflow the
+        // instruction cache (69 us against 44 for the residual of 48x48x36 cells)
+        if constexpr (STATE) mf = pw::maxwell_factors(a + L::base + 2, p.constants[0]);
         hex8_sweep<true, BF && OP == OP_RESIDUAL, T>(
             h, p.err, g, [&](int q, const T(&G)[3][3], const T(&C)[3][3], T det, T(&W)[3][3], T(&W0)[3]) {
                 const T rdet = T(1) / det;
@@ -251,7 +303,6 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c) {
                 } else {
 #pragma unroll
                     for (int f = 0; f < 9; ++f) s_x[f] *= rdet;
-                    L::load_qp(p, c, q, 8, a);
                     if constexpr (BF) {
                         const int sOff[1] = {0}, sOff_x[1] = {0};
                         double f0[3] = {0, 0, 0};
@@ -260,7 +311,14 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c) {
 #pragma unroll
                         for (int d = 0; d < 3; ++d) W0[d] = det * f0[d];
                     }
-                    call_f1<RHEO>(L::numA, aoff.v, a, s, s_x, p, x, f1);
+                    if constexpr (STATE) {  // gm3d_f1v with the cell's factors
+                        const double* st = state.take(q);
+                        pw::f1_minus_stress(pw::genmaxwell_stress(a[L::base], a[L::base + 1], a + L::base + 5, st,
+                                                                  pw::sym_from_vector(st + 18), mf, pw::strain(s_x)),
+                                            f1);
+                    } else {
+                        call_f1<RHEO>(L::numA, aoff.v, a, s, s_x, p, x, f1);
+                    }
                 }
 #pragma unroll
                 for (int f = 0; f < 3; ++f)

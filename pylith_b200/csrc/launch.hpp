@@ -34,6 +34,7 @@ bool launch_domain_apply_hexgroup(const DomainParams& p, int cell, int rheo, boo
 // Q1 hexahedra, one thread per cell (hex8.cu).
 void launch_hex8(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
 void launch_hex8_jv32(const DomainParams& p, int rheo, cudaStream_t s);
+void launch_hex8_update_state(const DomainParams& p, cudaStream_t s);
 // Q2 hexahedra, a plane of nodes per lane (hex27.cu).
 void launch_hex27(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
 // FP32 Jacobian action of hexahedra with a group of lanes per cell (FP64 geometry and tangent).

@@ -135,13 +135,26 @@ PL_HD R maxwell_dq(R dt, R tau) {
     return tau * (R(1.0) - exp(-dt / tau)) / dt;
 }
 
+// The two factors of each Maxwell element for a time step dt; they depend on the cell's aux fields
+// alone, so kernels that visit several points of a cell evaluate them once.
 template <typename R>
-PL_HD Sym<R> maxwell_viscous_strain(R tau, const Sym<R>& prev, const Sym<R>& total_prev,
-                                    const Sym<R>& e, R dt) {
+struct MaxwellFactors {
+    R dq[3], ef[3];
+};
+template <typename R>
+PL_HD MaxwellFactors<R> maxwell_factors(const R* tau, R dt) {
+    MaxwellFactors<R> m;
+    for (int i = 0; i < 3; ++i) {
+        m.dq[i] = maxwell_dq(dt, tau[i]);
+        m.ef[i] = exp(-dt / tau[i]);
+    }
+    return m;
+}
+
+template <typename R>
+PL_HD Sym<R> maxwell_viscous_strain(R dq, R ef, const Sym<R>& prev, const Sym<R>& total_prev, const Sym<R>& e) {
     const Sym<R> de = deviatoric(e);
     const Sym<R> dp = deviatoric(total_prev);
-    const R dq = maxwell_dq(dt, tau);
-    const R ef = exp(-dt / tau);
     Sym<R> v;
     v.xx = ef * prev.xx + dq * (de.xx - dp.xx);
     v.yy = ef * prev.yy + dq * (de.yy - dp.yy);
@@ -156,20 +169,13 @@ PL_HD Sym<R> maxwell_viscous_strain(R tau, const Sym<R>& prev, const Sym<R>& tot
 // mu, K, maxwell_time(3), shear_modulus_ratio(3), viscous_strain(18), total_strain(6);
 // constants[0] = dt.
 template <typename R>
-PL_HD Sym<R> genmaxwell_stress(int numA, const int* aOff, const R* a, const R* constants,
+PL_HD Sym<R> genmaxwell_stress(R mu, R K, const R* ratio, const R* visc, const Sym<R>& total, const MaxwellFactors<R>& m,
                                const Sym<R>& e) {
-    const R mu = a[aOff[numA - 6]];
-    const R K = a[aOff[numA - 5]];
-    const R* tau = &a[aOff[numA - 4]];
-    const R* ratio = &a[aOff[numA - 3]];
-    const R* visc = &a[aOff[numA - 2]];
-    const Sym<R> total = sym_from_vector(&a[aOff[numA - 1]]);
-    const R dt = constants[0];
     Sym<R> s = sym_zero<R>();
     add_mean_stress(K, e, &s);
     Sym<R> v[3];
     for (int i = 0; i < 3; ++i)
-        v[i] = maxwell_viscous_strain(tau[i], sym_from_vector(&visc[6 * i]), total, e, dt);
+        v[i] = maxwell_viscous_strain(m.dq[i], m.ef[i], sym_from_vector(&visc[6 * i]), total, e);
     const Sym<R> de = deviatoric(e);
     R r = R(1.0);
     for (int i = 0; i < 3; ++i) r -= ratio[i];
@@ -194,7 +200,10 @@ PL_HD Sym<R> genmaxwell_stress(int numA, const int* aOff, const R* a, const R* c
 template <typename R>
 PL_HD void gm3d_f1v(PLB_POINT_ARGS(R), const R* x, int numConstants, const R* constants, R* f1) {
     const Sym<R> e = strain(&s_x[sOff_x[0]]);
-    f1_minus_stress(genmaxwell_stress(numA, aOff, a, constants, e), f1);
+    const MaxwellFactors<R> m = maxwell_factors(&a[aOff[numA - 4]], constants[0]);
+    f1_minus_stress(genmaxwell_stress(a[aOff[numA - 6]], a[aOff[numA - 5]], &a[aOff[numA - 3]], &a[aOff[numA - 2]],
+                                      sym_from_vector(&a[aOff[numA - 1]]), m, e),
+                    f1);
 }
 
 // IsotropicLinearGenMaxwell3D::Jf3vu_infinitesimalStrain (IsotropicLinearGenMaxwell.hh:1143-1300).
@@ -212,21 +221,24 @@ PL_HD void gm3d_Jf3vu(PLB_POINT_ARGS(R), R s_tshift, const R* x, int numConstant
     jf3_isotropic(K + R(4.0) * shear / R(3.0), K - R(2.0) * shear / R(3.0), shear, Jf3);
 }
 
+// The three elements' viscous strains after the step, as vectors.
+template <typename R>
+PL_HD void genmaxwell_viscous_strain(const R* visc, const Sym<R>& total, const MaxwellFactors<R>& m, const Sym<R>& e, R* out) {
+    for (int i = 0; i < 3; ++i) {
+        const Sym<R> v = maxwell_viscous_strain(m.dq[i], m.ef[i], sym_from_vector(&visc[6 * i]), total, e);
+        R* o = out + 6 * i;
+        o[0] = v.xx; o[1] = v.yy; o[2] = v.zz; o[3] = v.xy; o[4] = v.yz; o[5] = v.xz;
+    }
+}
+
 // IsotropicLinearGenMaxwell3D::viscousStrain_infinitesimalStrain_asVector
 // (IsotropicLinearGenMaxwell.hh:1507-1549).
 template <typename R>
 PL_HD void gm3d_viscous_strain(PLB_POINT_ARGS(R), const R* x, int numConstants,
                                const R* constants, R* out) {
-    const R* tau = &a[aOff[numA - 4]];
-    const R* visc = &a[aOff[numA - 2]];
-    const Sym<R> total = sym_from_vector(&a[aOff[numA - 1]]);
     const Sym<R> e = strain(&s_x[sOff_x[0]]);
-    for (int i = 0; i < 3; ++i) {
-        const Sym<R> v =
-            maxwell_viscous_strain(tau[i], sym_from_vector(&visc[6 * i]), total, e, constants[0]);
-        R* o = out + 6 * i;
-        o[0] = v.xx; o[1] = v.yy; o[2] = v.zz; o[3] = v.xy; o[4] = v.yz; o[5] = v.xz;
-    }
+    genmaxwell_viscous_strain(&a[aOff[numA - 2]], sym_from_vector(&a[aOff[numA - 1]]),
+                              maxwell_factors(&a[aOff[numA - 4]], constants[0]), e, out);
 }
 
 // Elasticity3D::infinitesimalStrain_asVector (Elasticity.hh:587-612).

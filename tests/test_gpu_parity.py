@@ -687,3 +687,67 @@ def test_assembly_and_product_sizes(oracle_lib, torch_cuda, ctx, kind, genmaxwel
     A.spmv(dx, dy)
     ctx.synchronize()
     assert rel_l2(dy.cpu().numpy(), J @ x) <= TOL64
+
+
+# one cell; one more than a warp; one more than a block; the first size with 64-cell blocks, whose
+# state copies take more than the default shared memory
+@pytest.mark.parametrize("n", [(1, 1, 1), (11, 3, 1), (13, 5, 1), (24, 21, 19)])
+@pytest.mark.parametrize("subset", [False, True])
+def test_genmaxwell_hex8_sizes(oracle_lib, torch_cuda, ctx, n, subset):
+    """Generalized-Maxwell residual and state update of Q1 hexahedra at warp and block edges, for
+    all cells in one integrator and in two on complementary subsets."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh = M.box_hex(*n)
+    nc = mesh.num_cells
+    g = genmaxwell_setup(mesh, seed=14)
+    aux = genmaxwell_oracle_aux(O, g)
+    u = np.random.default_rng(15).standard_normal(mesh.num_nodes * 3) * 1e-2
+    r_ref = O.residual(mesh, u, aux, f1=F1_GM, constants=[MAT.YEAR])
+    visc_ref, total_ref = O.project_qp(
+        mesh, u, aux, ["IsotropicLinearGenMaxwell3D::viscousStrain_infinitesimalStrain_asVector",
+                       "Elasticity3D::infinitesimalStrain_asVector"], [18, 6], constants=[MAT.YEAR])
+    dm = FA.DeviceMesh(ctx, mesh)
+    du = dev(torch, u)
+    dr = torch.full_like(du, np.nan)
+    sets = [np.arange(0, nc, 2, dtype=np.int32), np.arange(1, nc, 2, dtype=np.int32)] if subset else [None]
+    visc, total = np.zeros((nc, 8, 18)), np.zeros((nc, 8, 6))
+    for k, ids in enumerate(sets):
+        at = slice(None) if ids is None else ids
+        if ids is not None and len(ids) == 0:
+            continue
+        ig = MAT.IsotropicLinearGenMaxwell(
+            g.density[at], g.shear_modulus[at], g.bulk_modulus[at], g.maxwell_time[at], g.shear_modulus_ratio[at],
+            g.viscous_strain[at], g.total_strain[at]).create_integrator(dm, MAT.YEAR, ids)
+        ig.compute_lhs_residual(0.0, MAT.YEAR, du, dr, mode=FA.ADD if k else FA.INSERT)
+        ig.update_state_vars(0.0, MAT.YEAR, du)
+        ctx.synchronize()
+        m = nc if ids is None else len(ids)
+        visc[at] = ig.get_aux("viscous_strain", (m, 8, 18))
+        total[at] = ig.get_aux("total_strain", (m, 8, 6))
+    assert rel_l2(dr.cpu().numpy(), r_ref) <= TOL64
+    assert rel_l2(visc, visc_ref) <= TOL64
+    assert rel_l2(total, total_ref) <= TOL64
+
+
+@pytest.mark.parametrize("ny,nz", [(1, 1), (7, 1), (8, 1), (3, 3), (17, 1)])
+def test_cohesive_kernel_sizes(oracle_lib, torch_cuda, ctx, ny, nz):
+    """Cohesive residual and actions for cell counts that do and do not fill a warp's eight cells."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh, fault = fault_setup(2, ny, nz)
+    u = np.random.default_rng(16).standard_normal(mesh.num_dof)
+    r_ref = O.cohesive_residual(mesh, u, fault.slip, fault.constants)
+    jv_ref = O.cohesive_jacobian(mesh, fault.constants) @ u
+    ig = fault.create_integrator(FA.DeviceMesh(ctx, mesh))
+    du = dev(torch, u)
+    dr, djv, d32 = torch.full_like(du, np.nan), torch.full_like(du, np.nan), torch.full_like(du.float(), np.nan)
+    ig.compute_lhs_residual(0.0, 0.0, du, dr)
+    ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, du, du, djv)
+    ig.compute_lhs_jacobian_action_f32(0.0, 0.0, du.float(), d32)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), r_ref) <= TOL64
+    assert rel_l2(djv.cpu().numpy(), jv_ref) <= TOL64
+    assert rel_l2(d32.double().cpu().numpy(), jv_ref) <= 1e-5
