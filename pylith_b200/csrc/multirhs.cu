@@ -183,8 +183,15 @@ PL_D bool take_last_ticket(unsigned int* counter) {
 template <int K>
 PL_D void sum_partials_last_block_in(const double* partials, double* out, double* prev, double (*sh)[K]) {
     const int k = threadIdx.x % K;
+    constexpr int STEP = kBThreads / K, U = 8;  // loads in flight: one block reads them all, a chain of L2 latencies
     double s = 0.0;
-    for (int b = threadIdx.x / K; b < (int)gridDim.x; b += kBThreads / K) s += __ldcg(&partials[b * K + k]);
+    for (int b = threadIdx.x / K; b < (int)gridDim.x; b += U * STEP) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = b + u * STEP < (int)gridDim.x ? __ldcg(&partials[(b + u * STEP) * K + k]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) s += v[u];
+    }
 #pragma unroll
     for (int o = K; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -204,6 +211,43 @@ template <int K>
 PL_D void sum_partials_last_block(const double* partials, double* out, double* prev) {
     __shared__ double sh[kBThreads / 32][K];
     sum_partials_last_block_in<K>(partials, out, prev, sh);
+}
+
+// The final sums of two partial arrays at once: fin.out_a (its old value to fin.prev_a) and fin.out_b.
+template <int K>
+PL_D void sum2_partials_last_block(const double* pa, const double* pb, const FinSpec& fin) {
+    __shared__ double sh[2][kBThreads / 32][K];
+    const int k = threadIdx.x % K;
+    constexpr int STEP = kBThreads / K, U = 5;
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x / K; i < (int)gridDim.x; i += U * STEP) {
+        double va[U], vb[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool on = i + u * STEP < (int)gridDim.x;
+            va[u] = on ? __ldcg(&pa[(i + u * STEP) * K + k]) : 0.0;
+            vb[u] = on ? __ldcg(&pb[(i + u * STEP) * K + k]) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) a += va[u], b += vb[u];
+    }
+#pragma unroll
+    for (int o = K; o < 32; o <<= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l < K) sh[0][w][l] = a, sh[1][w][l] = b;
+    __syncthreads();
+    if (threadIdx.x < 2 * K) {
+        const int kk = threadIdx.x % K, which = threadIdx.x / K;
+        double t = 0.0;
+#pragma unroll
+        for (int i = 0; i < kBThreads / 32; ++i) t += sh[which][i][kk];
+        double* out = which ? fin.out_b : fin.out_a;
+        if (!which && fin.prev_a) fin.prev_a[kk] = out[kk];
+        out[kk] = t;
+    }
 }
 
 // Block metadata in shared memory (two buffers: the gather reads one while the next block's is
@@ -323,16 +367,22 @@ __global__ void __launch_bounds__(kMultiBlockCells, 3) k_tet_blocked_jv32_multi(
             ln[3] = lc.w;
             // The registered tangent (Jf3vu_infinitesimalStrain) is isotropic: Jf3 = -C with
             // C = lambda d_ij d_kl + mu (d_ik d_jl + d_il d_jk); its (f,g,df,dg) = (0,1,0,1) and
-            // (0,1,1,0) entries are -lambda and -mu.
-            double a[L::size];
-            L::load_cell(p, c, a);
-            double x[3] = {0, 0, 0};
-            double Jf3d[81];
+            // (0,1,1,0) entries are -lambda and -mu, cached per cell by the solver's setup.
+            if (p.lm32) {
+                const float2 lm = reinterpret_cast<const float2*>(p.lm32)[c];
+                lam = lm.x;
+                mu = lm.y;
+            } else {
+                double a[L::size];
+                L::load_cell(p, c, a);
+                double x[3] = {0, 0, 0};
+                double Jf3d[81];
 #pragma unroll
-            for (int i = 0; i < 81; ++i) Jf3d[i] = 0.0;
-            call_jf3<RHEO_ILE>(L::numA, aoff.v, a, p, x, Jf3d);
-            lam = (float)(-Jf3d[((0 * 3 + 1) * 3 + 0) * 3 + 1]);
-            mu = (float)(-Jf3d[((0 * 3 + 1) * 3 + 1) * 3 + 0]);
+                for (int i = 0; i < 81; ++i) Jf3d[i] = 0.0;
+                call_jf3<RHEO_ILE>(L::numA, aoff.v, a, p, x, Jf3d);
+                lam = (float)(-Jf3d[((0 * 3 + 1) * 3 + 0) * 3 + 1]);
+                mu = (float)(-Jf3d[((0 * 3 + 1) * 3 + 1) * 3 + 0]);
+            }
         }
         __pipeline_wait_prior(0);
         __syncthreads();
@@ -517,6 +567,27 @@ PL_D void block_sum_by_rhs(double a, double* partials) {
     }
 }
 
+// Two of them with one pair of barriers.
+template <int K>
+PL_D void block_sum2_by_rhs(double a, double b, double* partials_a, double* partials_b) {
+    __shared__ double sh[2][kBThreads / 32][K];
+#pragma unroll
+    for (int o = K; o < 32; o <<= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l < K) sh[0][w][l] = a, sh[1][w][l] = b;
+    __syncthreads();
+    if (threadIdx.x < 2 * K) {
+        const int k = threadIdx.x % K, which = threadIdx.x / K;
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < kBThreads / 32; ++i) s += sh[which][i][k];
+        (which ? partials_b : partials_a)[blockIdx.x * K + k] = s;
+    }
+}
+
 // Per-block sums of K values per thread (used by the single-RHS outer residual).
 template <int K>
 PL_D void block_sumK(double (&acc)[K], double* partials) {
@@ -559,6 +630,13 @@ __global__ void __launch_bounds__(kBThreads) k_b_finish(const double* __restrict
         if (prev) prev[k] = out[k];
         out[k] = t;
     }
+}
+
+PL_D void pinv_local(const float* __restrict__ P, int64_t node, const float in[3], float out[3]) {
+    const float* B = P + 9 * node;
+    out[0] = B[0] * in[0] + B[1] * in[1] + B[2] * in[2];
+    out[1] = B[3] * in[0] + B[4] * in[1] + B[5] * in[2];
+    out[2] = B[6] * in[0] + B[7] * in[1] + B[8] * in[2];
 }
 
 template <int K>
@@ -609,42 +687,37 @@ __global__ void __launch_bounds__(kBThreads) k_b_pq(const float* p, const float*
     if (fin.counter && take_last_ticket(fin.counter)) sum_partials_last_block<K>(part, fin.out_a, fin.prev_a);
 }
 
-// alpha_k = active_k ? rz_k / pq_k : 0; r += alpha q; z = P r (stored when StoreZ); partial rz, rr
-// (x is updated by k_b_pupdate). One thread per (node, rhs).
-template <int K, bool StoreZ = true>
-__global__ void __launch_bounds__(kBThreads) k_b_update(float* r, const float* q, float* z,
-                                                        const uint8_t* mask, const float* P, int64_t nnodes,
-                                                        const double* rz, const double* pq, const int* active,
+// alpha_k = active_k ? rz_k / pq_k : 0; r += alpha q; z = P r (not stored: k_b_pupdate_jacobi forms it
+// again from r); partial rz, rr. One thread per (node, rhs), its loads independent of each other:
+// on small meshes the kernel is one chain of latencies, loads to final sums.
+template <int K>
+__global__ void __launch_bounds__(kBThreads) k_b_update(float* __restrict__ r, const float* __restrict__ q,
+                                                        const uint8_t* __restrict__ mask, const float* __restrict__ P,
+                                                        int64_t nnodes, const double* __restrict__ rz,
+                                                        const double* __restrict__ pq, const int* __restrict__ active,
                                                         double* part_rz, double* part_rr, FinSpec fin) {
     const int k = threadIdx.x % K;  // blockDim and the grid stride are multiples of K
     const float alpha = active[k] ? safe_step_f32(rz[k], pq[k]) : 0.0f;
     double srz = 0.0, srr = 0.0;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nnodes * K; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t nd = t / K;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            if (mask[3 * nd + c]) continue;
-            const int64_t i = (3 * nd + c) * K + k;
-            r[i] += alpha * q[i];
-        }
-        float zz[3];
-        pinv_apply<K>(P, r, nd, k, zz);
+        float rn[3], zz[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int64_t i = (3 * nd + c) * K + k;
-            const float ri = r[i];
-            if (StoreZ) z[i] = zz[c];
-            srz += (double)ri * zz[c];
-            srr += (double)ri * ri;
+            const float r0 = r[i], q0 = q[i];
+            rn[c] = mask[3 * nd + c] ? r0 : r0 + alpha * q0;
+        }
+        pinv_local(P, nd, rn, zz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            r[(3 * nd + c) * K + k] = rn[c];
+            srz += (double)rn[c] * zz[c];
+            srr += (double)rn[c] * rn[c];
         }
     }
-    block_sum_by_rhs<K>(srz, part_rz);
-    __syncthreads();
-    block_sum_by_rhs<K>(srr, part_rr);
-    if (fin.counter && take_last_ticket(fin.counter)) {
-        sum_partials_last_block<K>(part_rz, fin.out_a, fin.prev_a);
-        sum_partials_last_block<K>(part_rr, fin.out_b, nullptr);
-    }
+    block_sum2_by_rhs<K>(srz, srr, part_rz, part_rr);
+    if (fin.counter && take_last_ticket(fin.counter)) sum2_partials_last_block<K>(part_rz, part_rr, fin);
 }
 
 // x += alpha p (free DOFs; alpha_k = rz_old_k / pq_k, the step of this iteration, whose r.z is
@@ -673,10 +746,12 @@ __global__ void k_b_pupdate(float* x, float* p, const float* z, const uint8_t* m
 }
 
 // k_b_pupdate for the point-block Jacobi preconditioner, forming z = P r from r (one thread per
-// (node, rhs)) instead of reading a stored z.
+// (node, rhs)) instead of reading a stored z; it also clears q for the next operator application.
 template <int K>
-__global__ void __launch_bounds__(kBThreads) k_b_pupdate_jacobi(float* x, float* p, const float* r,
-                                                                const uint8_t* mask, const float* P, int64_t nnodes,
+__global__ void __launch_bounds__(kBThreads) k_b_pupdate_jacobi(float* __restrict__ x, float* __restrict__ p,
+                                                                const float* __restrict__ r, float* __restrict__ q,
+                                                                const uint8_t* __restrict__ mask, const float* __restrict__ P,
+                                                                int64_t nnodes,
                                                                 const double* rz, const double* rz_old,
                                                                 const double* pq, const int* active) {
     const int k = threadIdx.x % K;  // blockDim and the grid stride are multiples of K
@@ -684,14 +759,21 @@ __global__ void __launch_bounds__(kBThreads) k_b_pupdate_jacobi(float* x, float*
     const float beta = (active[k] && rz_old[k] != 0.0) ? (float)(rz[k] / rz_old[k]) : 0.0f;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nnodes * K; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t nd = t / K;
-        float zz[3];
-        pinv_apply<K>(P, r, nd, k, zz);
+        float rv[3], pv[3], xv[3], zz[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int64_t i = (3 * nd + c) * K + k;
-            const float pe = p[i];
-            if (!mask[3 * nd + c]) x[i] += alpha * pe;
-            p[i] = zz[c] + beta * pe;
+            rv[c] = r[i];
+            pv[c] = p[i];
+            xv[c] = mask[3 * nd + c] ? x[i] : x[i] + alpha * pv[c];
+        }
+        pinv_local(P, nd, rv, zz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int64_t i = (3 * nd + c) * K + k;
+            x[i] = xv[c];
+            p[i] = zz[c] + beta * pv[c];
+            q[i] = 0.0f;
         }
     }
 }
@@ -701,13 +783,6 @@ __global__ void __launch_bounds__(kBThreads) k_b_pupdate_jacobi(float* x, float*
 // "Iterative Methods for Sparse Linear Systems", 2nd ed., Algorithm 12.1), so the preconditioner is a
 // fixed polynomial, symmetric and positive definite while the eigenvalues of P A lie below the
 // upper bound. ----
-
-PL_D void pinv_local(const float* __restrict__ P, int64_t node, const float in[3], float out[3]) {
-    const float* B = P + 9 * node;
-    out[0] = B[0] * in[0] + B[1] * in[1] + B[2] * in[2];
-    out[1] = B[3] * in[0] + B[4] * in[1] + B[5] * in[2];
-    out[2] = B[6] * in[0] + B[7] * in[1] + B[8] * in[2];
-}
 
 // r += alpha q on free DOFs; partial r.r (the preconditioner runs after; x is updated by
 // k_b_pupdate).
@@ -893,6 +968,14 @@ __global__ void __launch_bounds__(kBThreads) k_b_col_prec(const float* r, float*
     block_sumK<1>(acc, part);
 }
 
+// Blocks of the vector kernels whose partial sums are counted by gridDim.x: two items per thread, at
+// most kBBlocks. Small tiles are then not dominated by blocks that only take a ticket (18,270 nodes x
+// 8: 14.1 us per update with 1,184 blocks and two passes over their partial sums one load at a time,
+// 5.7 us now; one or four items per thread are 1 to 2 % slower per solve).
+static int vec_blocks(int64_t items) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>((items + 2 * kBThreads - 1) / (2 * kBThreads), kBBlocks));
+}
+
 static int bgrid(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 8); }
 
 }  // namespace plb
@@ -967,7 +1050,7 @@ bool fuses_energies(pl_batch_solver B) {
 // tile's current r.z, B->scal[0..K)).
 template <int K>
 int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq, unsigned int* ticket, double* part,
-                  const double* scal) {
+                  const double* scal, bool cleared = false) {
     pl_mesh m = S->mesh;
     cudaStream_t s = m->ctx->stream;
     if (pq && S->ops.size() != 1) return fail(PL_ERR_UNSUPPORTED, "fused energies need a single integrator");
@@ -977,7 +1060,7 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
         k_b_unfold<K><<<bgrid(3 * K * S->npairs), 256, 0, s>>>(const_cast<float*>(v), S->d_pair_neg, S->d_pair_pos, S->npairs);
         count_launch();
     }
-    PLB_CUDA(cudaMemsetAsync(out, 0, n * K * sizeof(float), s));
+    if (!cleared) PLB_CUDA(cudaMemsetAsync(out, 0, n * K * sizeof(float), s));
     bool first = true;
     for (pl_integrator ig : S->ops) {
         DomainParams pp;
@@ -985,6 +1068,7 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
         if (rc) return rc;
         pp.t = S->t;
         pp.dt = S->dt;
+        if (ig->lm32_valid && ig->lm32_t == S->t && ig->lm32_dt == S->dt) pp.lm32 = ig->d_lm32;
         if (m->cell_type != PL_CELL_TET4 || ig->j3 != K_ILE_JF3VU || ig->subset)
             return fail(PL_ERR_UNSUPPORTED, "batched solves support P1 tetrahedra with isotropic linear elasticity");
         rc = ensure_blocked_layout(m);
@@ -1025,8 +1109,8 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
 }
 
 template <int K>
-int jv32_multi(pl_batch_solver B, const float* v, float* out, double* pq = nullptr) {
-    return jv32_multi_on<K>(B->base, B->n, v, out, pq, B->ticket, B->part_a, B->scal);
+int jv32_multi(pl_batch_solver B, const float* v, float* out, double* pq = nullptr, bool cleared = false) {
+    return jv32_multi_on<K>(B->base, B->n, v, out, pq, B->ticket, B->part_a, B->scal, cleared);
 }
 
 // z = q(P A) P r with the Chebyshev coefficients of the solver; partial r.z into part_a (and,
@@ -1338,9 +1422,10 @@ int precond_apply(pl_batch_solver B, FinSpec fin = FinSpec()) {
     return B->mg ? bmg_apply<K>(B, fin) : cheb_apply<K>(B, fin);
 }
 
-// One PCG iteration for all K vectors of the tile (capturable: kernels and memsets only).
+// One PCG iteration for all K vectors of the tile (capturable: kernels and memsets only). first:
+// q may hold anything; later iterations of a chunk find it cleared by the point-Jacobi update.
 template <int K>
-int pcg_iteration(pl_batch_solver B) {
+int pcg_iteration(pl_batch_solver B, bool first) {
     pl_solver S = B->base;
     cudaStream_t s = S->mesh->ctx->stream;
     double* rz = B->scal;
@@ -1349,7 +1434,7 @@ int pcg_iteration(pl_batch_solver B) {
     double* rr = B->scal + 3 * K;
     // the final sums are formed by the last block of each reduction kernel (no k_b_finish launches)
     const bool fused = fuses_energies(B);
-    int rc = jv32_multi<K>(B, B->p, B->q, fused ? pq : nullptr);
+    int rc = jv32_multi<K>(B, B->p, B->q, fused ? pq : nullptr, !first && !tile_preconditioned(B));
     if (rc) return rc;
     if (!fused) {
         FinSpec fpq;
@@ -1379,11 +1464,11 @@ int pcg_iteration(pl_batch_solver B) {
         fu.prev_a = rz_old;
         fu.out_b = rr;
         // z = P r is not stored: k_b_pupdate_jacobi forms it again from r
-        k_b_update<K, false><<<kBBlocks, kBThreads, 0, s>>>(B->r, B->q, nullptr, S->d_mask, S->d_pinv32, B->nnodes, rz,
-                                                            pq, B->active, B->part_a, B->part_b, fu);
+        k_b_update<K><<<vec_blocks(B->nnodes * K), kBThreads, 0, s>>>(B->r, B->q, S->d_mask, S->d_pinv32, B->nnodes, rz, pq,
+                                                                      B->active, B->part_a, B->part_b, fu);
         count_launch();
-        k_b_pupdate_jacobi<K><<<kBBlocks, kBThreads, 0, s>>>(B->x, B->p, B->r, S->d_mask, S->d_pinv32, B->nnodes, rz,
-                                                             rz_old, pq, B->active);
+        k_b_pupdate_jacobi<K><<<vec_blocks(B->nnodes * K), kBThreads, 0, s>>>(
+            B->x, B->p, B->r, B->q, S->d_mask, S->d_pinv32, B->nnodes, rz, rz_old, pq, B->active);
         count_launch();
         return PL_OK;
     }
@@ -1455,7 +1540,7 @@ int ensure_pcg_graph(pl_batch_solver B) {
     cudaGraph_t g;
     PLB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
     int rc = PL_OK;
-    for (int i = 0; i < chunk && rc == PL_OK; ++i) rc = pcg_iteration<K>(B);
+    for (int i = 0; i < chunk && rc == PL_OK; ++i) rc = pcg_iteration<K>(B, i == 0);
     cudaError_t e = cudaStreamEndCapture(s, &g);
     if (rc) return rc;
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
