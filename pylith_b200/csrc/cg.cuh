@@ -84,6 +84,51 @@ static __global__ void k_finish2(const double* __restrict__ partials, int nblk, 
     }
 }
 
+// The same sums inside the kernel that produced the partials (after block_sum2; every block calls it
+// with kRedThreads threads): the last block to take a ticket adds them in block order into scal[i0],
+// whose old value goes to scal[prev0] first when prev0 >= 0, and scal[i1] when i1 >= 0. *ticket is
+// zero between kernels. Saves a launch of one block, about 2 us with its gaps.
+PL_D void finish_by_last_block(const double* partials, unsigned int* ticket, double* scal, int i0, int i1, int prev0) {
+    __shared__ bool last;
+    __shared__ double sa[kRedThreads / 32], sb[kRedThreads / 32];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0u;  // every other block has taken its ticket
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    constexpr int U = 5;  // loads in flight
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += U * kRedThreads) {
+        double2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            v[u] = i + u * kRedThreads < (int)gridDim.x ? __ldcg(reinterpret_cast<const double2*>(partials) + i + u * kRedThreads)
+                                                        : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) a += v[u].x, b += v[u].y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) sa[w] = a, sb[w] = b;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double ta = 0.0, tb = 0.0;
+#pragma unroll
+        for (int i = 0; i < kRedThreads / 32; ++i) ta += sa[i], tb += sb[i];
+        if (prev0 >= 0) scal[prev0] = scal[i0];
+        scal[i0] = ta;
+        if (i1 >= 0) scal[i1] = tb;
+    }
+}
+
 // z = P^{-1} r with point blocks; constrained entries of r are zero and P^{-1} is the identity
 // on them, so z stays zero there.
 template <typename T>

@@ -29,7 +29,7 @@ namespace plb {
 
 namespace {
 
-constexpr int kMgRedBlocks = 296;
+constexpr int kMgRedBlocks = 1184;  // at most (mg_red_grid)
 
 enum MgScalar { M_RZ = 0, M_RZ_OLD, M_PQ, M_RR, M_ZROLD, M_COUNT };
 
@@ -107,56 +107,76 @@ __global__ void __launch_bounds__(256) k_dense_apply(const T* __restrict__ inv, 
 
 int mg_grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 8)); }
 
-// out = D^{-1} in / theta; d = out (first Chebyshev step from a zero guess).
-template <typename T>
-__global__ void k_mg_cheb_first(const T* __restrict__ in, const T* __restrict__ pinv, int64_t nn, double inv_theta,
-                                T* __restrict__ d, T* __restrict__ out) {
+// blocks of a reduction over n values (two per thread)
+int mg_red_grid(int64_t n) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>((n + 2 * kRedThreads - 1) / (2 * kRedThreads), kMgRedBlocks));
+}
+
+// The vector kernels of a cycle run between level operators q = J v that add into q, so each kernel
+// that reads q clears it for the next one, and the residual in + q (= in - A z) is formed where it is
+// used instead of in a pass of its own: nine launches per level and cycle, four of them operators
+// (18 with separate residuals, additions and clearing).
+
+// First Chebyshev step from a zero guess: d = D^{-1} rhs / theta. RES: rhs = in + q on free DOFs, 0
+// elsewhere, kept in t, and q is cleared; else rhs = in. out (may be NULL): out = d, or out += d.
+template <typename T, bool RES>
+__global__ void k_mg_cheb_first(const T* __restrict__ in, T* __restrict__ q, const uint8_t* __restrict__ mask,
+                                const T* __restrict__ pinv, int64_t nn, double inv_theta, T* __restrict__ t,
+                                T* __restrict__ d, T* __restrict__ out, bool add) {
     for (int64_t nd = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; nd < nn; nd += (int64_t)gridDim.x * blockDim.x) {
-        T z[3];
-        apply_pinv(pinv, in, nd, z);
+        T rhs[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) rhs[k] = RES ? (mask[3 * nd + k] ? T(0) : (T)(in[3 * nd + k] + q[3 * nd + k])) : in[3 * nd + k];
+        const T* B = pinv + 9 * nd;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const T v = (T)(z[k] * inv_theta);
+            const T z = B[3 * k] * rhs[0] + B[3 * k + 1] * rhs[1] + B[3 * k + 2] * rhs[2];
+            const T v = (T)(z * inv_theta);
+            if (RES) {
+                t[3 * nd + k] = rhs[k];
+                q[3 * nd + k] = T(0);
+            }
             d[3 * nd + k] = v;
-            out[3 * nd + k] = v;
+            if (out) out[3 * nd + k] = add ? out[3 * nd + k] + v : v;
         }
     }
 }
 
-// Chebyshev step: res = in - A out (= in + q on free DOFs, q = J out), d = c1 d + c2 D^{-1} res,
-// out += d.
+// Chebyshev step: res = rhs + q on free DOFs (q = J of the sum so far, cleared here), d = c1 d + c2
+// D^{-1} res, sum += d. The sum so far is in w (NULL: it is d itself, after the first step); out = the
+// new sum, or out += it (out may be w).
 template <typename T>
-__global__ void k_mg_cheb_next(const T* __restrict__ in, const T* __restrict__ q, const T* __restrict__ pinv,
+__global__ void k_mg_cheb_next(const T* __restrict__ rhs, T* __restrict__ q, const T* __restrict__ pinv,
                                const uint8_t* __restrict__ mask, int64_t nn, double c1, double c2, T* __restrict__ d,
-                               T* __restrict__ out) {
+                               const T* w, T* out, bool add) {
     for (int64_t nd = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; nd < nn; nd += (int64_t)gridDim.x * blockDim.x) {
-        T res[3];
+        T res[3], dold[3], sum[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) res[k] = mask[3 * nd + k] ? T(0) : (T)(in[3 * nd + k] + q[3 * nd + k]);
+        for (int k = 0; k < 3; ++k) {
+            res[k] = mask[3 * nd + k] ? T(0) : (T)(rhs[3 * nd + k] + q[3 * nd + k]);
+            dold[k] = d[3 * nd + k];
+            sum[k] = w ? w[3 * nd + k] : dold[k];
+        }
         const T* B = pinv + 9 * nd;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const T zr = B[3 * k] * res[0] + B[3 * k + 1] * res[1] + B[3 * k + 2] * res[2];
-            const T dv = (T)(c1 * d[3 * nd + k] + c2 * zr);
+            const T dv = (T)(c1 * dold[k] + c2 * zr);
+            const T v = sum[k] + dv;
             d[3 * nd + k] = dv;
-            out[3 * nd + k] += dv;
+            q[3 * nd + k] = T(0);
+            out[3 * nd + k] = add ? out[3 * nd + k] + v : v;
         }
     }
 }
 
-// t = in - A z = in + q on free DOFs, 0 elsewhere.
-template <typename T>
-__global__ void k_mg_residual(const T* __restrict__ in, const T* __restrict__ q, const uint8_t* __restrict__ mask,
-                              int64_t n, T* __restrict__ t) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        t[i] = mask[i] ? T(0) : (T)(in[i] + q[i]);
-}
-
 // coarse[c] = sum_j R[c][j] fine[col_j] (R = P^T in coarse rows) for the 3 components, 0 on the
 // coarse level's masked DOFs: one warp per coarse node, its lanes over the row's entries, a fixed
-// shuffle tree for the sums.
-template <typename T>
-__global__ void k_mg_restrict(const T* __restrict__ fine, const int32_t* __restrict__ row, const int32_t* __restrict__ col,
+// shuffle tree for the sums. RES: the fine vector is the residual fine + q on the fine level's free
+// DOFs, 0 elsewhere (q is left as it is: several rows read an entry).
+template <typename T, bool RES>
+__global__ void k_mg_restrict(const T* __restrict__ fine, const T* __restrict__ q, const uint8_t* __restrict__ fmask,
+                              const int32_t* __restrict__ row, const int32_t* __restrict__ col,
                               const double* __restrict__ val, const uint8_t* __restrict__ cmask, int64_t nc,
                               T* __restrict__ coarse) {
     const int lane = threadIdx.x & 31;
@@ -166,9 +186,12 @@ __global__ void k_mg_restrict(const T* __restrict__ fine, const int32_t* __restr
         for (int32_t j = row[c] + lane; j < row[c + 1]; j += 32) {
             const double w = val[j];
             const int64_t f = 3 * (int64_t)col[j];
-            s0 += w * (double)fine[f];
-            s1 += w * (double)fine[f + 1];
-            s2 += w * (double)fine[f + 2];
+            T v[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[k] = RES ? (fmask[f + k] ? T(0) : (T)(fine[f + k] + q[f + k])) : fine[f + k];
+            s0 += w * (double)v[0];
+            s1 += w * (double)v[1];
+            s2 += w * (double)v[2];
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -201,13 +224,16 @@ __global__ void k_mg_pair_map2(int32_t* map, const int32_t* __restrict__ neg, co
         map[pos[k]] = neg[k];
 }
 
-// fine[f] += sum_j P[f][j] coarse[col_j] on free DOFs (P in fine rows).
+// fine[f] += sum_j P[f][j] coarse[col_j] on free DOFs (P in fine rows of the nf mesh nodes); clears q
+// (n DOFs).
 template <typename T>
 __global__ void k_mg_prolong_add(const T* __restrict__ coarse, const int32_t* __restrict__ row,
                                  const int32_t* __restrict__ col, const double* __restrict__ val,
-                                 const uint8_t* __restrict__ mask, int64_t nf, T* __restrict__ fine) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * nf; i += (int64_t)gridDim.x * blockDim.x) {
-        if (mask[i]) continue;
+                                 const uint8_t* __restrict__ mask, int64_t nf, int64_t n, T* __restrict__ fine,
+                                 T* __restrict__ q) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        q[i] = T(0);
+        if (i >= 3 * nf || mask[i]) continue;
         const int64_t f = i / 3;
         const int k = (int)(i % 3);
         double s = 0.0;
@@ -220,11 +246,6 @@ template <typename T>
 __global__ void k_mg_mask(T* __restrict__ v, const uint8_t* __restrict__ mask, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         if (mask[i]) v[i] = T(0);
-}
-
-template <typename T>
-__global__ void k_mg_axpy(T* __restrict__ y, const T* __restrict__ x, int64_t n) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] += x[i];
 }
 
 template <typename A, typename B>
@@ -276,55 +297,69 @@ __global__ void k_mg_normalize(double* __restrict__ v, const double* __restrict_
 }
 
 // ---- outer flexible PCG (FP64) ----------------------------------------------------------------
-// partials of r.z and z.r_old (flexible beta) and r.r
-__global__ void __launch_bounds__(kRedThreads) k_mg_dots(const double* __restrict__ r, const double* __restrict__ z,
+// r.z and z.r_old (flexible beta) over the free DOFs into scal[M_RZ] (its old value to M_RZ_OLD) and
+// scal[M_ZROLD]; z in the precision Z of the cycle.
+template <typename Z>
+__global__ void __launch_bounds__(kRedThreads) k_mg_dots(const double* __restrict__ r, const Z* __restrict__ z,
                                                          const double* __restrict__ r_old, const uint8_t* __restrict__ mask,
-                                                         int64_t n, double* partials) {
+                                                         int64_t n, double* partials, unsigned int* ticket, double* scal) {
     double rz = 0.0, zro = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        if (mask[i]) continue;
-        rz += r[i] * z[i];
-        zro += z[i] * r_old[i];
+        const double zi = mask[i] ? 0.0 : (double)z[i];
+        rz += r[i] * zi;
+        zro += zi * r_old[i];
     }
     block_sum2(rz, zro, partials);
+    finish_by_last_block(partials, ticket, scal, M_RZ, M_ZROLD, M_RZ_OLD);
 }
 
+// -p.q over the free DOFs into scal[slot]
 __global__ void __launch_bounds__(kRedThreads) k_mg_pq(const double* __restrict__ p, const double* __restrict__ q,
-                                                       const uint8_t* __restrict__ mask, int64_t n, double* partials) {
+                                                       const uint8_t* __restrict__ mask, int64_t n, double* partials,
+                                                       unsigned int* ticket, double* scal, int slot) {
     double s = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         if (!mask[i]) s -= p[i] * q[i];
     block_sum2(s, 0.0, partials);
+    finish_by_last_block(partials, ticket, scal, slot, -1, -1);
 }
 
-// x += alpha p, r_old = r, r += alpha q (free DOFs); partial r.r
+// x += alpha p, r_old = r, r += alpha q (free DOFs), r32 = r (unless NULL), q = 0; r.r into scal[M_RR]
 __global__ void __launch_bounds__(kRedThreads) k_mg_update(double* __restrict__ x, double* __restrict__ r,
                                                            double* __restrict__ r_old, const double* __restrict__ p,
-                                                           const double* __restrict__ q, const uint8_t* __restrict__ mask,
-                                                           int64_t n, const double* __restrict__ scal, double* partials) {
+                                                           double* __restrict__ q, float* __restrict__ r32,
+                                                           const uint8_t* __restrict__ mask, int64_t n, double* scal,
+                                                           double* partials, unsigned int* ticket) {
     const double pq = scal[M_PQ];
     const double alpha = pq > 0.0 ? scal[M_RZ] / pq : 0.0;
     double rr = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        r_old[i] = r[i];
-        if (!mask[i]) {
-            x[i] += alpha * p[i];
-            r[i] += alpha * q[i];
-        }
-        rr += r[i] * r[i];
+        const double ro = r[i], qi = q[i], pi = p[i], xi = x[i];
+        const bool m = mask[i];
+        const double rn = m ? ro : ro + alpha * qi;
+        r_old[i] = ro;
+        x[i] = m ? xi : xi + alpha * pi;
+        r[i] = rn;
+        q[i] = 0.0;
+        if (r32) r32[i] = (float)rn;
+        rr += rn * rn;
     }
     block_sum2(rr, 0.0, partials);
+    finish_by_last_block(partials, ticket, scal, M_RR, -1, -1);
 }
 
-// beta = (r.z - z.r_old) / rz_old (Polak-Ribiere, for a preconditioner that may vary), p = z + beta p
-__global__ void k_mg_pupdate(double* __restrict__ p, const double* __restrict__ z, int64_t n, double* scal) {
+// beta = (r.z - z.r_old) / rz_old (Polak-Ribiere, for a preconditioner that may vary), p = z + beta p;
+// start: p = z
+template <typename Z>
+__global__ void k_mg_pupdate(double* __restrict__ p, const Z* __restrict__ z, const uint8_t* __restrict__ mask, int64_t n,
+                             const double* scal, bool start) {
     const double ro = scal[M_RZ_OLD];
-    const double beta = ro != 0.0 ? std::max(0.0, (scal[M_RZ] - scal[M_ZROLD]) / ro) : 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        p[i] = z[i] + beta * p[i];
+    const double beta = !start && ro != 0.0 ? std::max(0.0, (scal[M_RZ] - scal[M_ZROLD]) / ro) : 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double zi = mask[i] ? 0.0 : (double)z[i];
+        p[i] = start ? zi : zi + beta * p[i];
+    }
 }
-
-__global__ void k_mg_copy_scalar(double* scal, int from, int to) { scal[to] = scal[from]; }
 
 // ---- restriction = transpose of the prolongation, built on the device -------------------------
 // Entries per coarse node (cnt zeroed before).
@@ -417,7 +452,8 @@ struct pl_multigrid_s {
     pl_solver attached = nullptr;
     int batch_users = 0;  // batched solvers preconditioned by this hierarchy
     // outer PCG state
-    double *x = nullptr, *r = nullptr, *r_old = nullptr, *p = nullptr, *q = nullptr, *z = nullptr;
+    double *x = nullptr, *r = nullptr, *r_old = nullptr, *p = nullptr, *q = nullptr;
+    unsigned int* ticket = nullptr;  // last-block counter of the reductions (zero between kernels)
     double* scal = nullptr;
     double* partials = nullptr;
     cudaGraphExec_t graph = nullptr;
@@ -439,104 +475,133 @@ namespace {
 
 cudaStream_t mg_stream(pl_multigrid mg) { return mg->lv[0].S->mesh->ctx->stream; }
 
-// Chebyshev polynomial of point-block Jacobi on level l: out = p(D^-1 A) D^-1 in, from zero.
+// q += J v on level l (q holds zero: the vector kernels clear it)
 template <typename T>
-int cheb(pl_multigrid mg, int l, const T* in, T* out, int degree, double lower) {
+int level_apply(MgLevel& L, const T* v) {
+    if constexpr (sizeof(T) == 4) return solver_apply_J32(L.S, v, L.q32, true);
+    else return solver_apply_J(L.S, v, L.q, true);
+}
+
+// Chebyshev polynomial of point-block Jacobi on level l from zero: out = p(D^-1 A) D^-1 rhs, or out +=
+// it (add). residual: rhs = in + q (see k_mg_cheb_first), else rhs = in. Leaves q cleared.
+template <typename T>
+int cheb(pl_multigrid mg, int l, const T* in, bool residual, T* out, bool add, int degree, double lower) {
     MgLevel& L = mg->lv[l];
     cudaStream_t s = mg_stream(mg);
     const double b = 1.1 * L.lmax, a = lower * b;
     const double theta = 0.5 * (b + a), delta = 0.5 * (b - a), sigma = theta / delta;
-    T* d = sizeof(T) == 8 ? (T*)L.d : (T*)L.d32;
-    T* q = sizeof(T) == 8 ? (T*)L.q : (T*)L.q32;
-    const T* pinv = sizeof(T) == 8 ? (const T*)L.S->d_pinv : (const T*)L.S->d_pinv32;
-    k_mg_cheb_first<T><<<mg_grid(L.nn), 256, 0, s>>>(in, pinv, L.nn, 1.0 / theta, d, out);
+    constexpr bool f32 = sizeof(T) == 4;
+    T* d = f32 ? (T*)L.d32 : (T*)L.d;
+    T* q = f32 ? (T*)L.q32 : (T*)L.q;
+    T* t = f32 ? (T*)L.t32 : (T*)L.t;
+    T* w = f32 ? (T*)L.w32 : (T*)L.w;
+    const T* pinv = f32 ? (const T*)L.S->d_pinv32 : (const T*)L.S->d_pinv;
+    T* only = degree == 1 ? out : nullptr;
+    if (residual) k_mg_cheb_first<T, true><<<mg_grid(L.nn), 256, 0, s>>>(in, q, L.S->d_mask, pinv, L.nn, 1.0 / theta, t, d, only, add);
+    else k_mg_cheb_first<T, false><<<mg_grid(L.nn), 256, 0, s>>>(in, q, L.S->d_mask, pinv, L.nn, 1.0 / theta, t, d, only, add);
     count_launch();
+    const T* rhs = residual ? t : in;
     double rho_old = 1.0 / sigma;
     for (int k = 1; k < degree; ++k) {
-        int rc = sizeof(T) == 8 ? solver_apply_J(L.S, (const double*)out, (double*)q)
-                                : solver_apply_J32(L.S, (const float*)out, (float*)q);
+        int rc = level_apply<T>(L, k == 1 ? d : w);
         if (rc) return rc;
         const double rho = 1.0 / (2.0 * sigma - rho_old);
-        k_mg_cheb_next<T><<<mg_grid(L.nn), 256, 0, s>>>(in, q, pinv, L.S->d_mask, L.nn, rho * rho_old, 2.0 * rho / delta,
-                                                        d, out);
+        const bool lastk = k == degree - 1;
+        k_mg_cheb_next<T><<<mg_grid(L.nn), 256, 0, s>>>(rhs, q, pinv, L.S->d_mask, L.nn, rho * rho_old, 2.0 * rho / delta, d,
+                                                        k == 1 ? nullptr : w, lastk ? out : w, lastk && add);
         count_launch();
         rho_old = rho;
     }
     return PL_OK;
 }
 
-// z_l = V(r_l) on level l (vectors of the level's work set in precision T).
+// z_l = V(r) on level l (vectors of the level's work set in precision T; q holds zero before and
+// after).
 template <typename T>
-int vcycle(pl_multigrid mg, int l) {
+int vcycle(pl_multigrid mg, int l, const T* r) {
     MgLevel& L = mg->lv[l];
     cudaStream_t s = mg_stream(mg);
-    const bool f32 = sizeof(T) == 4;
-    T* r = f32 ? (T*)L.r32 : (T*)L.r;
+    constexpr bool f32 = sizeof(T) == 4;
     T* z = f32 ? (T*)L.z32 : (T*)L.z;
-    T* t = f32 ? (T*)L.t32 : (T*)L.t;
-    T* w = f32 ? (T*)L.w32 : (T*)L.w;
     T* q = f32 ? (T*)L.q32 : (T*)L.q;
     const int last = (int)mg->lv.size() - 1;
     if (l == last) {
-        if (!mg->dense_ok) return cheb<T>(mg, l, r, z, mg->coarse_degree, mg->coarse_lower);
-        PLB_CUDA(cudaMemsetAsync(z, 0, L.n * sizeof(T), s));
+        if (!mg->dense_ok) return cheb<T>(mg, l, r, false, z, false, mg->coarse_degree, mg->coarse_lower);
+        // z is zero off the dense unknowns (cleared when the solve starts)
         const T* inv = f32 ? (const T*)mg->d_dense32 : (const T*)mg->d_dense;
         k_dense_apply<T><<<std::max(1, std::min((mg->dense_n + 7) / 8, 148)), 256, 0, s>>>(inv, mg->d_dense_idx,
                                                                                              mg->dense_n, r, z);
         count_launch();
         return PL_OK;
     }
-    auto apply = [&](T* v) { return f32 ? solver_apply_J32(L.S, (const float*)v, (float*)q) : solver_apply_J(L.S, (const double*)v, (double*)q); };
     int rc = PL_OK;
-    const T* tr = r;  // the residual to restrict
-    if (mg->pre_smooth) {
-        if ((rc = cheb<T>(mg, l, r, z, mg->degree, mg->lower))) return rc;
-        if ((rc = apply(z))) return rc;
-        k_mg_residual<T><<<mg_grid(L.n), 256, 0, s>>>(r, q, L.S->d_mask, L.n, t);
-        tr = t;
-    } else {
-        PLB_CUDA(cudaMemsetAsync(z, 0, L.n * sizeof(T), s));
-    }
-    // restriction into the coarse level's r, folded and masked
+    // restriction into the coarse level's r, masked: its rows are the coarse level's reduced space
+    // (the prolongation columns were mapped onto it), so there is no fold; the Lagrange rows of the
+    // coarse vector stay zero (cleared when the solve starts)
     MgLevel& C = mg->lv[l + 1];
     T* rc_ = f32 ? (T*)C.r32 : (T*)C.r;
     T* zc = f32 ? (T*)C.z32 : (T*)C.z;
-    // the restriction's rows are the coarse level's reduced space (its prolongation columns were
-    // mapped onto it): no fold; the Lagrange rows of the coarse vector stay zero
-    if (C.n > 3 * C.nmesh) PLB_CUDA(cudaMemsetAsync(rc_ + 3 * C.nmesh, 0, (C.n - 3 * C.nmesh) * sizeof(T), s));
-    k_mg_restrict<T><<<mg_grid(32 * C.nmesh), 256, 0, s>>>(tr, L.r_row, L.r_col, L.r_val, C.S->d_mask, C.nmesh, rc_);
-    count_launch(2);
-    if ((rc = vcycle<T>(mg, l + 1))) return rc;
+    if (mg->pre_smooth) {
+        if ((rc = cheb<T>(mg, l, r, false, z, false, mg->degree, mg->lower))) return rc;
+        if ((rc = level_apply<T>(L, z))) return rc;
+        k_mg_restrict<T, true><<<mg_grid(32 * C.nmesh), 256, 0, s>>>(r, q, L.S->d_mask, L.r_row, L.r_col, L.r_val, C.S->d_mask,
+                                                                     C.nmesh, rc_);
+    } else {
+        PLB_CUDA(cudaMemsetAsync(z, 0, L.n * sizeof(T), s));
+        k_mg_restrict<T, false><<<mg_grid(32 * C.nmesh), 256, 0, s>>>(r, nullptr, nullptr, L.r_row, L.r_col, L.r_val, C.S->d_mask,
+                                                                      C.nmesh, rc_);
+    }
+    count_launch();
+    if ((rc = vcycle<T>(mg, l + 1, rc_))) return rc;
     // ... and the prolongation reads the coarse correction there: no unfold
-    k_mg_prolong_add<T><<<mg_grid(3 * L.nmesh), 256, 0, s>>>(zc, L.p_row, L.p_col, L.p_val, L.S->d_mask, L.nmesh, z);
+    k_mg_prolong_add<T><<<mg_grid(L.n), 256, 0, s>>>(zc, L.p_row, L.p_col, L.p_val, L.S->d_mask, L.nmesh, L.n, z, q);
     count_launch();
-    // post-smoothing on the new residual
     if (!mg->post_smooth) return PL_OK;
-    if ((rc = apply(z))) return rc;
-    k_mg_residual<T><<<mg_grid(L.n), 256, 0, s>>>(r, q, L.S->d_mask, L.n, t);
-    count_launch();
-    if ((rc = cheb<T>(mg, l, t, w, mg->degree, mg->lower))) return rc;
-    k_mg_axpy<T><<<mg_grid(L.n), 256, 0, s>>>(z, w, L.n);
-    count_launch();
-    return PL_OK;
+    // post-smoothing on the new residual, added to z
+    if ((rc = level_apply<T>(L, z))) return rc;
+    return cheb<T>(mg, l, r, true, z, true, mg->degree, mg->lower);
 }
 
-// z = M r on the fine level (FP64 vectors in and out; an FP32 V-cycle converts at the ends).
-int precondition(pl_multigrid mg, const double* r, double* z) {
-    MgLevel& L = mg->lv[0];
+// z_0 = V(r) on the fine level: r in FP64, or for an FP32 V-cycle its copy in the level's r32.
+int precondition(pl_multigrid mg) {
+    return mg->fp32 ? vcycle<float>(mg, 0, mg->lv[0].r32) : vcycle<double>(mg, 0, mg->r);
+}
+
+// r.z and z.r_old, then p = z + beta p (start: p = z) with the z of the last cycle.
+void dots_and_direction(pl_multigrid mg, const double* r_old, bool start) {
+    pl_solver S = mg->lv[0].S;
     cudaStream_t s = mg_stream(mg);
-    int rc;
-    if (mg->fp32) {
-        k_mg_convert<double, float><<<mg_grid(L.n), 256, 0, s>>>(r, L.r32, L.n);
-        count_launch();
-        if ((rc = vcycle<float>(mg, 0))) return rc;
-        k_mg_convert<float, double><<<mg_grid(L.n), 256, 0, s>>>(L.z32, z, L.n);
-        count_launch();
-    } else {
-        PLB_CUDA(cudaMemcpyAsync(L.r, r, L.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        if ((rc = vcycle<double>(mg, 0))) return rc;
-        PLB_CUDA(cudaMemcpyAsync(z, L.z, L.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    const int64_t n = S->n;
+    const MgLevel& L = mg->lv[0];
+    auto run = [&](const auto* z) {
+        using Z = std::remove_cv_t<std::remove_pointer_t<decltype(z)>>;
+        k_mg_dots<Z><<<mg_red_grid(n), kRedThreads, 0, s>>>(mg->r, z, r_old, S->d_mask, n, mg->partials, mg->ticket, mg->scal);
+        k_mg_pupdate<Z><<<mg_grid(n), 256, 0, s>>>(mg->p, z, S->d_mask, n, mg->scal, start);
+    };
+    if (mg->fp32) run((const float*)L.z32);
+    else run((const double*)L.z);
+    count_launch(2);
+}
+
+// What the cycles and iterations expect cleared: every level's q, the coarsest level's z (its dense
+// solve writes the unknowns only), the Lagrange rows of the coarse right-hand sides, the fine q.
+int clear_for_solve(pl_multigrid mg) {
+    cudaStream_t s = mg_stream(mg);
+    for (size_t l = 0; l < mg->lv.size(); ++l) {
+        MgLevel& L = mg->lv[l];
+        const int64_t tail = L.n - 3 * L.nmesh;
+        const bool last = l + 1 == mg->lv.size();
+        if (mg->fp32) {
+            PLB_CUDA(cudaMemsetAsync(L.q32, 0, L.n * sizeof(float), s));
+            if (last) PLB_CUDA(cudaMemsetAsync(L.z32, 0, L.n * sizeof(float), s));
+            if (l > 0 && tail > 0) PLB_CUDA(cudaMemsetAsync(L.r32 + 3 * L.nmesh, 0, tail * sizeof(float), s));
+        } else {
+            PLB_CUDA(cudaMemsetAsync(L.q, 0, L.n * sizeof(double), s));
+            if (last) PLB_CUDA(cudaMemsetAsync(L.z, 0, L.n * sizeof(double), s));
+            if (l > 0 && tail > 0) PLB_CUDA(cudaMemsetAsync(L.r + 3 * L.nmesh, 0, tail * sizeof(double), s));
+        }
     }
+    PLB_CUDA(cudaMemsetAsync(mg->q, 0, mg->lv[0].n * sizeof(double), s));
     return PL_OK;
 }
 
@@ -547,15 +612,16 @@ int estimate_eigenvalues(pl_multigrid mg, int iters = 12) {
     for (size_t l = 0; l < mg->lv.size(); ++l) {
         MgLevel& L = mg->lv[l];
         if (l + 1 == mg->lv.size() && mg->dense_ok) break;  // solved exactly: no smoother
-        k_mg_seed<<<kMgRedBlocks, kRedThreads, 0, s>>>(L.t, L.S->d_mask, L.n, mg->partials);
-        k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_RR, -1);
+        const int grid = mg_red_grid(L.n);
+        k_mg_seed<<<grid, kRedThreads, 0, s>>>(L.t, L.S->d_mask, L.n, mg->partials);
+        k_finish2<<<1, 1024, 0, s>>>(mg->partials, grid, mg->scal, M_RR, -1);
         k_mg_normalize<<<mg_grid(L.n), 256, 0, s>>>(L.t, L.t, L.n, mg->scal, M_RR);
         count_launch(3);
         for (int it = 0; it < iters; ++it) {
             int rc = solver_apply_J(L.S, L.t, L.q);
             if (rc) return rc;
-            k_mg_power<<<kMgRedBlocks, kRedThreads, 0, s>>>(L.q, L.S->d_pinv, L.S->d_mask, L.nn, L.w, mg->partials);
-            k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_RR, -1);
+            k_mg_power<<<grid, kRedThreads, 0, s>>>(L.q, L.S->d_pinv, L.S->d_mask, L.nn, L.w, mg->partials);
+            k_finish2<<<1, 1024, 0, s>>>(mg->partials, grid, mg->scal, M_RR, -1);
             k_mg_normalize<<<mg_grid(L.n), 256, 0, s>>>(L.t, L.w, L.n, mg->scal, M_RR);
             count_launch(3);
         }
@@ -653,21 +719,15 @@ int mg_iteration(pl_multigrid mg) {
     pl_solver S = mg->lv[0].S;
     cudaStream_t s = mg_stream(mg);
     const int64_t n = S->n;
-    int rc = solver_apply_J(S, mg->p, mg->q);
+    int rc = solver_apply_J(S, mg->p, mg->q, true);
     if (rc) return rc;
-    k_mg_pq<<<kMgRedBlocks, kRedThreads, 0, s>>>(mg->p, mg->q, S->d_mask, n, mg->partials);
-    k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_PQ, -1);
-    k_mg_copy_scalar<<<1, 1, 0, s>>>(mg->scal, M_RZ, M_RZ_OLD);
-    k_mg_update<<<kMgRedBlocks, kRedThreads, 0, s>>>(mg->x, mg->r, mg->r_old, mg->p, mg->q, S->d_mask, n, mg->scal,
-                                                       mg->partials);
-    k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_RR, -1);
-    count_launch(5);
-    if ((rc = precondition(mg, mg->r, mg->z))) return rc;
-    k_mg_mask<double><<<mg_grid(n), 256, 0, s>>>(mg->z, S->d_mask, n);
-    k_mg_dots<<<kMgRedBlocks, kRedThreads, 0, s>>>(mg->r, mg->z, mg->r_old, S->d_mask, n, mg->partials);
-    k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_RZ, M_ZROLD);
-    k_mg_pupdate<<<mg_grid(n), 256, 0, s>>>(mg->p, mg->z, n, mg->scal);
-    count_launch(4);
+    const int grid = mg_red_grid(n);
+    k_mg_pq<<<grid, kRedThreads, 0, s>>>(mg->p, mg->q, S->d_mask, n, mg->partials, mg->ticket, mg->scal, M_PQ);
+    k_mg_update<<<grid, kRedThreads, 0, s>>>(mg->x, mg->r, mg->r_old, mg->p, mg->q, mg->fp32 ? mg->lv[0].r32 : nullptr, S->d_mask,
+                                             n, mg->scal, mg->partials, mg->ticket);
+    count_launch(2);
+    if ((rc = precondition(mg))) return rc;
+    dots_and_direction(mg, mg->r_old, false);
     return PL_OK;
 }
 
@@ -713,16 +773,16 @@ int multigrid_solve(pl_multigrid mg, const double* b, double* x) {
             break;
         }
         k_mg_mask<double><<<mg_grid(n), 256, 0, s>>>(mg->r, S->d_mask, n);
-        k_mg_pq<<<kMgRedBlocks, kRedThreads, 0, s>>>(mg->r, mg->r, S->d_mask, n, mg->partials);  // -r.r
-        k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_RR, -1);
-        count_launch(3);
-        if ((rc = precondition(mg, mg->r, mg->z)) != PL_OK) break;
-        k_mg_mask<double><<<mg_grid(n), 256, 0, s>>>(mg->z, S->d_mask, n);
-        k_mg_dots<<<kMgRedBlocks, kRedThreads, 0, s>>>(mg->r, mg->z, mg->z, S->d_mask, n, mg->partials);
-        k_finish2<<<1, 1024, 0, s>>>(mg->partials, kMgRedBlocks, mg->scal, M_RZ, -1);
-        count_launch(3);
-        if (cudaMemcpyAsync(mg->p, mg->z, n * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
-            cudaMemcpyAsync(h, mg->scal, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        k_mg_pq<<<mg_red_grid(n), kRedThreads, 0, s>>>(mg->r, mg->r, S->d_mask, n, mg->partials, mg->ticket, mg->scal,
+                                                       M_RR);  // -r.r
+        count_launch(2);
+        if (mg->fp32) {
+            k_mg_convert<double, float><<<mg_grid(n), 256, 0, s>>>(mg->r, mg->lv[0].r32, n);
+            count_launch();
+        }
+        if ((rc = clear_for_solve(mg)) != PL_OK || (rc = precondition(mg)) != PL_OK) break;
+        dots_and_direction(mg, mg->r, true);
+        if (cudaMemcpyAsync(h, mg->scal, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess) {
             rc = fail(PL_ERR_CUDA, "multigrid start");
             break;
@@ -895,7 +955,9 @@ int pl_multigrid_create(pl_solver fine, int num_coarse, const pl_solver* coarse,
         d_tmp = nullptr;
     }
     const int64_t n = fine->n;
-    A(&mg->x, n); A(&mg->r, n); A(&mg->r_old, n); A(&mg->p, n); A(&mg->q, n); A(&mg->z, n);
+    A(&mg->x, n); A(&mg->r, n); A(&mg->r_old, n); A(&mg->p, n); A(&mg->q, n);
+    A(&mg->ticket, 1);
+    if (e == cudaSuccess) e = cudaMemsetAsync(mg->ticket, 0, sizeof(unsigned int), s);
     A(&mg->scal, M_COUNT);
     A(&mg->partials, 2 * kMgRedBlocks);
     if (e != cudaSuccess) {
@@ -904,7 +966,7 @@ int pl_multigrid_create(pl_solver fine, int num_coarse, const pl_solver* coarse,
                             L.r_row, L.r_col, L.r_val};
             for (void* p : ptrs) dev_free(p, s);
         }
-        void* ptrs[] = {mg->x, mg->r, mg->r_old, mg->p, mg->q, mg->z, mg->scal, mg->partials};
+        void* ptrs[] = {mg->x, mg->r, mg->r_old, mg->p, mg->q, mg->ticket, mg->scal, mg->partials};
         for (void* p : ptrs) dev_free(p, s);
         delete mg;
         return cuda_fail(e, "pl_multigrid_create");
@@ -973,7 +1035,7 @@ int pl_multigrid_destroy(pl_multigrid mg) {
                         L.r_row, L.r_col, L.r_val};
         for (void* p : ptrs) dev_free(p, mg->ctx ? mg->ctx->stream : nullptr);
     }
-    void* ptrs[] = {mg->x, mg->r, mg->r_old, mg->p, mg->q, mg->z, mg->scal, mg->partials,
+    void* ptrs[] = {mg->x, mg->r, mg->r_old, mg->p, mg->q, mg->ticket, mg->scal, mg->partials,
                     mg->d_dense_idx, mg->d_dense_map, mg->d_dense, mg->d_dense32, mg->d_gj, mg->d_flag};
     for (void* p : ptrs) dev_free(p, mg->ctx ? mg->ctx->stream : nullptr);
     if (mg->dense_A) pl_matrix_destroy(mg->dense_A);

@@ -313,35 +313,37 @@ void fault_fold(pl_solver S, T* v) {
 
 // out = P^T J P v: with S->reduced by the kernels' reduced fault space (every positive-side node
 // read as, and added into, its negative-side partner), else by unfolding v in place (its
-// positive-side entries are written) and folding the result.
-int apply_J(pl_solver S, const double* v, double* out) {
+// positive-side entries are written) and folding the result. cleared: out holds zero already (no
+// memset).
+int apply_J(pl_solver S, const double* v, double* out, bool cleared = false) {
     if (S->reduced) {
         for (size_t i = 0; i < S->ops.size(); ++i) {
-            int rc = jacobian_action_reduced(S->ops[i], S->t, S->dt, v, out, i == 0 ? PL_INSERT : PL_ADD);
+            int rc = jacobian_action_reduced(S->ops[i], S->t, S->dt, v, out, i == 0 && !cleared ? PL_INSERT : PL_ADD);
             if (rc) return rc;
         }
         return PL_OK;
     }
     fault_unfold(S, const_cast<double*>(v));
     for (size_t i = 0; i < S->ops.size(); ++i) {
-        int rc = pl_compute_lhs_jacobian_action(S->ops[i], S->t, S->dt, 0.0, nullptr, v, out, i == 0 ? PL_INSERT : PL_ADD);
+        int rc = pl_compute_lhs_jacobian_action(S->ops[i], S->t, S->dt, 0.0, nullptr, v, out,
+                                                i == 0 && !cleared ? PL_INSERT : PL_ADD);
         if (rc) return rc;
     }
     fault_fold(S, out);
     return PL_OK;
 }
 
-int apply_J32(pl_solver S, const float* v, float* out) {
+int apply_J32(pl_solver S, const float* v, float* out, bool cleared = false) {
     if (S->reduced) {
         for (size_t i = 0; i < S->ops.size(); ++i) {
-            int rc = jacobian_action_reduced_f32(S->ops[i], S->t, S->dt, v, out, i == 0 ? PL_INSERT : PL_ADD);
+            int rc = jacobian_action_reduced_f32(S->ops[i], S->t, S->dt, v, out, i == 0 && !cleared ? PL_INSERT : PL_ADD);
             if (rc) return rc;
         }
         return PL_OK;
     }
     fault_unfold(S, const_cast<float*>(v));
     for (size_t i = 0; i < S->ops.size(); ++i) {
-        int rc = pl_compute_lhs_jacobian_action_f32(S->ops[i], S->t, S->dt, v, out, i == 0 ? PL_INSERT : PL_ADD);
+        int rc = pl_compute_lhs_jacobian_action_f32(S->ops[i], S->t, S->dt, v, out, i == 0 && !cleared ? PL_INSERT : PL_ADD);
         if (rc) return rc;
     }
     fault_fold(S, out);
@@ -567,8 +569,8 @@ namespace plb {
 
 // Operator pieces for outside drivers (the multigrid hierarchy): q = J v with the fault's unfold
 // and fold (FP64, FP32), and the unfold / fold alone.
-int solver_apply_J(pl_solver S, const double* v, double* out) { return apply_J(S, v, out); }
-int solver_apply_J32(pl_solver S, const float* v, float* out) { return apply_J32(S, v, out); }
+int solver_apply_J(pl_solver S, const double* v, double* out, bool cleared) { return apply_J(S, v, out, cleared); }
+int solver_apply_J32(pl_solver S, const float* v, float* out, bool cleared) { return apply_J32(S, v, out, cleared); }
 void solver_unfold(pl_solver S, double* v) { fault_unfold(S, v); }
 void solver_unfold32(pl_solver S, float* v) { fault_unfold(S, v); }
 void solver_fold(pl_solver S, double* v) { fault_fold(S, v); }

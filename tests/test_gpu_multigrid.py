@@ -138,3 +138,41 @@ def test_batched_multigrid_green_functions(ctx):
         assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)
     assert st_mg["max_rel_residual"] <= 1e-11
     assert 5 * st_mg["inner_iterations"] <= st_j["inner_iterations"], (st_mg, st_j)
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3])
+@pytest.mark.parametrize("pre,post", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_cycle_forms_reach_the_same_solution(ctx, degree, pre, post, fp32):
+    """Every form of the V-cycle (smoother degrees with and without a second step, either smoothing
+    off, both precisions) preconditions a solve twice in a row, on an odd box with a fault, to the
+    solution of point-block-Jacobi PCG (relative residual 1e-12, solutions within 1e-8)."""
+    from pylith_b200 import feassemble as FA
+    from pylith_b200 import problems as P
+
+    nx, ny, nz = 12, 9, 7
+    levels = MG.build_hierarchy(nx, ny, nz, fault_x=0.0, max_coarse_nodes=120,
+                                constrained_faces=[(0, "neg", (0, 1, 2)), (0, "pos", (0, 1, 2))])
+    mesh = levels[0].mesh
+    mat = MAT.IsotropicLinearElasticity(*MAT.lognormal_elastic(mesh.num_cells, seed=5))
+    slip = np.zeros((mesh.num_lagrange, 3))
+    slip[: mesh.num_lagrange // 2, 1] = 2.0
+
+    def problem():
+        return P.QuasistaticProblem(ctx, mesh, [(mat, None)], levels[0].constrained, np.zeros(mesh.num_dof),
+                                    faults=[MAT.FaultCohesiveKin(slip)], rtol=1e-12)
+
+    ref = problem()
+    ref.step(0.0)
+    u_ref = ref.u.cpu().numpy()
+    prob = problem()
+    mg = MG.attach(ctx, prob.solver, levels, mat, fault_x=0.0, degree=degree,
+                   precision=FA.Solver.FP32_REFINED if fp32 else FA.Solver.FP64)
+    mg.set_cycle(pre, post)
+    for _ in range(2):
+        prob.u.zero_()
+        st = prob.step(0.0)
+        assert st.rel_residual <= 1e-12
+        u = prob.u.cpu().numpy()
+        assert np.linalg.norm(u - u_ref) <= 1e-8 * np.linalg.norm(u_ref)
+    mg.close()
