@@ -1,4 +1,5 @@
-// Cell-block kernels for P1 tetrahedra: the hot path of the residual and Jacobian action.
+// Cell-block kernels for P1 tetrahedra, one cell per thread: residual and Jacobian action of meshes
+// whose consecutive cells are too scattered for the pairs of tetpair.cu.
 //
 // Cells are processed in blocks of kTetBlockCells consecutive cells (meshes are ordered along
 // a Morton curve, so a block is a compact patch). Persistent CTAs walk every gridDim.x-th block.
@@ -25,6 +26,7 @@
 #include <thread>
 #include <vector>
 
+#include "bankplan.hpp"
 #include "domain_kernels.cuh"
 #include "internal.hpp"
 #include "launch.hpp"
@@ -1024,8 +1026,8 @@ static void launch_pipe_t(const DomainParams& p, const BlockedLayout& b, bool in
     }
 }
 
-// Which FP64 cell-block kernel runs, read once per process from PYLITH_B200_TET_KERNEL: "pad2" (the
-// default: two barriers per block over the padded layout), "pipe" (one barrier per block over the
+// Which FP64 kernel of this file runs, read once per process from PYLITH_B200_TET_KERNEL: "pad2" (also
+// where the variable is unset and the pairs of tetpair.cu do not serve the mesh: two barriers per block over the padded layout), "pipe" (one barrier per block over the
 // padded layout) or "twophase" (two barriers per block, per-thread 8-byte gathers of all node data).
 enum TetKernel { TK_PAD2, TK_PIPE, TK_TWOPHASE };
 static TetKernel tet_kernel_choice() {
@@ -1119,18 +1121,7 @@ bool launch_domain_jv32_blocked(const DomainParams& p, const BlockedLayout& b, i
     return true;
 }
 
-// Host: bank-aware numbering of one block's local nodes and order of their incidence sums.
-//
-// The kernels keep node values component-major in shared memory, so the bank pair of node i in
-// an FP64 array is i mod 16 (and the 16-byte bank group of an FP32 row of 28 floats is 7 i mod 8):
-// the 32 reads of one corner by a warp's 32 cells conflict when distinct nodes share an index
-// residue. Starting from the nodes sorted by global id, a local search over swaps of two nodes'
-// indices (deterministic, seeded by the block index) lowers the sum over (warp, corner) of the
-// largest number of distinct nodes on one residue. Within each residue class the nodes are then
-// placed by decreasing incidence count, so each warp of the per-node sums gets nodes of similar
-// counts and runs fewer steps. Finally each node's incidences are ordered, warp by warp and step
-// by step, so that the staged element entries read in one step (bank pair = cell mod 16) spread
-// over the banks. Any fixed order keeps the sums identical from run to run.
+// Host: one block's local nodes and incidences, numbered and ordered for the banks (bankplan.hpp).
 #ifndef PLB_PLAN_ITERS
 #define PLB_PLAN_ITERS 12000
 #endif
@@ -1143,51 +1134,8 @@ struct BlockPlan {
                                     // corner * 3 * kTetBlockCells + cell (padded-layout kernels)
 };
 
-// Orders each node's incidences (lists[k], entries cell * 4 + corner) so that the entries that
-// the lanes of one warp read in one step (bank pair = cell mod 16) spread over the banks; the
-// warp of node k is group(k) and its lanes run the group's nodes in increasing k. Returns the
-// per-node ordered lists.
-template <typename Group>
-static std::vector<std::vector<int>> order_for_banks(std::vector<std::vector<int>> lists, int ngroups, Group group) {
-    constexpr int R = 16;
-    const int nloc = (int)lists.size();
-    std::vector<std::vector<int>> members(ngroups), ordered(nloc);
-    for (int k = 0; k < nloc; ++k) members[group(k)].push_back(k);
-    for (const std::vector<int>& mem : members) {
-        const int nl = (int)mem.size();
-        if (nl == 0) continue;
-        std::vector<int> lanes(nl);
-        int depth = 0;
-        for (int k : mem) depth = std::max(depth, (int)lists[k].size());
-        for (int j = 0; j < depth; ++j) {
-            int c16[R] = {0};
-            for (int i = 0; i < nl; ++i) lanes[i] = i;
-            std::stable_sort(lanes.begin(), lanes.end(),
-                             [&](int x, int y) { return lists[mem[x]].size() > lists[mem[y]].size(); });
-            for (int i : lanes) {
-                std::vector<int>& L = lists[mem[i]];
-                if (L.empty()) continue;
-                size_t best = 0;
-                for (size_t t = 1; t < L.size(); ++t)
-                    if (c16[(L[t] >> 2) & (R - 1)] < c16[(L[best] >> 2) & (R - 1)]) best = t;
-                c16[(L[best] >> 2) & (R - 1)]++;
-                ordered[mem[i]].push_back(L[best]);
-                L.erase(L.begin() + best);
-            }
-        }
-    }
-    return ordered;
-}
-
-static uint64_t splitmix64(uint64_t& x) {
-    uint64_t z = (x += 0x9E3779B97F4A7C15ull);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    return z ^ (z >> 31);
-}
-
 static void plan_block(const int32_t* bc, int ncell, uint64_t seed, BlockPlan& P) {
-    constexpr int R = 16, W = 32, kIters = PLB_PLAN_ITERS;
+    constexpr int W = kWarp;
     P.loc.assign(bc, bc + 4 * (size_t)ncell);
     std::sort(P.loc.begin(), P.loc.end());
     P.loc.erase(std::unique(P.loc.begin(), P.loc.end()), P.loc.end());
@@ -1209,57 +1157,10 @@ static void plan_block(const int32_t* bc, int ncell, uint64_t seed, BlockPlan& P
             }
         }
     }
-    std::vector<int>& perm = P.newidx;
-    perm.resize(nloc);
-    for (int l = 0; l < nloc; ++l) perm[l] = l;
-    std::vector<int> cnt((size_t)ng * R, 0);
-    for (int l = 0; l < nloc; ++l)
-        for (int g : node_groups[l]) cnt[(size_t)g * R + (perm[l] & (R - 1))]++;
-    auto gmax = [&](int g) {
-        int m = 0;
-        for (int r = 0; r < R; ++r) m = std::max(m, cnt[(size_t)g * R + r]);
-        return m;
-    };
-    auto move = [&](int l, int from, int to) {
-        for (int g : node_groups[l]) {
-            cnt[(size_t)g * R + from]--;
-            cnt[(size_t)g * R + to]++;
-        }
-    };
-    std::vector<int> mark(ng, -1), aff;
-    uint64_t rs = seed;
-    for (int it = 0; it < kIters && nloc > 1; ++it) {
-        const int a = (int)(splitmix64(rs) % (uint64_t)nloc), b = (int)(splitmix64(rs) % (uint64_t)nloc);
-        const int ra = perm[a] & (R - 1), rb = perm[b] & (R - 1);
-        if (ra == rb) continue;
-        aff.clear();
-        for (int g : node_groups[a])
-            if (mark[g] != it) mark[g] = it, aff.push_back(g);
-        for (int g : node_groups[b])
-            if (mark[g] != it) mark[g] = it, aff.push_back(g);
-        int before = 0, after = 0;
-        for (int g : aff) before += gmax(g);
-        move(a, ra, rb);
-        move(b, rb, ra);
-        for (int g : aff) after += gmax(g);
-        if (after <= before) {
-            std::swap(perm[a], perm[b]);
-        } else {
-            move(a, rb, ra);
-            move(b, ra, rb);
-        }
-    }
-    // within each residue class: decreasing incidence count
     std::vector<int> deg(nloc, 0);
     for (int i = 0; i < 4 * ncell; ++i) deg[lcs[i]]++;
-    for (int r = 0; r < R; ++r) {
-        std::vector<int> nodes, slots;
-        for (int l = 0; l < nloc; ++l)
-            if ((perm[l] & (R - 1)) == r) nodes.push_back(l), slots.push_back(perm[l]);
-        std::sort(slots.begin(), slots.end());
-        std::stable_sort(nodes.begin(), nodes.end(), [&](int x, int y) { return deg[x] > deg[y]; });
-        for (size_t i = 0; i < nodes.size(); ++i) perm[nodes[i]] = slots[i];
-    }
+    std::vector<int32_t>& perm = P.newidx;
+    spread_nodes(node_groups, ng, deg, seed, PLB_PLAN_ITERS, perm);
     // incidences by new index, in (cell, corner) order, then ordered for the banks (the warps of
     // the node sums take 32 consecutive nodes)
     std::vector<std::vector<int>> lists(nloc);

@@ -414,6 +414,10 @@ int pl_mesh_set_cohesive(pl_mesh m, int64_t ncoh, const int32_t* coh, int64_t nl
         dev_free(m->blocked->d_slot_node_red, m->ctx->stream);
         m->blocked->d_slot_node_red = nullptr;
     }
+    if (m->pair) {
+        dev_free(m->pair->d_ids_red, m->ctx->stream);
+        m->pair->d_ids_red = nullptr;
+    }
     bump_state_epoch();  // captured solver graphs hold the reduced connectivity
     m->ncoh = ncoh;
     m->nlag = nlag;
@@ -434,6 +438,7 @@ static void mesh_free(pl_mesh m) {
     dev_free(m->d_coh, m->ctx->stream);
     dev_free(m->d_cells_red, m->ctx->stream);
     if (m->blocked) free_blocked_layout(m->blocked, m->ctx->stream);
+    free_pair_layout(m->pair, m->ctx->stream);
     delete m;
     if (--c->refs == 0 && c->destroy_requested) context_free(c);
 }
@@ -768,6 +773,29 @@ static bool use_blocked(pl_integrator ig) {
     return m->cell_type == PL_CELL_TET4 || ig->scatter == PL_SCATTER_BLOCKED || ig->scatter == PL_SCATTER_DETERMINISTIC;
 }
 
+// Whether the mesh's FP64 cell-block path runs on pairs of cells (after prepare_blocked).
+static bool uses_pairs(pl_mesh m) { return m->pair && m->pair->num_blocks > 0; }
+
+// The FP64 cell-block kernels (after prepare_blocked); false when they do not support the configuration.
+static bool apply_cells(pl_integrator ig, const DomainParams& p, int rheo, bool bf, int op, bool insert, bool reduced = false) {
+    pl_mesh m = ig->mesh;
+    cudaStream_t s = m->ctx->stream;
+    double* partial = !reduced && ig->scatter == PL_SCATTER_DETERMINISTIC ? ig->d_block_partial : nullptr;
+    if (uses_pairs(m)) return launch_domain_apply_pair(p, *m->pair, rheo, bf, op, insert, m->nnodes, partial, s, reduced);
+    return launch_domain_apply_blocked(p, *m->blocked, m->cell_type, rheo, bf, op, insert, m->nnodes, partial, s, reduced);
+}
+
+// The same for the FP32 action.
+static bool apply_cells_f32(pl_integrator ig, const DomainParams& p, int rheo, bool reduced = false) {
+    pl_mesh m = ig->mesh;
+    cudaStream_t s = m->ctx->stream;
+    if (uses_pairs(m)) return launch_domain_jv32_pair(p, *m->pair, rheo, s, reduced);
+    return launch_domain_jv32_blocked(p, *m->blocked, m->cell_type, rheo, m->nnodes, s, reduced);
+}
+
+// Reduced slot ids of the layout that apply_cells uses (after prepare_blocked and ensure_reduced_cells).
+static int ensure_cell_ids_reduced(pl_mesh m) { return uses_pairs(m) ? ensure_pair_reduced_ids(m) : ensure_reduced_ids(m); }
+
 // The reduced fault space's connectivity (each positive-side node replaced by its negative-side
 // partner) and node map. Refused (PL_ERR_UNSUPPORTED) when a pair's two nodes do not coincide:
 // the kernels then read the partner's coordinates in place of the node's own.
@@ -806,7 +834,7 @@ bool jacobian_action_reduced_supported(pl_integrator_s* ig) {
     if (ensure_reduced_cells(m) != PL_OK) return false;
     // the cell-block path of tetrahedra needs the reduced slot ids (built here, outside capture)
     if (use_blocked(ig) && m->cell_type == PL_CELL_TET4)
-        return prepare_blocked(ig) == PL_OK && ensure_reduced_ids(m) == PL_OK;
+        return prepare_blocked(ig) == PL_OK && ensure_cell_ids_reduced(m) == PL_OK;
     return true;
 }
 
@@ -828,10 +856,8 @@ int jacobian_action_reduced(pl_integrator_s* ig, double t, double dt, const doub
     p.dt = dt;
     if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(jv, 0, pl_mesh_num_dof(m) * sizeof(double), s));
     if (use_blocked(ig) && m->cell_type == PL_CELL_TET4) {
-        if ((rc = prepare_blocked(ig)) != PL_OK || (rc = ensure_reduced_ids(m)) != PL_OK) return rc;
-        if (!launch_domain_apply_blocked(p, *m->blocked, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, false, m->nnodes,
-                                         nullptr, s, true))
-            return PL_ERR_UNSUPPORTED;
+        if ((rc = prepare_blocked(ig)) != PL_OK || (rc = ensure_cell_ids_reduced(m)) != PL_OK) return rc;
+        if (!apply_cells(ig, p, rheo, false, OP_JACOBIAN_ACTION, false, true)) return PL_ERR_UNSUPPORTED;
     } else if (ig->scatter == PL_SCATTER_ATOMIC ||
                !launch_domain_apply_hexgroup(p, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, s)) {
         launch_domain_apply_atomic(p, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, s);
@@ -858,8 +884,8 @@ int jacobian_action_reduced_f32(pl_integrator_s* ig, double t, double dt, const 
         p.lm32 = ig->d_lm32;
     if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(jv, 0, pl_mesh_num_dof(m) * sizeof(float), s));
     if (use_blocked(ig) && m->cell_type == PL_CELL_TET4) {
-        if ((rc = ensure_blocked_layout(m)) != PL_OK || (rc = ensure_reduced_ids(m)) != PL_OK) return rc;
-        if (!launch_domain_jv32_blocked(p, *m->blocked, m->cell_type, rheo, m->nnodes, s, true)) return PL_ERR_UNSUPPORTED;
+        if ((rc = prepare_blocked(ig)) != PL_OK || (rc = ensure_cell_ids_reduced(m)) != PL_OK) return rc;
+        if (!apply_cells_f32(ig, p, rheo, true)) return PL_ERR_UNSUPPORTED;
     } else if (ig->scatter == PL_SCATTER_ATOMIC || !launch_domain_jv32_hexgroup(p, m->cell_type, rheo, s)) {
         launch_domain_jv_f32_atomic(p, m->cell_type, rheo, s);
     }
@@ -869,10 +895,12 @@ int jacobian_action_reduced_f32(pl_integrator_s* ig, double t, double dt, const 
 
 int prepare_blocked(pl_integrator_s* ig) {
     pl_mesh m = ig->mesh;
-    int rc = ensure_blocked_layout(m);
-    if (rc) return rc;
-    if (ig->scatter == PL_SCATTER_DETERMINISTIC && !ig->d_block_partial && m->blocked->num_slots > 0)
-        PLB_CUDA(dev_alloc(&ig->d_block_partial, 3 * m->blocked->num_slots));
+    int rc = PL_OK;
+    if (m->cell_type == PL_CELL_TET4 && tet_pairs_selected() && (rc = ensure_pair_layout(m)) != PL_OK) return rc;
+    if (!uses_pairs(m) && (rc = ensure_blocked_layout(m)) != PL_OK) return rc;
+    const int64_t slots = uses_pairs(m) ? m->pair->num_slots : m->blocked->num_slots;
+    if (ig->scatter == PL_SCATTER_DETERMINISTIC && !ig->d_block_partial && slots > 0)
+        PLB_CUDA(dev_alloc(&ig->d_block_partial, 3 * slots));
     return PL_OK;
 }
 }  // namespace plb
@@ -909,9 +937,7 @@ int pl_compute_lhs_residual(pl_integrator ig, double t, double dt, const double*
     p.t = t;
     p.dt = dt;
     if (use_blocked(ig) && (rc = prepare_blocked(ig)) == PL_OK &&
-        launch_domain_apply_blocked(p, *m->blocked, m->cell_type, rheo, bf, OP_RESIDUAL, mode == PL_INSERT,
-                                    m->nnodes, ig->scatter == PL_SCATTER_DETERMINISTIC ? ig->d_block_partial : nullptr,
-                                    s)) {
+        apply_cells(ig, p, rheo, bf, OP_RESIDUAL, mode == PL_INSERT)) {
         if (mode == PL_INSERT && m->nlag > 0)
             PLB_CUDA(cudaMemsetAsync(r + 3 * m->nnodes, 0, 3 * m->nlag * sizeof(double), s));
         PLB_CUDA(cudaGetLastError());
@@ -958,9 +984,7 @@ int pl_compute_lhs_jacobian_action(pl_integrator ig, double t, double dt, double
     p.dt = dt;
     p.s_tshift = s_tshift;
     if (use_blocked(ig) && (rc = prepare_blocked(ig)) == PL_OK &&
-        launch_domain_apply_blocked(p, *m->blocked, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, mode == PL_INSERT,
-                                    m->nnodes, ig->scatter == PL_SCATTER_DETERMINISTIC ? ig->d_block_partial : nullptr,
-                                    s)) {
+        apply_cells(ig, p, rheo, false, OP_JACOBIAN_ACTION, mode == PL_INSERT)) {
         if (mode == PL_INSERT && m->nlag > 0)
             PLB_CUDA(cudaMemsetAsync(jv + 3 * m->nnodes, 0, 3 * m->nlag * sizeof(double), s));
         PLB_CUDA(cudaGetLastError());
@@ -1004,8 +1028,7 @@ int pl_compute_lhs_jacobian_action_f32(pl_integrator ig, double t, double dt, co
     if ((m->cell_type == PL_CELL_HEX8 || m->cell_type == PL_CELL_TET4) && ig->lm32_valid && ig->lm32_t == t &&
         ig->lm32_dt == dt)
         p.lm32 = ig->d_lm32;
-    if (use_blocked(ig) && (rc = ensure_blocked_layout(m)) == PL_OK &&
-        launch_domain_jv32_blocked(p, *m->blocked, m->cell_type, rheo, m->nnodes, s)) {
+    if (use_blocked(ig) && (rc = prepare_blocked(ig)) == PL_OK && apply_cells_f32(ig, p, rheo)) {
         PLB_CUDA(cudaGetLastError());
         return PL_OK;
     }

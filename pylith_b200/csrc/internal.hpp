@@ -104,6 +104,24 @@ struct BlockedLayout {
     std::vector<int32_t> h_pipe_begin, h_block_node_begin;
 };
 
+// Cell-pair layout of a tetrahedral mesh (tetpair.cu; built once per mesh, num_blocks 0: not usable).
+struct PairLayout {
+    int64_t num_blocks = 0;
+    int ld = 0;                   // slots per block (constant stride)
+    int64_t num_slots = 0;        // num_blocks * ld
+    int32_t* d_nslots = nullptr;       // [num_blocks] used slots
+    uint32_t* d_ids = nullptr;         // [num_blocks][ld] node id | shared bit
+    uint32_t* d_ids_red = nullptr;     // as d_ids in the reduced fault space, built on first use
+    double* d_coords = nullptr;        // [num_blocks][3][ld]
+    uint16_t* d_off = nullptr;         // [num_blocks][ld + 8] slots + 1 incidence offsets
+    uint16_t* d_inc = nullptr;         // [num_blocks][5 * threads] staging offsets
+    uint32_t* d_items = nullptr;       // [num_blocks][threads][4]
+    // nodes not owned by exactly one block (in several or in no cell), with their slots in block order
+    int64_t num_fix = 0;
+    int32_t *d_fix_node = nullptr, *d_fix_off = nullptr, *d_fix_slot = nullptr;
+    std::vector<uint32_t> h_ids;  // host copy for the reduced slot ids
+};
+
 void context_retain(pl_context_s* c);
 void context_release(pl_context_s* c);
 void mesh_retain(pl_mesh_s* m);
@@ -149,6 +167,7 @@ struct pl_mesh_s {
     int32_t* d_coh = nullptr;
     std::vector<int32_t> h_coh;
     plb::BlockedLayout* blocked = nullptr;
+    plb::PairLayout* pair = nullptr;
     // The solvers' reduced fault space (each fault node's positive side follows its negative
     // side): the connectivity with every positive-side node replaced by its negative-side
     // partner, built on first use, and dropped when the cohesive cells change.

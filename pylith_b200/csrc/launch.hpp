@@ -60,6 +60,16 @@ void free_blocked_layout(BlockedLayout* b, cudaStream_t after);
 bool launch_domain_apply_blocked(const DomainParams& p, const BlockedLayout& b, int cell,
                                  int rheo, bool bf, int op, bool insert, int64_t nnodes, double* partial,
                                  cudaStream_t s, bool reduced = false);
+// The same on pairs of cells (tetpair.cu); returns false when the layout does not support the
+// configuration. The layout is built once per mesh; reduced slot ids as below.
+struct PairLayout;
+bool tet_pairs_selected();
+int ensure_pair_layout(pl_mesh_s* m);
+int ensure_pair_reduced_ids(pl_mesh_s* m);
+void free_pair_layout(PairLayout* L, cudaStream_t after);
+bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rheo, bool bf, int op, bool insert, int64_t nnodes,
+                              double* partial, cudaStream_t s, bool reduced = false);
+bool launch_domain_jv32_pair(const DomainParams& p, const PairLayout& L, int rheo, cudaStream_t s, bool reduced = false);
 // The padded layout's slot ids in the reduced fault space (mesh with faults, after
 // ensure_reduced_cells); call outside stream capture.
 int ensure_reduced_ids(pl_mesh_s* m);

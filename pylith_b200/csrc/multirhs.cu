@@ -1934,6 +1934,16 @@ int pl_batch_solver_create(pl_solver base, int tile, pl_batch_solver* out) {
     return PL_OK;
 }
 
+// The batched operator's layouts on S's mesh, with the slot ids of the reduced fault space where the
+// solver acts in it; outside any stream capture.
+static int prepare_multi_layout(pl_solver S) {
+    pl_mesh m = S->mesh;
+    int rc = ensure_blocked_layout(m);
+    if (rc == PL_OK && S->npairs > 0 && S->reduced && m->blocked->num_blocks > 0 && m->h_node_red.size() == (size_t)m->nnodes)
+        rc = ensure_reduced_ids(m);
+    return rc;
+}
+
 int pl_batch_solver_solve(pl_batch_solver B, int nrhs, const double* const* b_dev, double* const* x_dev) {
     if (!B || nrhs < 0 || (nrhs > 0 && (!b_dev || !x_dev))) return fail(PL_ERR_INVALID_ARG, "bad arguments");
     pl_solver S = B->base;
@@ -1946,13 +1956,14 @@ int pl_batch_solver_solve(pl_batch_solver B, int nrhs, const double* const* b_de
     PLB_CUDA(cudaEventRecord(B->ev_in, user));
     PLB_CUDA(cudaStreamWaitEvent(B->stream, B->ev_in, 0));
     c->stream = B->stream;
-    int rc = PL_OK;
-    if (nrhs > 0 && B->mg) {
+    int rc = nrhs > 0 ? prepare_multi_layout(S) : PL_OK;
+    if (rc == PL_OK && nrhs > 0 && B->mg) {
         // the hierarchy's eigenvalue estimates and dense coarsest inverse (made by its first solve
         // after a setup, or here)
         rc = multigrid_prepare(B->mg);
+        const MgView v = multigrid_view(B->mg);
+        for (size_t l = 0; rc == PL_OK && l < v.levels.size(); ++l) rc = prepare_multi_layout(v.levels[l].S);
         if (rc == PL_OK) {
-            const MgView v = multigrid_view(B->mg);
             bool changed = v.levels.size() != B->mgv.levels.size() || v.dense_inv32 != B->mgv.dense_inv32 ||
                            v.degree != B->mgv.degree || v.lower != B->mgv.lower ||
                            v.pre_smooth != B->mgv.pre_smooth || v.post_smooth != B->mgv.post_smooth;

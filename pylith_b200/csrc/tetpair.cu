@@ -1,0 +1,890 @@
+// P1 tetrahedra, residual and Jacobian actions: cell blocks of face-sharing pairs.
+//
+// As in blocked.cu a persistent CTA takes compact blocks of consecutive cells, stages the block's
+// nodes (coordinates and field) in shared memory one block ahead, forms element vectors in one phase
+// and sums them per node in the next; owned nodes are stored, shared ones reduced into the output.
+// That scheme is bound by shared-memory traffic: a cell reads 24 node values and its 12-entry element
+// vector is written and read again. Here a thread takes two tetrahedra that share a face: 30 node
+// values, 15 entries, five incidences for the pair, 60 % of the traffic, and the shared edges and
+// cross product are formed once. The host matches the cells of a block into pairs (98 % of them on
+// Delaunay and structured meshes); a cell left over takes a thread by itself.
+// Measured on B200 (L2 warm), residual or action against the one-cell-per-thread kernel k_tet_pad2:
+// 1,296,000 structured cells FP64 53.8 -> 45.4 us and FP32 45.8 -> 35.5; 54,737 Delaunay cells FP64
+// 9.5 -> 8.7, FP32 9.9 -> 8.7; 3,072 cells FP64 8.5 -> 6.7. What bounds it now: shared memory still
+// (reads of random nodes conflict about twofold after the numbering of bankplan.hpp), then HBM.
+// Block size: 240 cells in 128 items with 4 CTAs per SM (FP64, at most 128 registers) measured best
+// (two launches on 1,179,648 cells 80 us); 5 and 6 CTAs 80-92 (spills), 64, 96, 192 and 256 threads
+// 82-98, two lanes per node in the sums 89. FP32: 4, 5 and 6 CTAs 45.6, 40.1, 38.6 us.
+#include <cuda_pipeline.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+#include <queue>
+#include <thread>
+#include <vector>
+
+#include "bankplan.hpp"
+#include "domain_kernels.cuh"
+#include "internal.hpp"
+#include "launch.hpp"
+
+namespace plb {
+
+constexpr int kPairThreads = 128;    // items (pairs or single cells) of a block at most
+constexpr int kPairCells = 240;      // cells of a block at most: about 122 items
+constexpr int kPairMaxNodes = 2 * kPairThreads;  // nodes of a block at most (two per thread)
+constexpr int kPairSmallLd = 144;    // slots per block where all of a mesh's blocks fit (compact ones do)
+constexpr int kPairCtas = 4;         // resident CTAs per SM
+constexpr int kPairCtas32 = 6;       // of the FP32 action
+constexpr uint32_t kPairShared = 0x80000000u;
+constexpr uint32_t kNoNode = 0xffffffffu, kNoItem = 0xffffffffu;
+constexpr int kCellBias = 0x8000;
+
+// Per-block arrays have constant strides (LD slots per block), so their addresses need no loads.
+struct PairArrays {
+    const int32_t* nslots;      // [nblocks]
+    const uint32_t* ids;        // [nblocks][LD] node id | kPairShared (kNoNode past the block's nodes)
+    const double* coords;       // [nblocks][3][LD]
+    const uint16_t* off;        // [nblocks][LD + 8] nslots + 1 incidence offsets
+    const uint16_t* inc;        // [nblocks][5 * kPairThreads] staging offsets corner * 3 * threads + item
+    const uint4* items;         // [nblocks][kPairThreads] (see PairPlan)
+    double* partial;            // [nblocks][LD][3] deterministic partial sums
+    int64_t nblocks;
+};
+
+// Shared memory for blocks of at most LD nodes: element vectors [15][threads], two node buffers
+// (coordinates in FP64 and the field in T, component by component), two metadata buffers. LD is a
+// compile-time multiple of 16, so a node's six values sit at constant offsets.
+template <typename T, int LD>
+struct PairSmem {
+    T E[15 * kPairThreads];
+    struct Node {
+        double x[3 * LD];
+        T v[3 * LD];
+    } node[2];
+    struct Meta {
+        uint32_t ids[LD];
+        uint16_t off[LD + 8];
+        uint16_t inc[5 * kPairThreads];
+    } meta[2];
+};
+
+// This thread's slot ids of block b, and the block's slot count.
+template <int LD>
+PL_D void pair_load_ids(const PairArrays& A, int64_t b, uint32_t (&nd)[2], int& ns) {
+    nd[0] = nd[1] = kNoNode;
+    ns = 0;
+    if (b >= A.nblocks) return;
+    ns = A.nslots[b];
+    nd[0] = A.ids[b * LD + threadIdx.x];
+    if (threadIdx.x + kPairThreads < LD) nd[1] = A.ids[b * LD + threadIdx.x + kPairThreads];
+}
+
+// Asynchronous copies of block b (ids in nd and slot count ns read one block earlier): coordinates,
+// ids, offsets and incidences as aligned 16-byte runs, the field of its nodes one value at a time.
+template <typename T, int LD>
+PL_D void pair_stage(const T* __restrict__ field, const PairArrays& A, int64_t b, const uint32_t (&nd)[2], int ns,
+                     PairSmem<T, LD>& S, int buf) {
+    auto& node = S.node[buf];
+    auto& M = S.meta[buf];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+        if (nd[k] != kNoNode) {
+            const T* f = field + 3 * (int64_t)(nd[k] & ~kPairShared);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                __pipeline_memcpy_async(&node.v[d * LD + threadIdx.x + k * kPairThreads], f + d, sizeof(T));
+        }
+    const double* x = A.coords + b * 3 * LD;
+    if (2 * threadIdx.x < ns)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) __pipeline_memcpy_async(&node.x[d * LD + 2 * threadIdx.x], x + d * LD + 2 * threadIdx.x, 16);
+    if (4 * threadIdx.x < ns) __pipeline_memcpy_async(&M.ids[4 * threadIdx.x], &A.ids[b * LD + 4 * threadIdx.x], 16);
+    if (8 * threadIdx.x <= ns) __pipeline_memcpy_async(&M.off[8 * threadIdx.x], &A.off[b * (LD + 8) + 8 * threadIdx.x], 16);
+    if (threadIdx.x < 5 * kPairThreads / 8)
+        __pipeline_memcpy_async(&M.inc[8 * threadIdx.x], &A.inc[b * 5 * kPairThreads + 8 * threadIdx.x], 16);
+}
+
+PL_D uint4 pair_load_item(const PairArrays& A, int64_t b) {
+    return b < A.nblocks ? A.items[b * kPairThreads + threadIdx.x] : make_uint4(0, 0, 0, kNoItem);
+}
+PL_D bool pair_single(const uint4& it) { return it.z >> 16 == 0; }
+// The item's per-cell inputs, on their way to L2 (cell B lies near cell A).
+template <bool BF>
+PL_D void pair_prefetch_cells(const DomainParams& p, const uint4& it) {
+    if (it.w == kNoItem) return;
+    prefetch_l2(&p.mu[it.w]);
+    prefetch_l2(&p.K[it.w]);
+    if (BF)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) prefetch_l2(&p.body_force[d * p.ncells + it.w]);
+}
+// Per-cell inputs of the item's cells (a single cell's twice).
+template <typename L>
+PL_D void pair_load_cells(const DomainParams& p, const uint4& it, double (&aA)[L::size], double (&aB)[L::size]) {
+    if (it.w == kNoItem) return;
+    const int64_t cA = it.w, cB = pair_single(it) ? cA : cA + (int)(it.z >> 16) - kCellBias;
+    L::load_cell(p, cA, aA);
+    L::load_cell(p, cB, aB);
+}
+
+PL_D void cross3(const double (&a)[3], const double (&b)[3], double (&c)[3]) {
+    c[0] = a[1] * b[2] - a[2] * b[1];
+    c[1] = a[2] * b[0] - a[0] * b[2];
+    c[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+// One tetrahedron from its cofactor rows c0, c1, c2 (det J times the basis gradients of its corners
+// 1, 2, 3), det and the field differences g0, g1, g2 of those corners: v[k] = |K| f1 . grad(phi_{k+1})
+// (f1 C^T / 6), and, for the body force, bfw f0 (|K| / 4 times f0) in w.
+template <int RHEO, bool BF, int OP>
+PL_D void pair_tet(const DomainParams& p, const double* a, const double (&c0)[3], const double (&c1)[3], const double (&c2)[3],
+                   double det, const double (&g0)[3], const double (&g1)[3], const double (&g2)[3], double (&v)[3][3],
+                   double (&w)[3]) {
+    using L = AuxLayout<RHEO, BF>;
+    const AuxOffsets<RHEO, BF> aoff;
+    if (!(det > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
+    const double rdet = 1.0 / det;
+    double s_x[9], x[3] = {0, 0, 0}, s[3] = {0, 0, 0};
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s_x[c * 3 + d] = (g0[c] * c0[d] + g1[c] * c1[d] + g2[c] * c2[d]) * rdet;
+    double f0[3] = {0, 0, 0}, f1[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const double sixth = 1.0 / 6.0;
+    if (OP == OP_RESIDUAL) {
+        if (BF) {
+            const int sOff[1] = {0}, sOff_x[1] = {0};
+            pw::g0v_bodyforce<double>(3, 1, L::numA, sOff, sOff_x, s, nullptr, s_x, aoff.v, nullptr, a, nullptr, nullptr, p.t, x,
+                                      p.num_constants, p.constants, f0);
+            const double bfw = det * sixth * 0.25;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) w[c] = bfw * f0[c];
+        }
+        call_f1<RHEO>(L::numA, aoff.v, a, s, s_x, p, x, f1);
+    } else {
+        double Jf3[81];
+#pragma unroll
+        for (int i = 0; i < 81; ++i) Jf3[i] = 0.0;
+        call_jf3<RHEO>(L::numA, aoff.v, a, p, x, Jf3);
+        isotropic_jf3_contract<RHEO>(Jf3, s_x, f1);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        v[0][c] = (f1[3 * c] * c0[0] + f1[3 * c + 1] * c0[1] + f1[3 * c + 2] * c0[2]) * sixth;
+        v[1][c] = (f1[3 * c] * c1[0] + f1[3 * c + 1] * c1[1] + f1[3 * c + 2] * c1[2]) * sixth;
+        v[2][c] = (f1[3 * c] * c2[0] + f1[3 * c + 1] * c2[1] + f1[3 * c + 2] * c2[2]) * sixth;
+    }
+}
+
+// Differences of the item's nodes n1 .. n4 from n0: coordinates e, field g.
+template <typename T, int LD>
+PL_D void pair_edges(const uint4& it, const typename PairSmem<T, LD>::Node& node, double (&e)[4][3], T (&g)[4][3]) {
+    const int n[5] = {(int)(it.x & 0xffff), (int)(it.x >> 16), (int)(it.y & 0xffff), (int)(it.y >> 16), (int)(it.z & 0xffff)};
+    double x0[3];
+    T u0[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x0[d] = node.x[d * LD + n[0]], u0[d] = node.v[d * LD + n[0]];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            e[k][d] = node.x[d * LD + n[k + 1]] - x0[d];
+            g[k][d] = node.v[d * LD + n[k + 1]] - u0[d];
+        }
+}
+
+// The element vectors of one item into column E: tetrahedra (n0, n1, n2, n3) and, unless single,
+// (n0, n2, n1, n4).
+template <int RHEO, bool BF, int OP, int LD>
+PL_D void pair_item(const DomainParams& p, const uint4& it, const double* aA, const double* aB,
+                    const typename PairSmem<double, LD>::Node& node, double* E) {
+    double e[4][3], g[4][3];
+    pair_edges<double, LD>(it, node, e, g);
+    double n12[3], c0[3], c1[3], v[3][3], w[3] = {0, 0, 0}, r0[3], r1[3], r2[3];
+    cross3(e[0], e[1], n12);
+    cross3(e[1], e[2], c0);
+    cross3(e[2], e[0], c1);
+    double det = e[0][0] * c0[0] + e[0][1] * c0[1] + e[0][2] * c0[2];
+    pair_tet<RHEO, BF, OP>(p, aA, c0, c1, n12, det, g[0], g[1], g[2], v, w);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        r0[c] = w[c] - (v[0][c] + v[1][c] + v[2][c]);
+        r1[c] = v[0][c] + w[c];
+        r2[c] = v[1][c] + w[c];
+        E[(9 + c) * kPairThreads] = v[2][c] + w[c];
+    }
+    if (!pair_single(it)) {
+        double m[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) m[c] = -n12[c];
+        cross3(e[0], e[3], c0);  // of corner n2
+        cross3(e[3], e[1], c1);  // of corner n1
+        det = e[1][0] * c0[0] + e[1][1] * c0[1] + e[1][2] * c0[2];
+        pair_tet<RHEO, BF, OP>(p, aB, c0, c1, m, det, g[1], g[0], g[3], v, w);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            r0[c] += w[c] - (v[0][c] + v[1][c] + v[2][c]);
+            r2[c] += v[0][c] + w[c];
+            r1[c] += v[1][c] + w[c];
+            E[(12 + c) * kPairThreads] = v[2][c] + w[c];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        E[c * kPairThreads] = r0[c];
+        E[(3 + c) * kPairThreads] = r1[c];
+        E[(6 + c) * kPairThreads] = r2[c];
+    }
+}
+
+// One node's sum over its incidences j0 <= j < j1 of the staged element vectors.
+template <typename T>
+PL_D void pair_node_sum(const T* E, const uint16_t* inc, int j0, int j1, T (&r)[3]) {
+    r[0] = r[1] = r[2] = T(0);
+#pragma unroll 4
+    for (int j = j0; j < j1; ++j) {
+        const T* e = E + inc[j];
+        r[0] += e[0];
+        r[1] += e[kPairThreads];
+        r[2] += e[2 * kPairThreads];
+    }
+}
+
+// DET: a shared node's block sum goes to the partial-sum buffer for the fixup pass (bit-identical
+// results run to run); otherwise it is added into the output with an FP64 reduction (the output was
+// zeroed first for INSERT).
+template <int RHEO, bool BF, int OP, bool INSERT, bool DET, int LD>
+__global__ void __launch_bounds__(kPairThreads, kPairCtas) k_tet_pair(DomainParams p, PairArrays A) {
+    using L = AuxLayout<RHEO, BF>;
+    extern __shared__ __align__(16) char smem_raw[];
+    PairSmem<double, LD>& S = *reinterpret_cast<PairSmem<double, LD>*>(smem_raw);
+    const double* __restrict__ field = OP == OP_RESIDUAL ? p.u : p.v;
+    const int64_t G = gridDim.x;
+    int64_t b = blockIdx.x;
+    if (b >= A.nblocks) return;
+    uint32_t nd_next[2];
+    int ns, ns_next;
+    uint4 item = pair_load_item(A, b), item_next = pair_load_item(A, b + G);
+    double aA[L::size], aB[L::size];
+    {
+        uint32_t nd0[2];
+        pair_load_ids<LD>(A, b, nd0, ns);
+        pair_stage(field, A, b, nd0, ns, S, 0);
+        __pipeline_commit();
+        pair_load_ids<LD>(A, b + G, nd_next, ns_next);
+        pair_load_cells<L>(p, item, aA, aB);
+        pair_prefetch_cells<BF>(p, item_next);
+    }
+    for (int it = 0; b < A.nblocks; b += G, ++it) {
+        // what the next blocks need, so that no load of the loop waits for another or for HBM: the slot
+        // ids and the item two blocks ahead (its cells' inputs then start for L2, and are read between
+        // the two phases of the block before)
+        uint32_t nd_after[2];
+        int ns_after;
+        pair_load_ids<LD>(A, b + 2 * G, nd_after, ns_after);
+        const uint4 item_after = pair_load_item(A, b + 2 * G);
+        __pipeline_wait_prior(0);
+        // block b's copies have landed; every thread has finished the node sums of the previous block
+        // (its buffers are free for block b + G)
+        __syncthreads();
+        if (b + G < A.nblocks) pair_stage(field, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
+        __pipeline_commit();
+        nd_next[0] = nd_after[0], nd_next[1] = nd_after[1];
+        if (item.w != kNoItem) pair_item<RHEO, BF, OP, LD>(p, item, aA, aB, S.node[it & 1], S.E + threadIdx.x);
+        item = item_next, item_next = item_after;
+        pair_load_cells<L>(p, item, aA, aB);
+        pair_prefetch_cells<BF>(p, item_next);
+        __syncthreads();
+        const auto& M = S.meta[it & 1];
+        for (int k = threadIdx.x; k < ns; k += kPairThreads) {
+            const uint32_t id = M.ids[k];
+            double* o = p.out + 3 * (int64_t)(id & ~kPairShared);
+            double* pp = DET ? A.partial + 3 * (b * LD + k) : nullptr;
+            double r[3], old[3] = {0.0, 0.0, 0.0};
+            if (!INSERT && !(id & kPairShared))  // on its way while the sum runs (1 us of a 10 us launch)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) old[d] = o[d];
+            pair_node_sum(S.E, M.inc, M.off[k], M.off[k + 1], r);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if ((id & kPairShared) && DET) pp[d] = r[d];
+                else if (id & kPairShared) red_add(o + d, r[d]);
+                else o[d] = INSERT ? r[d] : old[d] + r[d];
+            }
+        }
+        ns = ns_next, ns_next = ns_after;
+    }
+    __pipeline_wait_prior(0);
+}
+
+// ---- FP32 Jacobian action --------------------------------------------------------------------
+// The isotropic tangent (lambda, mu) of the item's cells (a single cell's twice): the solver's cache
+// (p.lm32; CACHED) or the registered Jacobian kernel.
+template <bool CACHED>
+PL_D void pair_load_tangents(const DomainParams& p, const uint4& it, float2 (&lm)[2]) {
+    if (it.w == kNoItem) return;
+    const int64_t cells[2] = {(int64_t)it.w, pair_single(it) ? (int64_t)it.w : (int64_t)it.w + (int)(it.z >> 16) - kCellBias};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (CACHED) {
+            lm[k] = reinterpret_cast<const float2*>(p.lm32)[cells[k]];
+        } else {
+            using L = AuxLayout<RHEO_ILE, false>;
+            const AuxOffsets<RHEO_ILE, false> aoff;
+            double a[L::size], x[3] = {0, 0, 0}, Jf3[81];
+            L::load_cell(p, cells[k], a);
+#pragma unroll
+            for (int i = 0; i < 81; ++i) Jf3[i] = 0.0;
+            call_jf3<RHEO_ILE>(L::numA, aoff.v, a, p, x, Jf3);
+            lm[k] = make_float2((float)(-Jf3[((0 * 3 + 1) * 3 + 0) * 3 + 1]), (float)(-Jf3[((0 * 3 + 1) * 3 + 1) * 3 + 0]));
+        }
+    }
+}
+
+// pair_tet of the FP32 action: cofactors and det in FP64, gradient, flux and vectors in FP32.
+PL_D void pair_tet32(const DomainParams& p, float2 lm, const double (&c0)[3], const double (&c1)[3], const double (&c2)[3],
+                     double det, const float (&g0)[3], const float (&g1)[3], const float (&g2)[3], float (&v)[3][3]) {
+    if (!(det > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
+    const double rdet = 1.0 / det;
+    float inv[3][3], cf[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        inv[0][j] = (float)(c0[j] * rdet), cf[0][j] = (float)(c0[j] * (1.0 / 6.0));
+        inv[1][j] = (float)(c1[j] * rdet), cf[1][j] = (float)(c1[j] * (1.0 / 6.0));
+        inv[2][j] = (float)(c2[j] * rdet), cf[2][j] = (float)(c2[j] * (1.0 / 6.0));
+    }
+    float s[3][3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) s[c][d] = g0[c] * inv[0][d] + g1[c] * inv[1][d] + g2[c] * inv[2][d];
+    // flux f1 = -(lambda tr(e) I + 2 mu e), e = sym grad v
+    const float mu = lm.y, ltr = lm.x * (s[0][0] + s[1][1] + s[2][2]);
+    const float xy = -mu * (s[0][1] + s[1][0]), yz = -mu * (s[1][2] + s[2][1]), xz = -mu * (s[0][2] + s[2][0]);
+    const float f[3][3] = {{-(2.0f * mu * s[0][0] + ltr), xy, xz},
+                           {xy, -(2.0f * mu * s[1][1] + ltr), yz},
+                           {xz, yz, -(2.0f * mu * s[2][2] + ltr)}};
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[k][c] = f[c][0] * cf[k][0] + f[c][1] * cf[k][1] + f[c][2] * cf[k][2];
+}
+
+// FP32 Jacobian action of an isotropic tangent on the pairs (measured: head of the file), for the inner iterations of the
+// mixed-precision solvers: as k_tet_pair, with FP64 geometry and FP32 field, flux, element vectors
+// and sums. The output holds zero or the sum to add to.
+template <bool CACHED, int LD>
+__global__ void __launch_bounds__(kPairThreads, kPairCtas32) k_tet_pair_jv32(DomainParams p, PairArrays A) {
+    extern __shared__ __align__(16) char smem_raw[];
+    PairSmem<float, LD>& S = *reinterpret_cast<PairSmem<float, LD>*>(smem_raw);
+    const int64_t G = gridDim.x;
+    int64_t b = blockIdx.x;
+    if (b >= A.nblocks) return;
+    uint32_t nd_next[2];
+    int ns, ns_next;
+    uint4 item = pair_load_item(A, b), item_next = pair_load_item(A, b + G);
+    float2 lm[2];
+    {
+        uint32_t nd0[2];
+        pair_load_ids<LD>(A, b, nd0, ns);
+        pair_stage(p.v32, A, b, nd0, ns, S, 0);
+        __pipeline_commit();
+        pair_load_ids<LD>(A, b + G, nd_next, ns_next);
+        pair_load_tangents<CACHED>(p, item, lm);
+        if (CACHED && item_next.w != kNoItem) prefetch_l2(&p.lm32[2 * (int64_t)item_next.w]);
+    }
+    for (int it = 0; b < A.nblocks; b += G, ++it) {
+        uint32_t nd_after[2];
+        int ns_after;
+        pair_load_ids<LD>(A, b + 2 * G, nd_after, ns_after);
+        const uint4 item_after = pair_load_item(A, b + 2 * G);
+        __pipeline_wait_prior(0);
+        // as in k_tet_pair: block b has landed, and the buffers of block b + G are free
+        __syncthreads();
+        if (b + G < A.nblocks) pair_stage(p.v32, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
+        __pipeline_commit();
+        nd_next[0] = nd_after[0], nd_next[1] = nd_after[1];
+        if (item.w != kNoItem) {
+            float* E = S.E + threadIdx.x;
+            double e[4][3], n12[3], c0[3], c1[3];
+            float g[4][3], v[3][3], r0[3], r1[3], r2[3];
+            pair_edges<float, LD>(item, S.node[it & 1], e, g);
+            cross3(e[0], e[1], n12);
+            cross3(e[1], e[2], c0);
+            cross3(e[2], e[0], c1);
+            pair_tet32(p, lm[0], c0, c1, n12, e[0][0] * c0[0] + e[0][1] * c0[1] + e[0][2] * c0[2], g[0], g[1], g[2], v);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                r0[c] = -(v[0][c] + v[1][c] + v[2][c]);
+                r1[c] = v[0][c];
+                r2[c] = v[1][c];
+                E[(9 + c) * kPairThreads] = v[2][c];
+            }
+            if (!pair_single(item)) {
+                double m[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) m[c] = -n12[c];
+                cross3(e[0], e[3], c0);
+                cross3(e[3], e[1], c1);
+                pair_tet32(p, lm[1], c0, c1, m, e[1][0] * c0[0] + e[1][1] * c0[1] + e[1][2] * c0[2], g[1], g[0], g[3], v);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    r0[c] -= v[0][c] + v[1][c] + v[2][c];
+                    r2[c] += v[0][c];
+                    r1[c] += v[1][c];
+                    E[(12 + c) * kPairThreads] = v[2][c];
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                E[c * kPairThreads] = r0[c];
+                E[(3 + c) * kPairThreads] = r1[c];
+                E[(6 + c) * kPairThreads] = r2[c];
+            }
+        }
+        item = item_next, item_next = item_after;
+        pair_load_tangents<CACHED>(p, item, lm);
+        if (CACHED && item_next.w != kNoItem) prefetch_l2(&p.lm32[2 * (int64_t)item_next.w]);
+        __syncthreads();
+        const auto& M = S.meta[it & 1];
+        for (int k = threadIdx.x; k < ns; k += kPairThreads) {
+            const uint32_t id = M.ids[k];
+            float* o = p.out32 + 3 * (int64_t)(id & ~kPairShared);
+            float r[3], old[3] = {0.f, 0.f, 0.f};
+            if (!(id & kPairShared))
+#pragma unroll
+                for (int d = 0; d < 3; ++d) old[d] = o[d];
+            pair_node_sum(S.E, M.inc, M.off[k], M.off[k + 1], r);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (id & kPairShared) red_add(o + d, r[d]);
+                else o[d] = old[d] + r[d];
+            }
+        }
+        ns = ns_next, ns_next = ns_after;
+    }
+    __pipeline_wait_prior(0);
+}
+
+// Second pass of the deterministic mode: every node that is not owned by exactly one block gets the
+// sum of its blocks' partial sums, in block order (nodes in no cell get zero).
+template <bool INSERT>
+__global__ void k_pair_fixup(double* __restrict__ out, const double* __restrict__ partial, const int32_t* __restrict__ fix_node,
+                             const int32_t* __restrict__ fix_off, const int32_t* __restrict__ fix_slot, int64_t nfix) {
+    for (int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; f < nfix; f += (int64_t)gridDim.x * blockDim.x) {
+        double r[3] = {0.0, 0.0, 0.0};
+        for (int j = fix_off[f]; j < fix_off[f + 1]; ++j)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) r[d] += partial[3 * (int64_t)fix_slot[j] + d];
+        double* o = out + 3 * (int64_t)fix_node[f];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) o[d] = INSERT ? r[d] : o[d] + r[d];
+    }
+}
+
+// ---- host: layout ------------------------------------------------------------------------------
+namespace {
+
+struct PairPlan {
+    std::vector<int32_t> loc;       // global ids of the local nodes, by local index
+    // {n0 | n1 << 16, n2 | n3 << 16, n4 | (B - A + kCellBias) << 16, A}: local node indices, cells A and
+    // B (single cells: upper half of the third word 0)
+    std::vector<uint32_t> items;    // [nitems][4]
+    std::vector<uint16_t> off, inc;
+};
+
+struct Item {
+    int a, b;       // cells of the block (b = -1: single)
+    int32_t n[5];   // local node of each corner (n[4] = n[0] for a single)
+};
+
+// Corner order of cell v with corner k last that keeps its orientation.
+void apex_last(const int* v, int k, int32_t (&out)[4]) {
+    int m = 0;
+    for (int i = 0; i < 4; ++i)
+        if (i != k) out[m++] = v[i];
+    out[3] = v[k];
+    if ((3 - k) & 1) std::swap(out[0], out[1]);
+}
+
+// Face-sharing pairs of the block's cells (local connectivity lc): a maximal matching that takes the
+// cells with the fewest free neighbours first. Pairs whose orientations do not fit (cells that are
+// not consistently oriented across the face) stay single.
+std::vector<Item> match_cells(const std::vector<int>& lc, int ncell) {
+    struct Face {
+        uint64_t key;
+        int cell, k;
+    };
+    std::vector<Face> faces;
+    faces.reserve(4 * (size_t)ncell);
+    for (int c = 0; c < ncell; ++c)
+        for (int k = 0; k < 4; ++k) {
+            int f[3], m = 0;
+            for (int i = 0; i < 4; ++i)
+                if (i != k) f[m++] = lc[4 * c + i];
+            std::sort(f, f + 3);
+            faces.push_back({(uint64_t)f[0] << 40 | (uint64_t)f[1] << 20 | (uint64_t)f[2], c, k});
+        }
+    std::sort(faces.begin(), faces.end(), [](const Face& x, const Face& y) {
+        return x.key != y.key ? x.key < y.key : (x.cell != y.cell ? x.cell < y.cell : x.k < y.k);
+    });
+    struct Edge {
+        int cell, k, k2;  // neighbour, this cell's and its corner off the face
+    };
+    std::vector<std::vector<Edge>> adj(ncell);
+    for (size_t i = 0; i + 1 < faces.size(); ++i)
+        if (faces[i].key == faces[i + 1].key && faces[i].cell != faces[i + 1].cell) {
+            adj[faces[i].cell].push_back({faces[i + 1].cell, faces[i].k, faces[i + 1].k});
+            adj[faces[i + 1].cell].push_back({faces[i].cell, faces[i + 1].k, faces[i].k});
+        }
+    std::vector<int> deg(ncell);
+    std::vector<char> used(ncell, 0);
+    using Q = std::pair<int, int>;
+    std::priority_queue<Q, std::vector<Q>, std::greater<Q>> heap;
+    for (int c = 0; c < ncell; ++c) heap.push({deg[c] = (int)adj[c].size(), c});
+    std::vector<Item> items;
+    auto drop = [&](int c) {
+        used[c] = 1;
+        for (const Edge& e : adj[c])
+            if (!used[e.cell]) heap.push({--deg[e.cell], e.cell});
+    };
+    while (!heap.empty()) {
+        const auto [d, c] = heap.top();
+        heap.pop();
+        if (used[c] || d != deg[c]) continue;
+        const Edge* best = nullptr;
+        int32_t A[4], B[4];
+        for (const Edge& e : adj[c]) {
+            if (used[e.cell] || (best && deg[e.cell] >= deg[best->cell])) continue;
+            // cell c as (n0, n1, n2, n3); the other must be an even permutation of (n0, n2, n1, n4)
+            int32_t x[4], y[4];
+            apex_last(&lc[4 * c], e.k, x);
+            apex_last(&lc[4 * e.cell], e.k2, y);
+            bool fits = false;
+            for (int r = 0; r < 3; ++r) fits = fits || (y[r] == x[0] && y[(r + 1) % 3] == x[2] && y[(r + 2) % 3] == x[1]);
+            if (!fits) continue;
+            best = &e;
+            std::copy(x, x + 4, A);
+            std::copy(y, y + 4, B);
+        }
+        Item it;
+        it.a = c;
+        if (best) {
+            it.b = best->cell;
+            for (int i = 0; i < 4; ++i) it.n[i] = A[i];
+            it.n[4] = B[3];
+            const int other = best->cell;
+            drop(c);
+            drop(other);
+        } else {
+            it.b = -1;
+            for (int i = 0; i < 4; ++i) it.n[i] = lc[4 * c + i];
+            it.n[4] = it.n[0];
+            drop(c);
+        }
+        items.push_back(it);
+    }
+    std::sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.a < y.a; });
+    return items;
+}
+
+// Plans one block of the cells c0 .. c0 + ncell - 1 (connectivity bc[ncell][4]); false when they need more items or nodes than a block has.
+bool plan_pair_block(const int32_t* bc, int64_t c0, int ncell, PairPlan& P) {
+    std::vector<int32_t> sorted(bc, bc + 4 * (size_t)ncell);
+    std::sort(sorted.begin(), sorted.end());
+    sorted.erase(std::unique(sorted.begin(), sorted.end()), sorted.end());
+    const int nloc = (int)sorted.size();
+    if (nloc > kPairMaxNodes) return false;
+    std::vector<int> lc(4 * (size_t)ncell);
+    for (int i = 0; i < 4 * ncell; ++i) lc[i] = (int)(std::lower_bound(sorted.begin(), sorted.end(), bc[i]) - sorted.begin());
+    const std::vector<Item> items = match_cells(lc, ncell);
+    const int ni = (int)items.size();
+    if (ni > kPairThreads) return false;
+    std::vector<std::vector<int>> groups(nloc);
+    std::vector<int> deg(nloc, 0);
+    for (int i = 0; i < ni; ++i)
+        for (int k = 0; k < (items[i].b < 0 ? 4 : 5); ++k) {
+            const int l = items[i].n[k], g = i / kWarp * 5 + k;
+            deg[l]++;
+            if (groups[l].empty() || std::find(groups[l].begin(), groups[l].end(), g) == groups[l].end()) groups[l].push_back(g);
+        }
+    std::vector<int32_t> perm;
+    spread_nodes(groups, (ni + kWarp - 1) / kWarp * 5, deg, (uint64_t)c0, 8000, perm);
+    P.loc.resize(nloc);
+    for (int l = 0; l < nloc; ++l) P.loc[perm[l]] = sorted[l];
+    std::vector<std::vector<int>> lists(nloc);
+    P.items.clear();
+    for (int i = 0; i < ni; ++i) {
+        uint32_t n[5];
+        for (int k = 0; k < 5; ++k) {
+            n[k] = (uint32_t)perm[items[i].n[k]];
+            if (k < 4 || items[i].b >= 0) lists[n[k]].push_back(8 * i + k);
+        }
+        const uint32_t db = items[i].b < 0 ? 0u : (uint32_t)(items[i].b - items[i].a + kCellBias);
+        for (uint32_t w : {n[0] | n[1] << 16, n[2] | n[3] << 16, n[4] | db << 16, (uint32_t)(c0 + items[i].a)}) P.items.push_back(w);
+    }
+    const auto ordered = order_for_banks(lists, (nloc + kWarp - 1) / kWarp, [](int k) { return k / kWarp; }, 3);
+    P.off.assign(1, 0);
+    P.inc.clear();
+    for (int k = 0; k < nloc; ++k) {
+        for (int e : ordered[k]) P.inc.push_back((uint16_t)((e & 7) * 3 * kPairThreads + (e >> 3)));
+        P.off.push_back((uint16_t)P.inc.size());
+    }
+    return true;
+}
+
+// Blocks of the cells [begin, end): as even as kPairCells allows, a block that does not fit shrunk.
+bool plan_pair_range(const int32_t* cells, int64_t begin, int64_t end, std::vector<PairPlan>& out) {
+    for (int64_t c = begin; c < end;) {
+        const int64_t left = end - c, nb = (left + kPairCells - 1) / kPairCells;
+        int n = (int)((left + nb - 1) / nb);
+        PairPlan P;
+        while (!plan_pair_block(cells + 4 * c, c, n, P)) {
+            if (n <= kPairCells / 2) return false;  // scattered cells: see ensure_pair_layout
+            n -= std::max(2, n / 16);
+        }
+        out.push_back(std::move(P));
+        c += n;
+    }
+    return true;
+}
+
+int build_pair_layout(pl_mesh_s* m) {
+    PairLayout* L = new PairLayout();
+    m->pair = L;  // empty: not used for this mesh
+    if (m->cell_type != PL_CELL_TET4 || m->nnodes >= (int64_t)kPairShared || m->ncells >= (int64_t)INT32_MAX) return PL_OK;
+    // ranges of up to 16 blocks, planned in parallel (a range's plan depends only on its cells; the
+    // calling thread takes ranges too, so the layout is complete even where no helper thread can be
+    // started)
+    const int64_t nc = m->ncells, want = (nc + kPairCells - 1) / kPairCells;
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>(16, want / 64)), nr = (want + per - 1) / per;
+    std::vector<std::vector<PairPlan>> plans(nr);
+    std::atomic<int64_t> next{0};
+    std::atomic<bool> failed{false}, refused{false};
+    auto work = [&]() noexcept {
+        try {
+            for (int64_t r; !failed.load() && !refused.load() && (r = next.fetch_add(1)) < nr;)
+                if (!plan_pair_range(m->h_cells.data(), r * nc / nr, (r + 1) * nc / nr, plans[r])) refused.store(true);
+        } catch (...) {
+            failed.store(true);
+        }
+    };
+    const int nth = (int)std::min<int64_t>(std::min(15u, std::thread::hardware_concurrency()), nr);
+    std::vector<std::thread> th;
+    try {
+        for (int t = 1; t < nth; ++t) th.emplace_back(work);
+    } catch (...) {
+    }
+    work();
+    for (std::thread& x : th) x.join();
+    if (failed.load()) return fail(PL_ERR_OUT_OF_MEMORY, "cell-pair layout planning ran out of host memory");
+    if (refused.load()) return PL_OK;
+    int maxloc = 0;
+    int64_t nb = 0;
+    for (const std::vector<PairPlan>& range : plans)
+        for (const PairPlan& P : range) maxloc = std::max(maxloc, (int)P.loc.size()), ++nb;
+    const size_t LD = maxloc <= kPairSmallLd ? kPairSmallLd : kPairMaxNodes;
+    std::vector<int32_t> nslots(nb), nblocks_of(m->nnodes, 0);
+    std::vector<uint32_t> ids(nb * LD, kNoNode), items((size_t)nb * 4 * kPairThreads, kNoItem);
+    std::vector<double> coords(nb * 3 * LD, 0.0);
+    std::vector<uint16_t> off(nb * (LD + 8), 0), inc((size_t)nb * 5 * kPairThreads, 0);
+    size_t b = 0;
+    for (std::vector<PairPlan>& range : plans)
+        for (PairPlan& P : range) {
+            nslots[b] = (int32_t)P.loc.size();
+            for (int i = 0; i < nslots[b]; ++i) {
+                ids[b * LD + i] = (uint32_t)P.loc[i];
+                nblocks_of[P.loc[i]]++;
+                for (int d = 0; d < 3; ++d) coords[(3 * b + d) * LD + i] = m->h_coords[3 * (size_t)P.loc[i] + d];
+            }
+            std::copy(P.off.begin(), P.off.end(), off.begin() + b * (LD + 8));
+            std::copy(P.inc.begin(), P.inc.end(), inc.begin() + b * 5 * kPairThreads);
+            std::copy(P.items.begin(), P.items.end(), items.begin() + b * 4 * kPairThreads);
+            ++b;
+            P = PairPlan();
+        }
+    // nodes not owned by exactly one block, with their slots in block order
+    std::vector<int32_t> fix_node, fix_off(1, 0), fix_slot, first(m->nnodes + 1, 0);
+    for (uint32_t& id : ids)
+        if (id != kNoNode && nblocks_of[id] > 1) {
+            first[id + 1]++;
+            id |= kPairShared;
+        }
+    for (int64_t v = 0; v < m->nnodes; ++v) first[v + 1] += first[v];
+    std::vector<int32_t> slots(first[m->nnodes]), pos(first.begin(), first.end() - 1);
+    for (size_t at = 0; at < ids.size(); ++at)
+        if (ids[at] != kNoNode && (ids[at] & kPairShared)) slots[pos[ids[at] & ~kPairShared]++] = (int32_t)at;
+    for (int64_t v = 0; v < m->nnodes; ++v) {
+        if (nblocks_of[v] == 1) continue;
+        fix_node.push_back((int32_t)v);
+        fix_slot.insert(fix_slot.end(), slots.begin() + first[v], slots.begin() + first[v + 1]);
+        fix_off.push_back((int32_t)fix_slot.size());
+    }
+    cudaStream_t s = m->ctx->stream;
+    cudaError_t e = cudaSuccess;
+    auto up = [&](auto** dst, const auto& v) {
+        if (e != cudaSuccess || v.empty()) return;
+        const size_t bytes = v.size() * sizeof(v[0]);
+        e = dev_alloc((void**)dst, bytes);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(*dst, v.data(), bytes, cudaMemcpyHostToDevice, s);
+    };
+    up(&L->d_nslots, nslots);
+    up(&L->d_ids, ids);
+    up(&L->d_coords, coords);
+    up(&L->d_off, off);
+    up(&L->d_inc, inc);
+    up(&L->d_items, items);
+    up(&L->d_fix_node, fix_node);
+    up(&L->d_fix_off, fix_off);
+    up(&L->d_fix_slot, fix_slot);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(e, "cell-pair layout upload");
+    L->num_slots = (int64_t)ids.size();
+    L->num_fix = (int64_t)fix_node.size();
+    L->ld = (int)LD;
+    L->h_ids.swap(ids);
+    L->num_blocks = nb;
+    return PL_OK;
+}
+
+PairArrays arrays_of(const PairLayout& L, double* partial, bool reduced) {
+    PairArrays A;
+    A.nslots = L.d_nslots;
+    A.ids = reduced ? L.d_ids_red : L.d_ids;
+    A.coords = L.d_coords;
+    A.off = L.d_off;
+    A.inc = L.d_inc;
+    A.items = (const uint4*)L.d_items;
+    A.partial = partial;
+    A.nblocks = L.num_blocks;
+    return A;
+}
+
+template <typename T, int LD, typename Kernel>
+void launch_pairs(Kernel kern, const DomainParams& p, const PairArrays& A, cudaStream_t s) {
+    constexpr size_t smem = sizeof(PairSmem<T, LD>);
+    ensure_kernel_smem((const void*)kern, smem);
+    kern<<<(unsigned)std::min<int64_t>(A.nblocks, (int64_t)sm_count() * (sizeof(T) == 4 ? kPairCtas32 : kPairCtas)), kPairThreads, smem, s>>>(p, A);
+    count_launch();
+}
+
+template <bool BF, int OP, bool INSERT, bool DET>
+void launch_one(const DomainParams& p, const PairLayout& L, const PairArrays& A, cudaStream_t s) {
+    if (L.ld == kPairSmallLd) launch_pairs<double, kPairSmallLd>(k_tet_pair<RHEO_ILE, BF, OP, INSERT, DET, kPairSmallLd>, p, A, s);
+    else launch_pairs<double, kPairMaxNodes>(k_tet_pair<RHEO_ILE, BF, OP, INSERT, DET, kPairMaxNodes>, p, A, s);
+}
+
+template <bool CACHED>
+void launch_jv32(const DomainParams& p, const PairLayout& L, const PairArrays& A, cudaStream_t s) {
+    if (L.ld == kPairSmallLd) launch_pairs<float, kPairSmallLd>(k_tet_pair_jv32<CACHED, kPairSmallLd>, p, A, s);
+    else launch_pairs<float, kPairMaxNodes>(k_tet_pair_jv32<CACHED, kPairMaxNodes>, p, A, s);
+}
+
+template <bool BF, int OP>
+void launch_op(const DomainParams& p, const PairLayout& L, bool insert, double* partial, bool reduced, cudaStream_t s) {
+    const PairArrays A = arrays_of(L, partial, reduced);
+    if (partial && insert) launch_one<BF, OP, true, true>(p, L, A, s);
+    else if (partial) launch_one<BF, OP, false, true>(p, L, A, s);
+    else if (insert) launch_one<BF, OP, true, false>(p, L, A, s);
+    else launch_one<BF, OP, false, false>(p, L, A, s);
+    if (partial && L.num_fix > 0) {
+        const int g = (int)std::min<int64_t>((L.num_fix + 255) / 256, 148 * 8);
+        if (insert) k_pair_fixup<true><<<g, 256, 0, s>>>(p.out, partial, L.d_fix_node, L.d_fix_off, L.d_fix_slot, L.num_fix);
+        else k_pair_fixup<false><<<g, 256, 0, s>>>(p.out, partial, L.d_fix_node, L.d_fix_off, L.d_fix_slot, L.num_fix);
+        count_launch();
+    }
+}
+
+}  // namespace
+
+// PYLITH_B200_TET_KERNEL, read once per process: "pair" (the default) or a cell-block kernel of
+// blocked.cu.
+bool tet_pairs_selected() {
+    static const bool on = [] {
+        const char* v = std::getenv("PYLITH_B200_TET_KERNEL");
+        return !v || (std::strcmp(v, "pad2") != 0 && std::strcmp(v, "pipe") != 0 && std::strcmp(v, "twophase") != 0);
+    }();
+    return on;
+}
+
+// The mesh's pair layout (num_blocks 0: not usable). Meshes whose consecutive cells are scattered, so
+// that a block of kPairCells / 2 of them does not fit, keep the layout of single cells: 384,000 cells
+// shuffled throughout run 48.0 us there and 52.2 here (first call 252 and 386 ms); in their own order
+// 27.6 and 23.5 (235 and 132 ms).
+int ensure_pair_layout(pl_mesh_s* m) {
+    if (m->pair) return PL_OK;
+    int rc;
+    try {
+        rc = build_pair_layout(m);
+    } catch (const std::bad_alloc&) {
+        rc = fail(PL_ERR_OUT_OF_MEMORY, "cell-pair layout: out of host memory");
+    } catch (...) {
+        rc = fail(PL_ERR_INVALID_ARG, "cell-pair layout failed");
+    }
+    if (rc) {
+        free_pair_layout(m->pair, m->ctx->stream);
+        m->pair = nullptr;
+    }
+    return rc;
+}
+
+int ensure_pair_reduced_ids(pl_mesh_s* m) {
+    PairLayout* L = m->pair;
+    if (!L || L->num_blocks == 0) return fail(PL_ERR_UNSUPPORTED, "no cell-pair layout");
+    if (L->d_ids_red) return PL_OK;
+    if (m->h_node_red.size() != (size_t)m->nnodes) return fail(PL_ERR_UNSUPPORTED, "no reduced fault space");
+    // a node of the reduced space is owned by its block only if it has one slot in all blocks
+    std::vector<uint32_t> ids(L->h_ids.size(), 0u);
+    std::vector<int32_t> slots(m->nnodes, 0);
+    for (size_t at = 0; at < ids.size(); ++at)
+        ids[at] = L->h_ids[at] == kNoNode ? kNoNode : (uint32_t)m->h_node_red[L->h_ids[at] & ~kPairShared];
+    for (uint32_t id : ids)
+        if (id != kNoNode) slots[id]++;
+    for (uint32_t& id : ids)
+        if (id != kNoNode && slots[id] > 1) id |= kPairShared;
+    uint32_t* d = nullptr;
+    PLB_CUDA(dev_alloc(&d, ids.size()));
+    cudaError_t e = cudaMemcpyAsync(d, ids.data(), ids.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, m->ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(m->ctx->stream);
+    if (e != cudaSuccess) {
+        dev_free(d, m->ctx->stream);
+        return cuda_fail(e, "reduced slot ids");
+    }
+    L->d_ids_red = d;
+    return PL_OK;
+}
+
+bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rheo, bool bf, int op, bool insert, int64_t nnodes,
+                              double* partial, cudaStream_t s, bool reduced) {
+    if (rheo != RHEO_ILE || L.num_blocks == 0 || (reduced && (insert || partial || !L.d_ids_red))) return false;
+    // INSERT without partial sums: shared nodes are reduced into zeros
+    if (insert && !partial && L.num_fix > 0)
+        if (cudaMemsetAsync(p.out, 0, 3 * nnodes * sizeof(double), s) != cudaSuccess) return false;
+    if (op != OP_RESIDUAL) launch_op<false, OP_JACOBIAN_ACTION>(p, L, insert, partial, reduced, s);
+    else if (bf) launch_op<true, OP_RESIDUAL>(p, L, insert, partial, reduced, s);
+    else launch_op<false, OP_RESIDUAL>(p, L, insert, partial, reduced, s);
+    return true;
+}
+
+// The FP32 action; with the solver's cached tangent any isotropic rheology.
+bool launch_domain_jv32_pair(const DomainParams& p, const PairLayout& L, int rheo, cudaStream_t s, bool reduced) {
+    if ((rheo != RHEO_ILE && !p.lm32) || L.num_blocks == 0 || (reduced && !L.d_ids_red)) return false;
+    const PairArrays A = arrays_of(L, nullptr, reduced);
+    if (p.lm32) launch_jv32<true>(p, L, A, s);
+    else launch_jv32<false>(p, L, A, s);
+    return true;
+}
+
+void free_pair_layout(PairLayout* L, cudaStream_t after) {
+    if (!L) return;
+    for (void* p : {(void*)L->d_nslots, (void*)L->d_ids, (void*)L->d_ids_red,
+                    (void*)L->d_coords, (void*)L->d_off, (void*)L->d_inc, (void*)L->d_items, (void*)L->d_fix_node,
+                    (void*)L->d_fix_off, (void*)L->d_fix_slot})
+        dev_free(p, after);
+    delete L;
+}
+
+}  // namespace plb

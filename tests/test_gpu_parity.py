@@ -751,3 +751,54 @@ def test_cohesive_kernel_sizes(oracle_lib, torch_cuda, ctx, ny, nz):
     assert rel_l2(dr.cpu().numpy(), r_ref) <= TOL64
     assert rel_l2(djv.cpu().numpy(), jv_ref) <= TOL64
     assert rel_l2(d32.double().cpu().numpy(), jv_ref) <= 1e-5
+
+
+# one cell; one pair; one more than an item's two; one less than, exactly and one more than a block of
+# pairs; several blocks; mixed within windows (more nodes per block than consecutive cells have); mixed
+# throughout (the layout of single cells)
+@pytest.mark.parametrize("nc,window", [(1, 0), (2, 0), (3, 0), (239, 0), (240, 0), (241, 0), (1296, 0), (1296, 432), (1296, 1296)])
+def test_tet_pair_kernel_sizes(oracle_lib, torch_cuda, ctx, nc, window):
+    """The tetrahedral kernels on pairs of cells at item and block edges and for mixed cell orders:
+    residual with body force (INSERT and ADD), action, FP32 action and the deterministic mode; nodes
+    outside the first nc cells belong to no cell."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    rng = np.random.default_rng(17)
+    mesh = M.box_tet_kuhn(6, 6, 6)
+    mesh.cells = mesh.cells[:nc].copy()
+    for i in range(0, nc if window else 0, window or 1):
+        rng.shuffle(mesh.cells[i:i + window])
+    mat = elastic_setup(mesh, seed=18, body_force=True)
+    aux = oracle_aux(O, mat)
+    plain = O.AuxFields([(a[:, None], "cell") for a in (mat.density, mat.shear_modulus, mat.bulk_modulus)])
+    u = rng.standard_normal(mesh.num_nodes * 3)
+    r_ref = O.residual(mesh, u, aux, f0="Elasticity::g0v_bodyforce", f1=F1_ILE)
+    jv_ref = O.jacobian_action(mesh, u, plain, g3=JF3_ILE)
+    ig = mat.create_integrator(FA.DeviceMesh(ctx, mesh))
+    du = dev(torch, u)
+    dr, djv, d32 = torch.full_like(du, np.nan), torch.full_like(du, np.nan), torch.full_like(du.float(), np.nan)
+    ig.compute_lhs_residual(0.0, 0.0, du, dr)
+    ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, djv)
+    ig.compute_lhs_jacobian_action_f32(0.0, 0.0, du.float(), d32)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), r_ref) <= TOL64
+    assert rel_l2(djv.cpu().numpy(), jv_ref) <= TOL64
+    assert rel_l2(d32.double().cpu().numpy(), jv_ref) <= 1e-5
+    ig.compute_lhs_residual(0.0, 0.0, du, dr, mode=FA.ADD)
+    ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, djv, mode=FA.ADD)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), 2 * r_ref) <= TOL64
+    assert rel_l2(djv.cpu().numpy(), 2 * jv_ref) <= TOL64
+    ig.set_scatter(FA.SCATTER_DETERMINISTIC)
+    runs = []
+    for _ in range(2):
+        dr.fill_(np.nan)
+        ig.compute_lhs_residual(0.0, 0.0, du, dr)
+        ctx.synchronize()
+        runs.append(dr.cpu().numpy())
+    assert np.array_equal(runs[0], runs[1])
+    assert rel_l2(runs[0], r_ref) <= TOL64
+    ig.compute_lhs_residual(0.0, 0.0, du, dr, mode=FA.ADD)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), 2 * r_ref) <= TOL64
