@@ -773,9 +773,6 @@ static bool use_blocked(pl_integrator ig) {
     return m->cell_type == PL_CELL_TET4 || ig->scatter == PL_SCATTER_BLOCKED || ig->scatter == PL_SCATTER_DETERMINISTIC;
 }
 
-// Whether the mesh's FP64 cell-block path runs on pairs of cells (after prepare_blocked).
-static bool uses_pairs(pl_mesh m) { return m->pair && m->pair->num_blocks > 0; }
-
 // The FP64 cell-block kernels (after prepare_blocked); false when they do not support the configuration.
 static bool apply_cells(pl_integrator ig, const DomainParams& p, int rheo, bool bf, int op, bool insert, bool reduced = false) {
     pl_mesh m = ig->mesh;
@@ -792,9 +789,6 @@ static bool apply_cells_f32(pl_integrator ig, const DomainParams& p, int rheo, b
     if (uses_pairs(m)) return launch_domain_jv32_pair(p, *m->pair, rheo, s, reduced);
     return launch_domain_jv32_blocked(p, *m->blocked, m->cell_type, rheo, m->nnodes, s, reduced);
 }
-
-// Reduced slot ids of the layout that apply_cells uses (after prepare_blocked and ensure_reduced_cells).
-static int ensure_cell_ids_reduced(pl_mesh m) { return uses_pairs(m) ? ensure_pair_reduced_ids(m) : ensure_reduced_ids(m); }
 
 // The reduced fault space's connectivity (each positive-side node replaced by its negative-side
 // partner) and node map. Refused (PL_ERR_UNSUPPORTED) when a pair's two nodes do not coincide:
@@ -895,9 +889,8 @@ int jacobian_action_reduced_f32(pl_integrator_s* ig, double t, double dt, const 
 
 int prepare_blocked(pl_integrator_s* ig) {
     pl_mesh m = ig->mesh;
-    int rc = PL_OK;
-    if (m->cell_type == PL_CELL_TET4 && tet_pairs_selected() && (rc = ensure_pair_layout(m)) != PL_OK) return rc;
-    if (!uses_pairs(m) && (rc = ensure_blocked_layout(m)) != PL_OK) return rc;
+    const int rc = m->cell_type == PL_CELL_TET4 ? prepare_tet_layout(m) : ensure_blocked_layout(m);
+    if (rc) return rc;
     const int64_t slots = uses_pairs(m) ? m->pair->num_slots : m->blocked->num_slots;
     if (ig->scatter == PL_SCATTER_DETERMINISTIC && !ig->d_block_partial && slots > 0)
         PLB_CUDA(dev_alloc(&ig->d_block_partial, 3 * slots));

@@ -63,9 +63,13 @@ bool launch_domain_apply_blocked(const DomainParams& p, const BlockedLayout& b, 
 // The same on pairs of cells (tetpair.cu); returns false when the layout does not support the
 // configuration. The layout is built once per mesh; reduced slot ids as below.
 struct PairLayout;
-bool tet_pairs_selected();
+bool uses_pairs(const pl_mesh_s* m);
 int ensure_pair_layout(pl_mesh_s* m);
 int ensure_pair_reduced_ids(pl_mesh_s* m);
+// The layout that serves a tetrahedral mesh (pairs, or single cells), and its reduced slot ids (after
+// ensure_reduced_cells); call outside stream capture.
+int prepare_tet_layout(pl_mesh_s* m);
+int ensure_cell_ids_reduced(pl_mesh_s* m);
 void free_pair_layout(PairLayout* L, cudaStream_t after);
 bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rheo, bool bf, int op, bool insert, int64_t nnodes,
                               double* partial, cudaStream_t s, bool reduced = false);

@@ -25,6 +25,7 @@
 #include "domain_kernels.cuh"
 #include "internal.hpp"
 #include "launch.hpp"
+#include "tetpair.cuh"
 
 namespace plb {
 
@@ -171,7 +172,7 @@ PL_D bool take_last_ticket(unsigned int* counter) {
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        last = atomicAdd(counter, 1u) == gridDim.x * gridDim.y - 1;
         if (last) *counter = 0u;  // every other block has taken its ticket
     }
     __syncthreads();
@@ -179,11 +180,11 @@ PL_D bool take_last_ticket(unsigned int* counter) {
     return last;
 }
 
-// sh: kBThreads / 32 * K doubles of shared memory.
-template <int K>
+// sh: T / 32 * K doubles of shared memory (T threads per block).
+template <int K, int T = kBThreads, int U = 8>
 PL_D void sum_partials_last_block_in(const double* partials, double* out, double* prev, double (*sh)[K]) {
     const int k = threadIdx.x % K;
-    constexpr int STEP = kBThreads / K, U = 8;  // loads in flight: one block reads them all, a chain of L2 latencies
+    constexpr int STEP = T / K;  // loads in flight: one block reads them all, a chain of L2 latencies
     double s = 0.0;
     for (int b = threadIdx.x / K; b < (int)gridDim.x; b += U * STEP) {
         double v[U];
@@ -200,7 +201,7 @@ PL_D void sum_partials_last_block_in(const double* partials, double* out, double
     if (threadIdx.x < K) {
         double t = 0.0;
 #pragma unroll
-        for (int i = 0; i < kBThreads / 32; ++i) t += sh[i][threadIdx.x];
+        for (int i = 0; i < T / 32; ++i) t += sh[i][threadIdx.x];
         if (prev) prev[threadIdx.x] = out[threadIdx.x];
         out[threadIdx.x] = t;
     }
@@ -537,6 +538,233 @@ __global__ void __launch_bounds__(kMultiBlockCells, 3) k_tet_blocked_jv32_multi(
             sum_partials_last_block_in<K>(pq_part, fin.out_a, fin.prev_a,
                                           reinterpret_cast<double (*)[K]>(sh + kMultiBlockCells / 32 * K));
     }
+}
+
+// The same on the pairs of tetpair.cu, one CTA per (block, KC right-hand sides): blockIdx.y is the
+// chunk. A thread forms the element vectors of two tetrahedra that share a face (15 entries for the
+// pair instead of 24); with cf = cofactors / 6 and lambda, mu times 6 / det one set of factors serves
+// both the gradient and the test functions. In the sums a thread takes a node's three components (one
+// component per thread: 16.3 us for 15.5). Measured with 94,080 cells and K = 8, in the PCG on B200:
+// 18.1 -> 15.5 us against k_tet_blocked_jv32_multi; bound by issue and shared memory in about equal
+// parts, with a tail of 3 us for the energies' last-CTA sum. 3 CTAs per SM are as fast, 5 spill (28 us).
+template <int LD>
+constexpr int kPairMultiCtas = LD == kPairSmallLd ? 4 : 3;  // by shared memory and registers
+
+template <int K, int LD>
+__global__ void __launch_bounds__(kPairThreads, kPairMultiCtas<LD>)
+    k_tet_pair_jv32_multi(DomainParams p, PairArrays A, const float* __restrict__ v, float* out, bool store_owned,
+                          double* pq_part, const double* __restrict__ pq_rz, FinSpec fin) {
+    constexpr int KC = MultiChunk<K>::value, T = kPairThreads;
+    using Smem = PairSmem<float, LD, KC>;
+    extern __shared__ __align__(16) char smem_raw[];
+    Smem& S = *reinterpret_cast<Smem*>(smem_raw);
+    __shared__ float s_sig[KC];  // energy scales (pq_part)
+    const int r0 = blockIdx.y * KC, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t G = gridDim.x;
+    // odd chunks run backwards, so that the CTAs with one block more spread over the SMs
+    int64_t b = blockIdx.y & 1 ? G - 1 - blockIdx.x : blockIdx.x;
+    uint32_t nd_next[2];
+    int ns, ns_next;
+    uint4 item = pair_load_item(A, b), item_next = pair_load_item(A, b + G);
+    float2 lm[2];
+    auto load_tangents = [&] {
+        if (p.lm32) pair_load_tangents<true>(p, item, lm);
+        else pair_load_tangents<false>(p, item, lm);
+        if (p.lm32 && item_next.w != kNoItem) prefetch_l2(&p.lm32[2 * (int64_t)item_next.w]);
+    };
+    {
+        uint32_t nd0[2];
+        pair_load_ids<LD>(A, b, nd0, ns);
+        pair_stage<LD, KC>(v + r0, K, A, b, nd0, ns, S, 0);
+        __pipeline_commit();
+        pair_load_ids<LD>(A, b + G, nd_next, ns_next);
+        load_tangents();
+    }
+    if (pq_part && threadIdx.x < KC) {
+        const double rz = pq_rz[r0 + threadIdx.x];
+        s_sig[threadIdx.x] = (rz > 0.0 && rz < 1e300) ? (float)fmin(fmax(1.0 / sqrt(rz), 1e-30), 1e30) : 1.0f;
+    }
+    double pq_acc = 0.0;  // this lane's energy sum (warp_chunk_sum)
+    for (int it = 0; b < A.nblocks; b += G, ++it) {
+        uint32_t nd_after[2];
+        int ns_after;
+        pair_load_ids<LD>(A, b + 2 * G, nd_after, ns_after);
+        const uint4 item_after = pair_load_item(A, b + 2 * G);
+        __pipeline_wait_prior(0);
+        // block b's copies have landed; every thread has finished the node sums of the previous block
+        __syncthreads();
+        if (b + G < A.nblocks) pair_stage<LD, KC>(v + r0, K, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
+        __pipeline_commit();
+        nd_next[0] = nd_after[0], nd_next[1] = nd_after[1];
+        float en[KC];
+#pragma unroll
+        for (int rr = 0; rr < KC; ++rr) en[rr] = 0.f;
+        if (item.w != kNoItem) {
+            int n[5];
+            pair_nodes(item, n);
+            float cf[2][3][3], lam[2], mu[2];
+            {
+                double e[4][3], n12[3], c0[3], c1[3];
+                pair_diffs<LD>(n, S.node[it & 1].x, e);
+                cross3(e[0], e[1], n12);
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    // corners of the cofactor rows: n1, n2, n3 and n2, n1, n4 (edges 1, 0, 3)
+                    if (t == 0) cross3(e[1], e[2], c0), cross3(e[2], e[0], c1);
+                    else cross3(e[0], e[3], c0), cross3(e[3], e[1], c1);
+                    const double* e0 = e[t];
+                    const double det = e0[0] * c0[0] + e0[1] * c0[1] + e0[2] * c0[2];
+                    const bool on = t == 0 || !pair_single(item);
+                    if (on && !(det > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
+                    const double r6 = on ? 6.0 / det : 0.0, sg = t ? -1.0 / 6.0 : 1.0 / 6.0;
+                    lam[t] = (float)(lm[t].x * r6);
+                    mu[t] = (float)(lm[t].y * r6);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        cf[t][0][d] = on ? (float)(c0[d] * (1.0 / 6.0)) : 0.f;
+                        cf[t][1][d] = on ? (float)(c1[d] * (1.0 / 6.0)) : 0.f;
+                        cf[t][2][d] = on ? (float)(n12[d] * sg) : 0.f;
+                    }
+                }
+            }
+            // gradients of the two cells times their volumes
+            float s[2][KC][3][3];
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) {
+                const float* V = S.node[it & 1].v + KC * cc * LD;
+                float u0[KC], g[4][KC];
+                ld_vec<KC>(V + KC * n[0], u0);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    ld_vec<KC>(V + KC * n[k + 1], g[k]);
+#pragma unroll
+                    for (int rr = 0; rr < KC; ++rr) g[k][rr] -= u0[rr];
+                }
+#pragma unroll
+                for (int rr = 0; rr < KC; ++rr)
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        s[0][rr][cc][d] = g[0][rr] * cf[0][0][d] + g[1][rr] * cf[0][1][d] + g[2][rr] * cf[0][2][d];
+                        s[1][rr][cc][d] = g[1][rr] * cf[1][0][d] + g[0][rr] * cf[1][1][d] + g[3][rr] * cf[1][2][d];
+                    }
+            }
+            // flux f1 = -(lambda tr(e) I + 2 mu e) in place of the gradients (and the energies
+            // vol (lambda tr(e)^2 + 2 mu e:e) first)
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int rr = 0; rr < KC; ++rr) {
+                    float(&q)[3][3] = s[t][rr];
+                    const float tr = q[0][0] + q[1][1] + q[2][2], ltr = lam[t] * tr;
+                    const float sxy = q[0][1] + q[1][0], syz = q[1][2] + q[2][1], sxz = q[0][2] + q[2][0];
+                    if (pq_part) {
+                        // scaled gradient; every product pairs a modulus-weighted factor with a bare one
+                        const float g = s_sig[rr];
+                        const float h = g * tr, a = g * q[0][0], c = g * q[1][1], d = g * q[2][2];
+                        const float u = g * sxy, w = g * syz, z = g * sxz;
+                        en[rr] += (lam[t] * h) * h + (2.0f * mu[t] * a) * a + (2.0f * mu[t] * c) * c + (2.0f * mu[t] * d) * d +
+                                  (mu[t] * u) * u + (mu[t] * w) * w + (mu[t] * z) * z;
+                    }
+                    q[0][0] = -(2.0f * mu[t] * q[0][0] + ltr);
+                    q[1][1] = -(2.0f * mu[t] * q[1][1] + ltr);
+                    q[2][2] = -(2.0f * mu[t] * q[2][2] + ltr);
+                    q[0][1] = q[1][0] = -mu[t] * sxy;
+                    q[1][2] = q[2][1] = -mu[t] * syz;
+                    q[0][2] = q[2][0] = -mu[t] * sxz;
+                }
+            float* E = S.E + KC * threadIdx.x;
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) {
+                float w[5][KC];
+#pragma unroll
+                for (int rr = 0; rr < KC; ++rr) {
+                    float a[2][3];
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+#pragma unroll
+                        for (int k = 0; k < 3; ++k)
+                            a[t][k] = s[t][rr][cc][0] * cf[t][k][0] + s[t][rr][cc][1] * cf[t][k][1] + s[t][rr][cc][2] * cf[t][k][2];
+                    w[0][rr] = -(a[0][0] + a[0][1] + a[0][2]) - (a[1][0] + a[1][1] + a[1][2]);
+                    w[1][rr] = a[0][0] + a[1][1];
+                    w[2][rr] = a[0][1] + a[1][0];
+                    w[3][rr] = a[0][2];
+                    w[4][rr] = a[1][2];
+                }
+#pragma unroll
+                for (int k = 0; k < 5; ++k) st_vec<KC>(E + KC * T * (3 * k + cc), w[k]);
+            }
+        }
+        if (pq_part) warp_chunk_sum<KC>(en, 0, pq_acc);
+        item = item_next, item_next = item_after;
+        load_tangents();
+        __syncthreads();
+        const auto& M = S.meta[it & 1];
+        for (int k = threadIdx.x; k < ns; k += T) {
+            const uint32_t id = M.ids[k];
+            float* o = out + K * 3 * (int64_t)(id & ~kPairShared) + r0;
+            float acc[3][KC], old[3][KC];
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) {
+#pragma unroll
+                for (int rr = 0; rr < KC; ++rr) acc[cc][rr] = old[cc][rr] = 0.f;
+                if (!store_owned && !(id & kPairShared)) ld_vec<KC>(o + cc * K, old[cc]);
+            }
+            const int j0 = M.off[k], j1 = M.off[k + 1];
+#pragma unroll 2
+            for (int j = j0; j < j1; ++j) {
+                const float* e = S.E + KC * M.inc[j];
+#pragma unroll
+                for (int cc = 0; cc < 3; ++cc) {
+                    float t[KC];
+                    ld_vec<KC>(e + KC * cc * T, t);
+#pragma unroll
+                    for (int rr = 0; rr < KC; ++rr) acc[cc][rr] += t[rr];
+                }
+            }
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) {
+                if (id & kPairShared) {
+                    red_vec<KC>(o + cc * K, acc[cc]);
+                } else {
+#pragma unroll
+                    for (int rr = 0; rr < KC; ++rr) acc[cc][rr] += old[cc][rr];
+                    st_vec<KC>(o + cc * K, acc[cc]);
+                }
+            }
+        }
+        ns = ns_next, ns_next = ns_after;
+    }
+    __pipeline_wait_prior(0);
+    if (pq_part) {
+        __syncthreads();  // the element vectors are no longer read: their space holds the sums
+        double* sh = reinterpret_cast<double*>(smem_raw);  // [warps][KC], then [warps][K]
+        const int rhs = warp_chunk_rhs<KC>(lane);
+        if (rhs >= 0) {
+            const double g = s_sig[rhs];
+            sh[warp * KC + rhs] = pq_acc / (g * g);
+        }
+        __syncthreads();
+        if (threadIdx.x < KC) {
+            double t = 0.0;
+#pragma unroll
+            for (int i = 0; i < T / 32; ++i) t += sh[i * KC + threadIdx.x];
+            pq_part[blockIdx.x * K + r0 + threadIdx.x] = t;
+        }
+        if (fin.counter && take_last_ticket(fin.counter))
+            sum_partials_last_block_in<K, T, 20>(pq_part, fin.out_a, fin.prev_a, reinterpret_cast<double (*)[K]>(sh + T / 32 * KC));
+    }
+}
+
+template <int K, int LD>
+void launch_pair_multi(const DomainParams& p, const PairArrays& A, const float* v, float* out, bool store_owned, double* part,
+                       const double* scal, const FinSpec& fin, cudaStream_t s) {
+    constexpr int chunks = K / MultiChunk<K>::value;
+    constexpr size_t smem = sizeof(PairSmem<float, LD, MultiChunk<K>::value>);
+    ensure_kernel_smem((const void*)k_tet_pair_jv32_multi<K, LD>, smem);
+    const int64_t gx = std::max<int64_t>(1, (int64_t)sm_count() * kPairMultiCtas<LD> / chunks);
+    k_tet_pair_jv32_multi<K, LD><<<dim3((unsigned)std::min(A.nblocks, gx), chunks), kPairThreads, smem, s>>>(
+        p, A, v, out, store_owned, part, scal, fin);
+    count_launch();
 }
 
 template <int K>
@@ -1055,7 +1283,10 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
     cudaStream_t s = m->ctx->stream;
     if (pq && S->ops.size() != 1) return fail(PL_ERR_UNSUPPORTED, "fused energies need a single integrator");
     // the solver's reduced fault space directly (slot ids of the reduced space: no unfold or fold)
-    const bool reduced = S->npairs > 0 && S->reduced && m->blocked && m->blocked->d_slot_node_red;
+    int rc = prepare_tet_layout(m);
+    if (rc) return rc;
+    const bool pairs = uses_pairs(m);
+    const bool reduced = S->npairs > 0 && S->reduced && (pairs ? (void*)m->pair->d_ids_red : (void*)m->blocked->d_slot_node_red);
     if (S->npairs > 0 && !reduced) {
         k_b_unfold<K><<<bgrid(3 * K * S->npairs), 256, 0, s>>>(const_cast<float*>(v), S->d_pair_neg, S->d_pair_pos, S->npairs);
         count_launch();
@@ -1064,15 +1295,26 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
     bool first = true;
     for (pl_integrator ig : S->ops) {
         DomainParams pp;
-        int rc = bind_domain_jacobian(ig, &pp);
-        if (rc) return rc;
+        if ((rc = bind_domain_jacobian(ig, &pp)) != PL_OK) return rc;
         pp.t = S->t;
         pp.dt = S->dt;
         if (ig->lm32_valid && ig->lm32_t == S->t && ig->lm32_dt == S->dt) pp.lm32 = ig->d_lm32;
         if (m->cell_type != PL_CELL_TET4 || ig->j3 != K_ILE_JF3VU || ig->subset)
             return fail(PL_ERR_UNSUPPORTED, "batched solves support P1 tetrahedra with isotropic linear elasticity");
-        rc = ensure_blocked_layout(m);
-        if (rc) return rc;
+        FinSpec fin;
+        if (pq) {
+            fin.counter = ticket;
+            fin.out_a = pq;
+        }
+        if (pairs) {
+            const PairArrays A = pair_arrays_of(*m->pair, nullptr, reduced);
+            if (m->pair->ld == kPairSmallLd)
+                launch_pair_multi<K, kPairSmallLd>(pp, A, v, out, first, pq ? part : nullptr, scal, fin, s);
+            else
+                launch_pair_multi<K, kPairMaxNodes>(pp, A, v, out, first, pq ? part : nullptr, scal, fin, s);
+            first = false;
+            continue;
+        }
         const BlockedLayout& L = *m->blocked;
         if (L.num_blocks == 0) return fail(PL_ERR_UNSUPPORTED, "no cell-block layout for this mesh");
         if (L.max_local_nodes > 2 * kMultiBlockCells)
@@ -1089,11 +1331,6 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
             per_sm_smem = smem;
         }
         const int grid = (int)std::min<int64_t>(L.num_blocks, (int64_t)sm_count() * per_sm);
-        FinSpec fin;
-        if (pq) {
-            fin.counter = ticket;
-            fin.out_a = pq;
-        }
         k_tet_blocked_jv32_multi<K><<<grid, kMultiBlockCells, smem, s>>>(
             pp, L.d_cell_begin, L.d_block_node_begin, reduced ? L.d_slot_node_red : L.d_slot_node,
             (const ushort4*)L.d_local_cells, L.d_inc_off, L.d_inc,
@@ -1917,7 +2154,7 @@ int pl_batch_solver_create(pl_solver base, int tile, pl_batch_solver* out) {
     A(&B->jx64, B->n);
     // the cell-block layout is built here, outside any stream capture
     if (e == cudaSuccess) {
-        const int rc = ensure_blocked_layout(base->mesh);
+        const int rc = prepare_tet_layout(base->mesh);
         if (rc) {
             pl_batch_solver_destroy(B);
             return rc;
@@ -1934,13 +2171,14 @@ int pl_batch_solver_create(pl_solver base, int tile, pl_batch_solver* out) {
     return PL_OK;
 }
 
-// The batched operator's layouts on S's mesh, with the slot ids of the reduced fault space where the
+// The batched operator's layout on S's mesh, with the slot ids of the reduced fault space where the
 // solver acts in it; outside any stream capture.
 static int prepare_multi_layout(pl_solver S) {
     pl_mesh m = S->mesh;
-    int rc = ensure_blocked_layout(m);
-    if (rc == PL_OK && S->npairs > 0 && S->reduced && m->blocked->num_blocks > 0 && m->h_node_red.size() == (size_t)m->nnodes)
-        rc = ensure_reduced_ids(m);
+    int rc = prepare_tet_layout(m);
+    if (rc == PL_OK && S->npairs > 0 && S->reduced && m->h_node_red.size() == (size_t)m->nnodes &&
+        (uses_pairs(m) || m->blocked->num_blocks > 0))
+        rc = ensure_cell_ids_reduced(m);
     return rc;
 }
 
@@ -2083,7 +2321,7 @@ int pl_batch_solver_set_multigrid(pl_batch_solver B, pl_multigrid mg) {
     for (const MgLevelView& L : v.levels) {
         pl_mesh lm = L.S->mesh;
         if (lm->cell_type != PL_CELL_TET4) return fail(PL_ERR_UNSUPPORTED, "batched multigrid needs P1 tetrahedral levels");
-        int rc = ensure_blocked_layout(lm);
+        int rc = prepare_tet_layout(lm);
         if (rc) return rc;
     }
     B->bmg.resize(v.levels.size());

@@ -15,8 +15,6 @@
 // Block size: 240 cells in 128 items with 4 CTAs per SM (FP64, at most 128 registers) measured best
 // (two launches on 1,179,648 cells 80 us); 5 and 6 CTAs 80-92 (spills), 64, 96, 192 and 256 threads
 // 82-98, two lanes per node in the sums 89. FP32: 4, 5 and 6 CTAs 45.6, 40.1, 38.6 us.
-#include <cuda_pipeline.h>
-
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
@@ -26,115 +24,13 @@
 #include <vector>
 
 #include "bankplan.hpp"
-#include "domain_kernels.cuh"
-#include "internal.hpp"
 #include "launch.hpp"
+#include "tetpair.cuh"
 
 namespace plb {
 
-constexpr int kPairThreads = 128;    // items (pairs or single cells) of a block at most
-constexpr int kPairCells = 240;      // cells of a block at most: about 122 items
-constexpr int kPairMaxNodes = 2 * kPairThreads;  // nodes of a block at most (two per thread)
-constexpr int kPairSmallLd = 144;    // slots per block where all of a mesh's blocks fit (compact ones do)
-constexpr int kPairCtas = 4;         // resident CTAs per SM
-constexpr int kPairCtas32 = 6;       // of the FP32 action
-constexpr uint32_t kPairShared = 0x80000000u;
-constexpr uint32_t kNoNode = 0xffffffffu, kNoItem = 0xffffffffu;
-constexpr int kCellBias = 0x8000;
-
-// Per-block arrays have constant strides (LD slots per block), so their addresses need no loads.
-struct PairArrays {
-    const int32_t* nslots;      // [nblocks]
-    const uint32_t* ids;        // [nblocks][LD] node id | kPairShared (kNoNode past the block's nodes)
-    const double* coords;       // [nblocks][3][LD]
-    const uint16_t* off;        // [nblocks][LD + 8] nslots + 1 incidence offsets
-    const uint16_t* inc;        // [nblocks][5 * kPairThreads] staging offsets corner * 3 * threads + item
-    const uint4* items;         // [nblocks][kPairThreads] (see PairPlan)
-    double* partial;            // [nblocks][LD][3] deterministic partial sums
-    int64_t nblocks;
-};
-
-// Shared memory for blocks of at most LD nodes: element vectors [15][threads], two node buffers
-// (coordinates in FP64 and the field in T, component by component), two metadata buffers. LD is a
-// compile-time multiple of 16, so a node's six values sit at constant offsets.
-template <typename T, int LD>
-struct PairSmem {
-    T E[15 * kPairThreads];
-    struct Node {
-        double x[3 * LD];
-        T v[3 * LD];
-    } node[2];
-    struct Meta {
-        uint32_t ids[LD];
-        uint16_t off[LD + 8];
-        uint16_t inc[5 * kPairThreads];
-    } meta[2];
-};
-
-// This thread's slot ids of block b, and the block's slot count.
-template <int LD>
-PL_D void pair_load_ids(const PairArrays& A, int64_t b, uint32_t (&nd)[2], int& ns) {
-    nd[0] = nd[1] = kNoNode;
-    ns = 0;
-    if (b >= A.nblocks) return;
-    ns = A.nslots[b];
-    nd[0] = A.ids[b * LD + threadIdx.x];
-    if (threadIdx.x + kPairThreads < LD) nd[1] = A.ids[b * LD + threadIdx.x + kPairThreads];
-}
-
-// Asynchronous copies of block b (ids in nd and slot count ns read one block earlier): coordinates,
-// ids, offsets and incidences as aligned 16-byte runs, the field of its nodes one value at a time.
-template <typename T, int LD>
-PL_D void pair_stage(const T* __restrict__ field, const PairArrays& A, int64_t b, const uint32_t (&nd)[2], int ns,
-                     PairSmem<T, LD>& S, int buf) {
-    auto& node = S.node[buf];
-    auto& M = S.meta[buf];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-        if (nd[k] != kNoNode) {
-            const T* f = field + 3 * (int64_t)(nd[k] & ~kPairShared);
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                __pipeline_memcpy_async(&node.v[d * LD + threadIdx.x + k * kPairThreads], f + d, sizeof(T));
-        }
-    const double* x = A.coords + b * 3 * LD;
-    if (2 * threadIdx.x < ns)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) __pipeline_memcpy_async(&node.x[d * LD + 2 * threadIdx.x], x + d * LD + 2 * threadIdx.x, 16);
-    if (4 * threadIdx.x < ns) __pipeline_memcpy_async(&M.ids[4 * threadIdx.x], &A.ids[b * LD + 4 * threadIdx.x], 16);
-    if (8 * threadIdx.x <= ns) __pipeline_memcpy_async(&M.off[8 * threadIdx.x], &A.off[b * (LD + 8) + 8 * threadIdx.x], 16);
-    if (threadIdx.x < 5 * kPairThreads / 8)
-        __pipeline_memcpy_async(&M.inc[8 * threadIdx.x], &A.inc[b * 5 * kPairThreads + 8 * threadIdx.x], 16);
-}
-
-PL_D uint4 pair_load_item(const PairArrays& A, int64_t b) {
-    return b < A.nblocks ? A.items[b * kPairThreads + threadIdx.x] : make_uint4(0, 0, 0, kNoItem);
-}
-PL_D bool pair_single(const uint4& it) { return it.z >> 16 == 0; }
-// The item's per-cell inputs, on their way to L2 (cell B lies near cell A).
-template <bool BF>
-PL_D void pair_prefetch_cells(const DomainParams& p, const uint4& it) {
-    if (it.w == kNoItem) return;
-    prefetch_l2(&p.mu[it.w]);
-    prefetch_l2(&p.K[it.w]);
-    if (BF)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) prefetch_l2(&p.body_force[d * p.ncells + it.w]);
-}
-// Per-cell inputs of the item's cells (a single cell's twice).
-template <typename L>
-PL_D void pair_load_cells(const DomainParams& p, const uint4& it, double (&aA)[L::size], double (&aB)[L::size]) {
-    if (it.w == kNoItem) return;
-    const int64_t cA = it.w, cB = pair_single(it) ? cA : cA + (int)(it.z >> 16) - kCellBias;
-    L::load_cell(p, cA, aA);
-    L::load_cell(p, cB, aB);
-}
-
-PL_D void cross3(const double (&a)[3], const double (&b)[3], double (&c)[3]) {
-    c[0] = a[1] * b[2] - a[2] * b[1];
-    c[1] = a[2] * b[0] - a[0] * b[2];
-    c[2] = a[0] * b[1] - a[1] * b[0];
-}
+constexpr int kPairCtas = 4;    // resident CTAs per SM
+constexpr int kPairCtas32 = 6;  // of the FP32 action
 
 // One tetrahedron from its cofactor rows c0, c1, c2 (det J times the basis gradients of its corners
 // 1, 2, 3), det and the field differences g0, g1, g2 of those corners: v[k] = |K| f1 . grad(phi_{k+1})
@@ -179,30 +75,16 @@ PL_D void pair_tet(const DomainParams& p, const double* a, const double (&c0)[3]
     }
 }
 
-// Differences of the item's nodes n1 .. n4 from n0: coordinates e, field g.
-template <typename T, int LD>
-PL_D void pair_edges(const uint4& it, const typename PairSmem<T, LD>::Node& node, double (&e)[4][3], T (&g)[4][3]) {
-    const int n[5] = {(int)(it.x & 0xffff), (int)(it.x >> 16), (int)(it.y & 0xffff), (int)(it.y >> 16), (int)(it.z & 0xffff)};
-    double x0[3];
-    T u0[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) x0[d] = node.x[d * LD + n[0]], u0[d] = node.v[d * LD + n[0]];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            e[k][d] = node.x[d * LD + n[k + 1]] - x0[d];
-            g[k][d] = node.v[d * LD + n[k + 1]] - u0[d];
-        }
-}
-
 // The element vectors of one item into column E: tetrahedra (n0, n1, n2, n3) and, unless single,
 // (n0, n2, n1, n4).
 template <int RHEO, bool BF, int OP, int LD>
 PL_D void pair_item(const DomainParams& p, const uint4& it, const double* aA, const double* aB,
                     const typename PairSmem<double, LD>::Node& node, double* E) {
+    int n[5];
     double e[4][3], g[4][3];
-    pair_edges<double, LD>(it, node, e, g);
+    pair_nodes(it, n);
+    pair_diffs<LD>(n, node.x, e);
+    pair_diffs<LD>(n, node.v, g);
     double n12[3], c0[3], c1[3], v[3][3], w[3] = {0, 0, 0}, r0[3], r1[3], r2[3];
     cross3(e[0], e[1], n12);
     cross3(e[1], e[2], c0);
@@ -272,7 +154,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas) k_tet_pair(DomainPara
     {
         uint32_t nd0[2];
         pair_load_ids<LD>(A, b, nd0, ns);
-        pair_stage(field, A, b, nd0, ns, S, 0);
+        pair_stage<LD, 1>(field, 1, A, b, nd0, ns, S, 0);
         __pipeline_commit();
         pair_load_ids<LD>(A, b + G, nd_next, ns_next);
         pair_load_cells<L>(p, item, aA, aB);
@@ -290,7 +172,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas) k_tet_pair(DomainPara
         // block b's copies have landed; every thread has finished the node sums of the previous block
         // (its buffers are free for block b + G)
         __syncthreads();
-        if (b + G < A.nblocks) pair_stage(field, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
+        if (b + G < A.nblocks) pair_stage<LD, 1>(field, 1, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
         __pipeline_commit();
         nd_next[0] = nd_after[0], nd_next[1] = nd_after[1];
         if (item.w != kNoItem) pair_item<RHEO, BF, OP, LD>(p, item, aA, aB, S.node[it & 1], S.E + threadIdx.x);
@@ -321,29 +203,6 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas) k_tet_pair(DomainPara
 }
 
 // ---- FP32 Jacobian action --------------------------------------------------------------------
-// The isotropic tangent (lambda, mu) of the item's cells (a single cell's twice): the solver's cache
-// (p.lm32; CACHED) or the registered Jacobian kernel.
-template <bool CACHED>
-PL_D void pair_load_tangents(const DomainParams& p, const uint4& it, float2 (&lm)[2]) {
-    if (it.w == kNoItem) return;
-    const int64_t cells[2] = {(int64_t)it.w, pair_single(it) ? (int64_t)it.w : (int64_t)it.w + (int)(it.z >> 16) - kCellBias};
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        if (CACHED) {
-            lm[k] = reinterpret_cast<const float2*>(p.lm32)[cells[k]];
-        } else {
-            using L = AuxLayout<RHEO_ILE, false>;
-            const AuxOffsets<RHEO_ILE, false> aoff;
-            double a[L::size], x[3] = {0, 0, 0}, Jf3[81];
-            L::load_cell(p, cells[k], a);
-#pragma unroll
-            for (int i = 0; i < 81; ++i) Jf3[i] = 0.0;
-            call_jf3<RHEO_ILE>(L::numA, aoff.v, a, p, x, Jf3);
-            lm[k] = make_float2((float)(-Jf3[((0 * 3 + 1) * 3 + 0) * 3 + 1]), (float)(-Jf3[((0 * 3 + 1) * 3 + 1) * 3 + 0]));
-        }
-    }
-}
-
 // pair_tet of the FP32 action: cofactors and det in FP64, gradient, flux and vectors in FP32.
 PL_D void pair_tet32(const DomainParams& p, float2 lm, const double (&c0)[3], const double (&c1)[3], const double (&c2)[3],
                      double det, const float (&g0)[3], const float (&g1)[3], const float (&g2)[3], float (&v)[3][3]) {
@@ -390,7 +249,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas32) k_tet_pair_jv32(Dom
     {
         uint32_t nd0[2];
         pair_load_ids<LD>(A, b, nd0, ns);
-        pair_stage(p.v32, A, b, nd0, ns, S, 0);
+        pair_stage<LD, 1>(p.v32, 1, A, b, nd0, ns, S, 0);
         __pipeline_commit();
         pair_load_ids<LD>(A, b + G, nd_next, ns_next);
         pair_load_tangents<CACHED>(p, item, lm);
@@ -404,14 +263,17 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas32) k_tet_pair_jv32(Dom
         __pipeline_wait_prior(0);
         // as in k_tet_pair: block b has landed, and the buffers of block b + G are free
         __syncthreads();
-        if (b + G < A.nblocks) pair_stage(p.v32, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
+        if (b + G < A.nblocks) pair_stage<LD, 1>(p.v32, 1, A, b + G, nd_next, ns_next, S, (it + 1) & 1);
         __pipeline_commit();
         nd_next[0] = nd_after[0], nd_next[1] = nd_after[1];
         if (item.w != kNoItem) {
             float* E = S.E + threadIdx.x;
             double e[4][3], n12[3], c0[3], c1[3];
             float g[4][3], v[3][3], r0[3], r1[3], r2[3];
-            pair_edges<float, LD>(item, S.node[it & 1], e, g);
+            int n[5];
+            pair_nodes(item, n);
+            pair_diffs<LD>(n, S.node[it & 1].x, e);
+            pair_diffs<LD>(n, S.node[it & 1].v, g);
             cross3(e[0], e[1], n12);
             cross3(e[1], e[2], c0);
             cross3(e[2], e[0], c1);
@@ -750,19 +612,6 @@ int build_pair_layout(pl_mesh_s* m) {
     return PL_OK;
 }
 
-PairArrays arrays_of(const PairLayout& L, double* partial, bool reduced) {
-    PairArrays A;
-    A.nslots = L.d_nslots;
-    A.ids = reduced ? L.d_ids_red : L.d_ids;
-    A.coords = L.d_coords;
-    A.off = L.d_off;
-    A.inc = L.d_inc;
-    A.items = (const uint4*)L.d_items;
-    A.partial = partial;
-    A.nblocks = L.num_blocks;
-    return A;
-}
-
 template <typename T, int LD, typename Kernel>
 void launch_pairs(Kernel kern, const DomainParams& p, const PairArrays& A, cudaStream_t s) {
     constexpr size_t smem = sizeof(PairSmem<T, LD>);
@@ -785,7 +634,7 @@ void launch_jv32(const DomainParams& p, const PairLayout& L, const PairArrays& A
 
 template <bool BF, int OP>
 void launch_op(const DomainParams& p, const PairLayout& L, bool insert, double* partial, bool reduced, cudaStream_t s) {
-    const PairArrays A = arrays_of(L, partial, reduced);
+    const PairArrays A = pair_arrays_of(L, partial, reduced);
     if (partial && insert) launch_one<BF, OP, true, true>(p, L, A, s);
     else if (partial) launch_one<BF, OP, false, true>(p, L, A, s);
     else if (insert) launch_one<BF, OP, true, false>(p, L, A, s);
@@ -802,7 +651,7 @@ void launch_op(const DomainParams& p, const PairLayout& L, bool insert, double* 
 
 // PYLITH_B200_TET_KERNEL, read once per process: "pair" (the default) or a cell-block kernel of
 // blocked.cu.
-bool tet_pairs_selected() {
+static bool tet_pairs_selected() {
     static const bool on = [] {
         const char* v = std::getenv("PYLITH_B200_TET_KERNEL");
         return !v || (std::strcmp(v, "pad2") != 0 && std::strcmp(v, "pipe") != 0 && std::strcmp(v, "twophase") != 0);
@@ -857,6 +706,17 @@ int ensure_pair_reduced_ids(pl_mesh_s* m) {
     return PL_OK;
 }
 
+// Whether the mesh's cell-block kernels run on pairs (after prepare_tet_layout).
+bool uses_pairs(const pl_mesh_s* m) { return m->pair && m->pair->num_blocks > 0; }
+
+int prepare_tet_layout(pl_mesh_s* m) {
+    int rc = PL_OK;
+    if (tet_pairs_selected() && (rc = ensure_pair_layout(m)) != PL_OK) return rc;
+    return uses_pairs(m) ? PL_OK : ensure_blocked_layout(m);
+}
+
+int ensure_cell_ids_reduced(pl_mesh_s* m) { return uses_pairs(m) ? ensure_pair_reduced_ids(m) : ensure_reduced_ids(m); }
+
 bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rheo, bool bf, int op, bool insert, int64_t nnodes,
                               double* partial, cudaStream_t s, bool reduced) {
     if (rheo != RHEO_ILE || L.num_blocks == 0 || (reduced && (insert || partial || !L.d_ids_red))) return false;
@@ -872,7 +732,7 @@ bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rh
 // The FP32 action; with the solver's cached tangent any isotropic rheology.
 bool launch_domain_jv32_pair(const DomainParams& p, const PairLayout& L, int rheo, cudaStream_t s, bool reduced) {
     if ((rheo != RHEO_ILE && !p.lm32) || L.num_blocks == 0 || (reduced && !L.d_ids_red)) return false;
-    const PairArrays A = arrays_of(L, nullptr, reduced);
+    const PairArrays A = pair_arrays_of(L, nullptr, reduced);
     if (p.lm32) launch_jv32<true>(p, L, A, s);
     else launch_jv32<false>(p, L, A, s);
     return true;

@@ -308,6 +308,39 @@ def test_batched_green_functions_match_single_fp64_solves(ctx):
         assert st["solves"] == len(imps) and st["inner_iterations"] > 0
 
 
+# cells in order; mixed within windows (more nodes per block); mixed throughout (the layout of single
+# cells)
+@pytest.mark.parametrize("window", [0, 432, 1296])
+@pytest.mark.parametrize("tile,integrators", [(1, 1), (2, 1), (8, 1), (8, 2)])
+def test_batched_operator_cell_orders(ctx, window, tile, integrators):
+    """Batched solves for mixed cell orders and for sums of two integrators match FP64 solves of one
+    right-hand side at a time to <= 1e-8."""
+    import torch
+    from pylith_b200 import feassemble as FA
+
+    rng = np.random.default_rng(21)
+    mesh = M.box_tet_kuhn(6, 6, 6)
+    for i in range(0, mesh.num_cells if window else 0, window or 1):
+        rng.shuffle(mesh.cells[i:i + window])
+    cons = np.zeros((mesh.num_nodes, 3), dtype=bool)
+    cons[M.boundary_mask(mesh, 0, "neg")] = True
+    dm = FA.DeviceMesh(ctx, mesh)
+    igs = [MAT.IsotropicLinearElasticity(*MAT.lognormal_elastic(mesh.num_cells, seed=22 + i)).create_integrator(dm)
+           for i in range(integrators)]
+    bs = [torch.from_numpy(rng.standard_normal(mesh.num_dof)).cuda() for _ in range(tile + 1)]
+    refined = FA.Solver(dm, cons.ravel(), igs, rtol=1e-11, precision=FA.Solver.FP32_REFINED, inner_rtol=1e-4)
+    refined.setup()
+    xs = [torch.zeros_like(b) for b in bs]
+    FA.BatchSolver(refined, tile).solve(bs, xs)
+    S = FA.Solver(dm, cons.ravel(), igs, rtol=1e-11)
+    S.setup()
+    for b, x in zip(bs, xs):
+        ref = torch.zeros_like(b)
+        S.solve(b, ref)
+        ctx.synchronize()
+        assert torch.linalg.norm(x - ref) <= 1e-8 * torch.linalg.norm(ref)
+
+
 def test_batched_chebyshev_jacobi_eigen_estimate_and_solutions(ctx, oracle_lib):
     """Chebyshev-Jacobi preconditioning of the batched FP32 PCG on a Kuhn tetrahedral mesh: the
     power-iteration estimate of lambda_max(P A) lies within [0.85, 1.0001] of the largest
