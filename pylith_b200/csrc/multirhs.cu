@@ -1152,22 +1152,11 @@ __global__ void k_b_fold(float* v, const int32_t* neg, const int32_t* pos, int64
     }
 }
 
-// FP64 [K][n] (RHS-major) residuals -> FP32 [n][K]
-__global__ void k_b_pack(const double* src, int64_t n, int K, int kk, float* dst) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i * K + kk] = (float)src[i];
-}
-// x64[kk] += d32[:, kk] on free DOFs
-__global__ void k_b_unpack_add(const float* d, int64_t n, int K, int kk, const uint8_t* mask, double* x) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        if (!mask[i]) x[i] += (double)d[i * K + kk];
-}
-
-// d[:, kk] = 0
-__global__ void k_b_col_zero(float* d, int64_t n, int K, int kk) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        d[i * K + kk] = 0.0f;
-}
+// FP64 vectors of a tile's columns; a kernel takes those whose bit is set in its `flags`.
+template <int K>
+struct Columns {
+    double* x[K];
+};
 
 // dst[:, kk] = src[:, kk]
 __global__ void k_b_col_copy(float* dst, const float* src, int64_t n, int K, int kk) {
@@ -1175,25 +1164,82 @@ __global__ void k_b_col_copy(float* dst, const float* src, int64_t n, int K, int
         dst[i * K + kk] = src[i * K + kk];
 }
 
-// z[:, kk] = P r[:, kk] (constrained DOFs zero); partial r.z of the column
-__global__ void __launch_bounds__(kBThreads) k_b_col_prec(const float* r, float* z, const uint8_t* mask,
-                                                          const float* P, int64_t nnodes, int K, int kk,
-                                                          double* part) {
+// Flagged columns: d[:, k] = 0, after x[k] += d[:, k] on free DOFs where x[k] is set.
+template <int K>
+__global__ void k_b_flush(float* __restrict__ d, Columns<K> cols, unsigned flags, const uint8_t* __restrict__ mask, int64_t n) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * K; e += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(e % K);
+        if (!(flags >> k & 1)) continue;
+        const int64_t i = e / K;
+        if (cols.x[k] && !mask[i]) cols.x[k][i] += (double)d[e];
+        d[e] = 0.0f;
+    }
+}
+
+// Flagged columns: x's positive-side fault nodes follow their negative sides.
+template <int K>
+__global__ void k_b_unfold64(Columns<K> cols, unsigned flags, const int32_t* __restrict__ neg, const int32_t* __restrict__ pos,
+                             int64_t npairs) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 3 * npairs * K; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e % (3 * npairs);
+        const int k = (int)(e / (3 * npairs));
+        if (flags >> k & 1) cols.x[k][3 * (int64_t)pos[i / 3] + i % 3] = cols.x[k][3 * (int64_t)neg[i / 3] + i % 3];
+    }
+}
+
+// P^T (Jx + b) minus b's own rows: every negative-side row of Jx gets its positive-side partner's and b's.
+__global__ void k_b_fold64(double* __restrict__ Jx, const double* __restrict__ b, const int32_t* __restrict__ neg,
+                           const int32_t* __restrict__ pos, int64_t npairs) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * npairs; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t ip = 3 * (int64_t)pos[i / 3] + i % 3;
+        Jx[3 * (int64_t)neg[i / 3] + i % 3] += Jx[ip] + b[ip];
+    }
+}
+
+// r[:, kk] = b + Jx on free DOFs (Jx after k_b_fold64); |r|^2, in FP64, into fin.out_a.
+__global__ void __launch_bounds__(kBThreads) k_b_residual64(const double* __restrict__ b, const double* __restrict__ Jx,
+                                                            const uint8_t* __restrict__ mask, int64_t n, int K, int kk,
+                                                            float* __restrict__ r, double* part, FinSpec fin) {
     double s = 0.0;
-    for (int64_t nd = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; nd < nnodes; nd += (int64_t)gridDim.x * blockDim.x) {
-        float in[3], out[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) in[c] = r[(3 * nd + c) * K + kk];
-        pinv_local(P, nd, in, out);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float v = mask[3 * nd + c] ? 0.0f : out[c];
-            z[(3 * nd + c) * K + kk] = v;
-            s += (double)in[c] * v;
-        }
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double v = mask[i] ? 0.0 : b[i] + Jx[i];
+        r[i * K + kk] = (float)v;
+        s += v * v;
     }
     double acc[1] = {s};
     block_sumK<1>(acc, part);
+    if (take_last_ticket(fin.counter)) sum_partials_last_block<1>(part, fin.out_a, fin.prev_a);
+}
+
+// Flagged columns: z[:, k] = P r[:, k] (constrained DOFs zero), p[:, k] = z[:, k] where `start` has the
+// column's bit, and r.z into rz[k]; sums: K doubles of scratch.
+template <int K>
+__global__ void __launch_bounds__(kBThreads) k_b_cols_prec(const float* __restrict__ r, float* __restrict__ z, float* __restrict__ p,
+                                                           const uint8_t* __restrict__ mask, const float* __restrict__ P,
+                                                           int64_t nnodes, unsigned flags, unsigned start, double* part,
+                                                           double* rz, double* sums, unsigned int* counter) {
+    double a = 0.0;
+    const int k = threadIdx.x % K;
+    if (flags >> k & 1)
+        for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnodes * K; e += (int64_t)gridDim.x * blockDim.x) {
+            const int64_t nd = e / K;
+            float in[3], out[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) in[c] = r[(3 * nd + c) * K + k];
+            pinv_local(P, nd, in, out);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float v = mask[3 * nd + c] ? 0.0f : out[c];
+                z[(3 * nd + c) * K + k] = v;
+                if (start >> k & 1) p[(3 * nd + c) * K + k] = v;
+                a += (double)in[c] * v;
+            }
+        }
+    block_sum_by_rhs<K>(a, part);
+    if (take_last_ticket(counter)) {
+        sum_partials_last_block<K>(part, sums, nullptr);
+        if (threadIdx.x < K && (flags >> k & 1)) rz[k] = sums[k];
+    }
 }
 
 // Blocks of the vector kernels whose partial sums are counted by gridDim.x: two items per thread, at
@@ -1220,8 +1266,7 @@ struct pl_batch_solver_s {
     double* part_a = nullptr;
     double* part_b = nullptr;
     unsigned int* ticket = nullptr;  // last-block counter of the fused reductions (zero between kernels)
-    double* r64 = nullptr;    // single-RHS FP64 outer residual
-    double* jx64 = nullptr;
+    double* jx64 = nullptr;   // single-RHS FP64 action
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
     unsigned long long graph_epoch = 0;
@@ -1849,53 +1894,73 @@ int apply_J64(pl_solver S, const double* v, double* out) {
     return PL_OK;
 }
 
-__global__ void k_unfold64(double* v, const int32_t* neg, const int32_t* pos, int64_t npairs) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * npairs; i += (int64_t)gridDim.x * blockDim.x)
-        v[3 * (int64_t)pos[i / 3] + i % 3] = v[3 * (int64_t)neg[i / 3] + i % 3];
-}
-__global__ void k_fold64(double* v, const int32_t* neg, const int32_t* pos, int64_t npairs) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3 * npairs; i += (int64_t)gridDim.x * blockDim.x)
-        v[3 * (int64_t)neg[i / 3] + i % 3] += v[3 * (int64_t)pos[i / 3] + i % 3];
-}
-// r = P^T b + P^T J x on free DOFs (Jx already folded), returns partial |r|^2 per block
-__global__ void k_outer64(const double* bf, const double* Jx, const uint8_t* mask, int64_t n, double* r, double* part) {
-    double s = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = mask[i] ? 0.0 : bf[i] + Jx[i];
-        r[i] = v;
-        s += v * v;
-    }
-    double acc[1] = {s};
-    block_sumK<1>(acc, part);
+// A right-hand side b with its FP64 solution x in column k of the tile; zero: x is zero (J x is not formed).
+struct Column {
+    int k;
+    const double* b;
+    double* x;
+    bool zero;
+};
+
+// The given columns' solutions with the positive sides of the faults following the negative ones.
+template <int K>
+void unfold_columns(pl_batch_solver B, const Column* cols, int count) {
+    pl_solver S = B->base;
+    if (count == 0 || S->npairs == 0) return;
+    Columns<K> C{};
+    unsigned flags = 0;
+    for (int i = 0; i < count; ++i) if (!cols[i].zero) C.x[cols[i].k] = cols[i].x, flags |= 1u << cols[i].k;
+    if (!flags) return;
+    k_b_unfold64<K><<<bgrid(3 * S->npairs * K), 256, 0, S->mesh->ctx->stream>>>(C, flags, S->d_pair_neg, S->d_pair_pos, S->npairs);
+    count_launch();
 }
 
-// FP64 true residual of right-hand side kk, r = P^T (b + J x) on free DOFs (x unfolded first for
-// faults), packed into column kk of the FP32 tile residual; returns |r|.
-int col_true_residual(pl_batch_solver B, int K, int kk, const double* b, double* x, double* rnorm) {
+// FP64 true residuals of the given columns, r = P^T (b + J x) on free DOFs (x unfolded first for
+// faults), into the FP32 tile residual; norms[i] = |r| of cols[i]. The columns' launches follow one
+// another without a host wait, which comes once, for all the norms. (One column at a time, with a copy
+// of b, separate folds, sum and packing, took 70 us each with 18,270 nodes; 14 us now.)
+template <int K>
+int true_residuals(pl_batch_solver B, const Column* cols, int count, double* norms) {
+    if (count == 0) return PL_OK;
     pl_solver S = B->base;
     cudaStream_t s = S->mesh->ctx->stream;
     const int64_t n = B->n;
-    if (S->npairs > 0) {
-        k_unfold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(x, S->d_pair_neg, S->d_pair_pos, S->npairs);
+    unfold_columns<K>(B, cols, count);
+    double* out = B->scal + 4 * kMaxTile;
+    for (int i = 0; i < count; ++i) {
+        const Column& c = cols[i];
+        if (c.zero) {
+            PLB_CUDA(cudaMemsetAsync(B->jx64, 0, n * sizeof(double), s));
+        } else {
+            const int rc = apply_J64(S, c.x, B->jx64);
+            if (rc) return rc;
+        }
+        if (S->npairs > 0) {
+            k_b_fold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(B->jx64, c.b, S->d_pair_neg, S->d_pair_pos, S->npairs);
+            count_launch();
+        }
+        FinSpec fin;
+        fin.counter = B->ticket;
+        fin.out_a = out + c.k;
+        k_b_residual64<<<vec_blocks(n), kBThreads, 0, s>>>(c.b, B->jx64, S->d_mask, n, K, c.k, B->r, B->part_a, fin);
         count_launch();
     }
-    int rc = apply_J64(S, x, B->jx64);
-    if (rc) return rc;
-    PLB_CUDA(cudaMemcpyAsync(B->r64, b, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    if (S->npairs > 0) {
-        k_fold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(B->jx64, S->d_pair_neg, S->d_pair_pos, S->npairs);
-        k_fold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(B->r64, S->d_pair_neg, S->d_pair_pos, S->npairs);
-        count_launch(2);
-    }
-    k_outer64<<<kBBlocks, kBThreads, 0, s>>>(B->r64, B->jx64, S->d_mask, n, B->r64, B->part_a);
-    k_b_finish<1><<<1, kBThreads, 0, s>>>(B->part_a, kBBlocks, B->scal + 4 * kMaxTile, nullptr);
-    k_b_pack<<<bgrid(n), 256, 0, s>>>(B->r64, n, K, kk, B->r);
-    count_launch(3);
-    double h;
-    PLB_CUDA(cudaMemcpyAsync(&h, B->scal + 4 * kMaxTile, sizeof(double), cudaMemcpyDeviceToHost, s));
+    double h[K];
+    PLB_CUDA(cudaMemcpyAsync(h, out, K * sizeof(double), cudaMemcpyDeviceToHost, s));
     PLB_CUDA(cudaStreamSynchronize(s));
-    *rnorm = std::sqrt(h);
+    for (int i = 0; i < count; ++i) norms[i] = std::sqrt(h[cols[i].k]);
     return PL_OK;
+}
+
+// The given columns' FP32 corrections added to their solutions (columns with x null: dropped) and cleared.
+template <int K>
+void flush_columns(pl_batch_solver B, const Column* cols, int count) {
+    if (count == 0) return;
+    Columns<K> C{};
+    unsigned flags = 0;
+    for (int i = 0; i < count; ++i) C.x[cols[i].k] = cols[i].x, flags |= 1u << cols[i].k;
+    k_b_flush<K><<<bgrid(B->n * K), 256, 0, B->base->mesh->ctx->stream>>>(B->x, C, flags, B->base->d_mask, B->n);
+    count_launch();
 }
 
 // All right-hand sides with reliable updates (van der Vorst and Ye, "Residual replacement
@@ -1921,40 +1986,42 @@ int solve_reliable(pl_batch_solver B, int nrhs, const double* const* bs, double*
     int rc = PL_OK;
     PLB_CUDA(cudaMemsetAsync(B->r, 0, n * K * sizeof(float), s));
     PLB_CUDA(cudaMemsetAsync(B->x, 0, n * K * sizeof(float), s));
-    // final FP64 solution of right-hand side j (faults: the positive side follows the negative)
-    auto finish_rhs = [&](int j) {
-        if (S->npairs > 0) {
-            k_unfold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(xs[j], S->d_pair_neg, S->d_pair_pos, S->npairs);
+    // the columns of `free` take the next pending right-hand sides with a nonzero residual (r = b, x = 0);
+    // a column that finds none stays inactive, its residual zero
+    auto assign = [&](unsigned free) -> int {
+        for (int k = 0; k < K; ++k)
+            if (free >> k & 1) slot[k] = -1, act[k] = 0;
+        while (free && next < nrhs) {
+            Column cols[K];
+            double norms[K];
+            int count = 0, js[K];
+            for (int k = 0; k < K && next < nrhs; ++k) {
+                if (!(free >> k & 1)) continue;
+                js[count] = next++;
+                PLB_CUDA(cudaMemsetAsync(xs[js[count]], 0, n * sizeof(double), s));
+                cols[count] = {k, bs[js[count]], xs[js[count]], true};
+                ++count;
+            }
+            const int r2 = true_residuals<K>(B, cols, count, norms);
+            if (r2) return r2;
+            B->outer_iterations += count;
+            for (int i = 0; i < count; ++i) {
+                if (!(norms[i] > 0.0)) continue;
+                const int k = cols[i].k;
+                slot[k] = js[i];
+                act[k] = 1;
+                bnorm[k] = rref[k] = norms[i];
+                iters[k] = 0;
+                free &= ~(1u << k);
+            }
+        }
+        if (free) {  // no right-hand side left
+            k_b_flush<K><<<bgrid(n * K), 256, 0, s>>>(B->r, Columns<K>{}, free, S->d_mask, n);
             count_launch();
         }
-    };
-    // column k takes the next pending right-hand side with a nonzero residual (r = b, x = 0)
-    auto assign = [&](int k) -> int {
-        slot[k] = -1;
-        act[k] = 0;
-        while (next < nrhs) {
-            const int j = next++;
-            PLB_CUDA(cudaMemsetAsync(xs[j], 0, n * sizeof(double), s));
-            double bn = 0.0;
-            int r2 = col_true_residual(B, K, k, bs[j], xs[j], &bn);
-            if (r2) return r2;
-            B->outer_iterations++;
-            if (bn > 0.0) {
-                slot[k] = j;
-                act[k] = 1;
-                bnorm[k] = rref[k] = bn;
-                iters[k] = 0;
-                return PL_OK;
-            }
-            finish_rhs(j);
-        }
-        // no right-hand side left: the column's residual is cleared (it stays inactive)
-        k_b_col_zero<<<bgrid(n), 256, 0, s>>>(B->r, n, K, k);
-        count_launch();
         return PL_OK;
     };
-    for (int k = 0; k < K; ++k)
-        if ((rc = assign(k)) != PL_OK) return rc;
+    if ((rc = assign((1u << K) - 1)) != PL_OK) return rc;
     k_b_init<K><<<kBBlocks, kBThreads, 0, s>>>(B->r, B->z, B->p, S->d_mask, S->d_pinv32, B->nnodes, B->part_a, B->part_b);
     k_b_finish<K><<<K, kBThreads, 0, s>>>(B->part_a, kBBlocks, B->scal, nullptr);
     k_b_finish<K><<<K, kBThreads, 0, s>>>(B->part_b, kBBlocks, B->scal + 3 * K, nullptr);
@@ -1976,7 +2043,8 @@ int solve_reliable(pl_batch_solver B, int nrhs, const double* const* bs, double*
         B->inner_iterations += chunk;
         PLB_CUDA(cudaMemcpyAsync(h, B->scal, 4 * K * sizeof(double), cudaMemcpyDeviceToHost, s));
         PLB_CUDA(cudaStreamSynchronize(s));
-        bool changed = false, update_z = false;
+        Column flush[K], todo[K];
+        int nflush = 0, ntodo = 0;
         for (int k = 0; k < K; ++k) {
             fresh[k] = replaced[k] = false;
             if (!act[k]) continue;
@@ -1986,51 +2054,51 @@ int solve_reliable(pl_batch_solver B, int nrhs, const double* const* bs, double*
             // FP32 breakdown (the iterated residual not a number or far above the last true one):
             // drop the column's FP32 correction and restart it from its FP64 true residual
             const bool broke = !(rn == rn) || rn > kBreakdownGrowth * rref[k];
-            if (broke) {
-                if (++breakdowns[k] > kMaxBreakdowns)
-                    return fail(PL_ERR_NOT_CONVERGED, "batched PCG broke down repeatedly");
-                k_b_col_zero<<<bgrid(n), 256, 0, s>>>(B->x, n, K, k);
-                count_launch();
-                double rt = 0.0;
-                if ((rc = col_true_residual(B, K, k, bs[slot[k]], xs[slot[k]], &rt)) != PL_OK) return rc;
-                B->outer_iterations++;
-                rref[k] = rt;
-                fresh[k] = update_z = true;  // p = z again
-                continue;
-            }
-            if (rn > B->reliable_delta * rref[k] && rn > 0.5 * S->rtol * bnorm[k]) continue;
+            if (!broke && rn > B->reliable_delta * rref[k] && rn > 0.5 * S->rtol * bnorm[k]) continue;
+            if (broke && ++breakdowns[k] > kMaxBreakdowns)
+                return fail(PL_ERR_NOT_CONVERGED, "batched PCG broke down repeatedly");
             const int j = slot[k];
-            k_b_unpack_add<<<bgrid(n), 256, 0, s>>>(B->x, n, K, k, S->d_mask, xs[j]);
-            k_b_col_zero<<<bgrid(n), 256, 0, s>>>(B->x, n, K, k);
-            count_launch(2);
-            double rt = 0.0;
-            if ((rc = col_true_residual(B, K, k, bs[j], xs[j], &rt)) != PL_OK) return rc;
-            B->reliable_updates++;
-            B->outer_iterations++;
-            if (rt <= S->rtol * bnorm[k]) {
-                B->max_rel_residual = std::max(B->max_rel_residual, rt / bnorm[k]);
-                finish_rhs(j);
-                if ((rc = assign(k)) != PL_OK) return rc;
-                changed = true;
-                if (act[k]) fresh[k] = update_z = true;
-                continue;
-            }
-            rref[k] = rt;
-            replaced[k] = update_z = true;
+            fresh[k] = broke;  // p = z again
+            flush[nflush++] = {k, bs[j], broke ? nullptr : xs[j], false};
+            todo[ntodo++] = {k, bs[j], xs[j], false};
         }
+        flush_columns<K>(B, flush, nflush);
+        double norms[K];
+        if ((rc = true_residuals<K>(B, todo, ntodo, norms)) != PL_OK) return rc;
+        B->outer_iterations += ntodo;
+        unsigned done = 0, update = 0, start = 0;
+        for (int i = 0; i < ntodo; ++i) {
+            const int k = todo[i].k;
+            rref[k] = norms[i];
+            if (fresh[k]) continue;
+            B->reliable_updates++;
+            if (norms[i] <= S->rtol * bnorm[k]) {
+                B->max_rel_residual = std::max(B->max_rel_residual, norms[i] / bnorm[k]);
+                done |= 1u << k;  // (its solution is unfolded: true_residuals)
+            } else {
+                replaced[k] = true;
+            }
+        }
+        const bool changed = done != 0;
+        if (changed && (rc = assign(done)) != PL_OK) return rc;
+        for (int k = 0; k < K; ++k) {
+            if ((done >> k & 1) && act[k]) fresh[k] = true;
+            if (fresh[k]) start |= 1u << k;
+            if (fresh[k] || replaced[k]) update |= 1u << k;
+        }
+        const bool update_z = update != 0;
         if (update_z && B->mg) {
             // multigrid (flexible steps): no V-cycle of the whole tile here, which would cost as
             // much as an iteration. A replaced residual keeps its column's z, the V-cycle of the
             // residual it replaces (they differ by the FP32 drift, which the flexible step
             // absorbs); a new (or restarted) column starts from point-block Jacobi, z = P r, and
             // meets the V-cycle at its next iteration. Then r.z of every column again.
-            for (int k = 0; k < K; ++k)
-                if (fresh[k]) {
-                    k_b_col_prec<<<kBBlocks, kBThreads, 0, s>>>(B->r, B->z, S->d_mask, S->d_pinv32, B->nnodes, K, k,
-                                                                B->part_a);
-                    k_b_col_copy<<<bgrid(n), 256, 0, s>>>(B->p, B->z, n, K, k);
-                    count_launch(2);
-                }
+            if (start) {
+                k_b_cols_prec<K><<<vec_blocks(B->nnodes * K), kBThreads, 0, s>>>(B->r, B->z, B->p, S->d_mask, S->d_pinv32, B->nnodes,
+                                                                                 start, start, B->part_a, B->scal,
+                                                                                 B->scal + 4 * kMaxTile, B->ticket);
+                count_launch();
+            }
             k_b_rz<K><<<kBBlocks, kBThreads, 0, s>>>(B->r, B->z, nullptr, S->d_mask, B->n, B->part_a, B->part_b, FinSpec());
             k_b_finish<K><<<K, kBThreads, 0, s>>>(B->part_a, kBBlocks, B->scal, nullptr);
             count_launch(2);
@@ -2041,21 +2109,18 @@ int solve_reliable(pl_batch_solver B, int nrhs, const double* const* bs, double*
                 if ((rc = precond_apply<K>(B)) != PL_OK) return rc;
                 k_b_finish<K><<<K, kBThreads, 0, s>>>(B->part_a, kBBlocks, B->scal, nullptr);
                 count_launch();
+                // a new right-hand side starts from p = z
+                for (int k = 0; k < K; ++k)
+                    if (fresh[k]) {
+                        k_b_col_copy<<<bgrid(n), 256, 0, s>>>(B->p, B->z, n, K, k);
+                        count_launch();
+                    }
             } else {
-                for (int k = 0; k < K; ++k) {
-                    if (!fresh[k] && !replaced[k]) continue;
-                    k_b_col_prec<<<kBBlocks, kBThreads, 0, s>>>(B->r, B->z, S->d_mask, S->d_pinv32, B->nnodes, K, k,
-                                                                B->part_a);
-                    k_b_finish<1><<<1, kBThreads, 0, s>>>(B->part_a, kBBlocks, B->scal + k, nullptr);
-                    count_launch(2);
-                }
+                k_b_cols_prec<K><<<vec_blocks(B->nnodes * K), kBThreads, 0, s>>>(B->r, B->z, B->p, S->d_mask, S->d_pinv32, B->nnodes,
+                                                                                 update, start, B->part_a, B->scal,
+                                                                                 B->scal + 4 * kMaxTile, B->ticket);
+                count_launch();
             }
-            // a new right-hand side starts from p = z
-            for (int k = 0; k < K; ++k)
-                if (fresh[k]) {
-                    k_b_col_copy<<<bgrid(n), 256, 0, s>>>(B->p, B->z, n, K, k);
-                    count_launch();
-                }
         }
         if (changed) PLB_CUDA(cudaMemcpyAsync(B->active, act, K * sizeof(int), cudaMemcpyHostToDevice, s));
         any = false;
@@ -2071,51 +2136,30 @@ int solve_tile(pl_batch_solver B, int nact, const double* const* bs, double* con
     cudaStream_t s = S->mesh->ctx->stream;
     const int64_t n = B->n;
     double bnorm[kMaxTile] = {0}, rn[kMaxTile] = {0};
+    Column cols[K];
     for (int k = 0; k < nact; ++k) PLB_CUDA(cudaMemsetAsync(xs[k], 0, n * sizeof(double), s));
     for (int outer = 0; outer < 30; ++outer) {
         // FP64 outer residual of every RHS of the tile, packed into the FP32 tile
         PLB_CUDA(cudaMemsetAsync(B->r, 0, n * K * sizeof(float), s));
         bool done = true;
+        for (int k = 0; k < nact; ++k) cols[k] = {k, bs[k], xs[k], outer == 0};
+        int rc = true_residuals<K>(B, cols, nact, rn);
+        if (rc) return rc;
         for (int k = 0; k < nact; ++k) {
-            if (S->npairs > 0) {
-                k_unfold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(xs[k], S->d_pair_neg, S->d_pair_pos, S->npairs);
-                count_launch();
-            }
-            int rc = apply_J64(S, xs[k], B->jx64);
-            if (rc) return rc;
-            PLB_CUDA(cudaMemcpyAsync(B->r64, bs[k], n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-            if (S->npairs > 0) {
-                k_fold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(B->jx64, S->d_pair_neg, S->d_pair_pos, S->npairs);
-                k_fold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(B->r64, S->d_pair_neg, S->d_pair_pos, S->npairs);
-                count_launch(2);
-            }
-            k_outer64<<<kBBlocks, kBThreads, 0, s>>>(B->r64, B->jx64, S->d_mask, n, B->r64, B->part_a);
-            k_b_finish<1><<<1, kBThreads, 0, s>>>(B->part_a, kBBlocks, B->scal, nullptr);
-            k_b_pack<<<bgrid(n), 256, 0, s>>>(B->r64, n, K, k, B->r);
-            count_launch(3);
-            double h;
-            PLB_CUDA(cudaMemcpyAsync(&h, B->scal, sizeof(double), cudaMemcpyDeviceToHost, s));
-            PLB_CUDA(cudaStreamSynchronize(s));
-            rn[k] = std::sqrt(h);
             if (outer == 0) bnorm[k] = rn[k];
             if (rn[k] > S->rtol * bnorm[k] && bnorm[k] > 0.0) done = false;
         }
         B->outer_iterations++;
         if (done) break;
         int it = 0;
-        int rc = tile_pcg<K>(B, nact, S->inner_rtol, S->max_iter, &it);
+        rc = tile_pcg<K>(B, nact, S->inner_rtol, S->max_iter, &it);
         if (rc && rc != PL_ERR_NOT_CONVERGED) return rc;
         B->inner_iterations += it;
-        for (int k = 0; k < nact; ++k) {
-            k_b_unpack_add<<<bgrid(n), 256, 0, s>>>(B->x, n, K, k, S->d_mask, xs[k]);
-            count_launch();
-        }
+        flush_columns<K>(B, cols, nact);
     }
+    for (int k = 0; k < nact; ++k) cols[k].zero = false;
+    unfold_columns<K>(B, cols, nact);
     for (int k = 0; k < nact; ++k) {
-        if (S->npairs > 0) {
-            k_unfold64<<<bgrid(3 * S->npairs), 256, 0, s>>>(xs[k], S->d_pair_neg, S->d_pair_pos, S->npairs);
-            count_launch();
-        }
         const double rel = bnorm[k] > 0.0 ? rn[k] / bnorm[k] : 0.0;
         B->max_rel_residual = std::max(B->max_rel_residual, rel);
         if (rel > S->rtol) return fail(PL_ERR_NOT_CONVERGED, "batched refinement did not reach the tolerance");
@@ -2150,7 +2194,6 @@ int pl_batch_solver_create(pl_solver base, int tile, pl_batch_solver* out) {
     A(&B->part_b, (size_t)kBBlocks * kMaxTile);
     A(&B->ticket, 1);
     if (e == cudaSuccess) e = cudaMemset(B->ticket, 0, sizeof(unsigned int));
-    A(&B->r64, B->n);
     A(&B->jx64, B->n);
     // the cell-block layout is built here, outside any stream capture
     if (e == cudaSuccess) {
@@ -2355,7 +2398,7 @@ int pl_batch_solver_destroy(pl_batch_solver B) {
     if (B->ev_in) cudaEventDestroy(B->ev_in);
     if (B->ev_out) cudaEventDestroy(B->ev_out);
     if (B->stream) cudaStreamDestroy(B->stream);
-    void* ptrs[] = {B->r, B->z, B->p, B->q, B->x, B->scal, B->active, B->part_a, B->part_b, B->r64, B->jx64, B->res, B->d, B->ticket};
+    void* ptrs[] = {B->r, B->z, B->p, B->q, B->x, B->scal, B->active, B->part_a, B->part_b, B->jx64, B->res, B->d, B->ticket};
     for (void* p : ptrs) dev_free(p, m->ctx->stream);
     pl_solver base = B->base;
     delete B;

@@ -341,6 +341,39 @@ def test_batched_operator_cell_orders(ctx, window, tile, integrators):
         assert torch.linalg.norm(x - ref) <= 1e-8 * torch.linalg.norm(ref)
 
 
+# fewer right-hand sides than columns; more, with zero ones in the first tile, in a refill and last; all zero
+@pytest.mark.parametrize("zero", [(0, 1, 0), (1, 0, 1, 1, 0, 0, 1, 0, 1, 0, 1), (1,) * 6])
+@pytest.mark.parametrize("reliable", [True, False])
+def test_batched_columns_with_zero_right_hand_sides(ctx, zero, reliable):
+    """Tiles of 4 on a faulted mesh: columns that start, finish and stay empty match FP64 solves of one
+    right-hand side at a time to <= 1e-8; zero right-hand sides give zero."""
+    import torch
+    from pylith_b200 import feassemble as FA
+
+    rng = np.random.default_rng(23)
+    mesh = M.box_tet_kuhn(6, 5, 4, fault_x=0.0, seed=3)
+    cons = np.zeros((mesh.num_nodes, 3), dtype=bool)
+    cons[M.boundary_mask(mesh, 0, "neg")] = True
+    cons = np.concatenate([cons.ravel(), np.zeros(3 * mesh.num_lagrange, dtype=bool)])
+    dm = FA.DeviceMesh(ctx, mesh)
+    ig = MAT.IsotropicLinearElasticity(*MAT.lognormal_elastic(mesh.num_cells, seed=24)).create_integrator(dm)
+    bs = [torch.from_numpy(rng.standard_normal(mesh.num_dof) * (1 - z)).cuda() for z in zero]
+    refined = FA.Solver(dm, cons, [ig], rtol=1e-11, precision=FA.Solver.FP32_REFINED, inner_rtol=1e-4)
+    refined.setup()
+    batch = FA.BatchSolver(refined, 4)
+    batch.set_reliable(reliable)
+    xs = [torch.full_like(b, np.nan) for b in bs]
+    batch.solve(bs, xs)
+    S = FA.Solver(dm, cons, [ig], rtol=1e-11)
+    S.setup()
+    for b, x, z in zip(bs, xs, zero):
+        ref = torch.zeros_like(b)
+        if not z:
+            S.solve(b, ref)
+        ctx.synchronize()
+        assert torch.linalg.norm(x - ref) <= 1e-8 * torch.linalg.norm(ref)
+
+
 def test_batched_chebyshev_jacobi_eigen_estimate_and_solutions(ctx, oracle_lib):
     """Chebyshev-Jacobi preconditioning of the batched FP32 PCG on a Kuhn tetrahedral mesh: the
     power-iteration estimate of lambda_max(P A) lies within [0.85, 1.0001] of the largest
