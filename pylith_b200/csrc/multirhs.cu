@@ -214,41 +214,30 @@ PL_D void sum_partials_last_block(const double* partials, double* out, double* p
     sum_partials_last_block_in<K>(partials, out, prev, sh);
 }
 
-// The final sums of two partial arrays at once: fin.out_a (its old value to fin.prev_a) and fin.out_b.
+// The final sum of partials[count][K] for right-hand side threadIdx.x % K, formed by every block of the
+// kernel that uses it (all in the same order): no ticket, fence and last block at the end of the kernel
+// that wrote the partials, and the loads overlap the caller's own. sh: kBThreads / 32 * K doubles.
 template <int K>
-PL_D void sum2_partials_last_block(const double* pa, const double* pb, const FinSpec& fin) {
-    __shared__ double sh[2][kBThreads / 32][K];
+PL_D double sum_partials(const double* __restrict__ partials, int count, double (*sh)[K]) {
     const int k = threadIdx.x % K;
-    constexpr int STEP = kBThreads / K, U = 5;
-    double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x / K; i < (int)gridDim.x; i += U * STEP) {
-        double va[U], vb[U];
+    constexpr int STEP = kBThreads / K, U = 10;
+    double s = 0.0;
+    for (int b = threadIdx.x / K; b < count; b += U * STEP) {
+        double v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const bool on = i + u * STEP < (int)gridDim.x;
-            va[u] = on ? __ldcg(&pa[(i + u * STEP) * K + k]) : 0.0;
-            vb[u] = on ? __ldcg(&pb[(i + u * STEP) * K + k]) : 0.0;
-        }
+        for (int u = 0; u < U; ++u) v[u] = b + u * STEP < count ? partials[(b + u * STEP) * K + k] : 0.0;
 #pragma unroll
-        for (int u = 0; u < U; ++u) a += va[u], b += vb[u];
+        for (int u = 0; u < U; ++u) s += v[u];
     }
 #pragma unroll
-    for (int o = K; o < 32; o <<= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
+    for (int o = K; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l < K) sh[0][w][l] = a, sh[1][w][l] = b;
+    if (l < K) sh[w][l] = s;
     __syncthreads();
-    if (threadIdx.x < 2 * K) {
-        const int kk = threadIdx.x % K, which = threadIdx.x / K;
-        double t = 0.0;
+    double t = 0.0;
 #pragma unroll
-        for (int i = 0; i < kBThreads / 32; ++i) t += sh[which][i][kk];
-        double* out = which ? fin.out_b : fin.out_a;
-        if (!which && fin.prev_a) fin.prev_a[kk] = out[kk];
-        out[kk] = t;
-    }
+    for (int i = 0; i < kBThreads / 32; ++i) t += sh[i][k];
+    return t;
 }
 
 // Block metadata in shared memory (two buffers: the gather reads one while the next block's is
@@ -545,8 +534,9 @@ __global__ void __launch_bounds__(kMultiBlockCells, 3) k_tet_blocked_jv32_multi(
 // pair instead of 24); with cf = cofactors / 6 and lambda, mu times 6 / det one set of factors serves
 // both the gradient and the test functions. In the sums a thread takes a node's three components (one
 // component per thread: 16.3 us for 15.5). Measured with 94,080 cells and K = 8, in the PCG on B200:
-// 18.1 -> 15.5 us against k_tet_blocked_jv32_multi; bound by issue and shared memory in about equal
-// parts, with a tail of 3 us for the energies' last-CTA sum. 3 CTAs per SM are as fast, 5 spill (28 us).
+// 18.1 -> 15.5 us against k_tet_blocked_jv32_multi, 13.6 with the energies' partials summed by the kernel
+// that uses them; bound by issue and shared memory in about equal parts. 3 CTAs per SM are as fast, 5
+// spill (28 us).
 template <int LD>
 constexpr int kPairMultiCtas = LD == kPairSmallLd ? 4 : 3;  // by shared memory and registers
 
@@ -757,12 +747,13 @@ __global__ void __launch_bounds__(kPairThreads, kPairMultiCtas<LD>)
 
 template <int K, int LD>
 void launch_pair_multi(const DomainParams& p, const PairArrays& A, const float* v, float* out, bool store_owned, double* part,
-                       const double* scal, const FinSpec& fin, cudaStream_t s) {
+                       const double* scal, const FinSpec& fin, int* npart, cudaStream_t s) {
     constexpr int chunks = K / MultiChunk<K>::value;
     constexpr size_t smem = sizeof(PairSmem<float, LD, MultiChunk<K>::value>);
     ensure_kernel_smem((const void*)k_tet_pair_jv32_multi<K, LD>, smem);
-    const int64_t gx = std::max<int64_t>(1, (int64_t)sm_count() * kPairMultiCtas<LD> / chunks);
-    k_tet_pair_jv32_multi<K, LD><<<dim3((unsigned)std::min(A.nblocks, gx), chunks), kPairThreads, smem, s>>>(
+    const int64_t gx = std::min(A.nblocks, std::max<int64_t>(1, (int64_t)sm_count() * kPairMultiCtas<LD> / chunks));
+    if (npart) *npart = (int)gx;
+    k_tet_pair_jv32_multi<K, LD><<<dim3((unsigned)gx, chunks), kPairThreads, smem, s>>>(
         p, A, v, out, store_owned, part, scal, fin);
     count_launch();
 }
@@ -915,28 +906,52 @@ __global__ void __launch_bounds__(kBThreads) k_b_pq(const float* p, const float*
     if (fin.counter && take_last_ticket(fin.counter)) sum_partials_last_block<K>(part, fin.out_a, fin.prev_a);
 }
 
+// P (row-major 3x3) in.
+PL_D void mat3_apply(const float (&P)[9], const float (&in)[3], float (&out)[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[c] = P[3 * c] * in[0] + P[3 * c + 1] * in[1] + P[3 * c + 2] * in[2];
+}
+
 // alpha_k = active_k ? rz_k / pq_k : 0; r += alpha q; z = P r (not stored: k_b_pupdate_jacobi forms it
-// again from r); partial rz, rr. One thread per (node, rhs), its loads independent of each other:
-// on small meshes the kernel is one chain of latencies, loads to final sums.
+// again from r); partial rz, rr. pq: the sum of npart partials (npart 0: scal's). scal holds rz, rz_old,
+// pq, rr [K] each; block 0 sets rz_old = rz and pq, which no block reads here. One thread per (node,
+// rhs): on small meshes the kernel is one chain of latencies, so its first loads are issued before the
+// partials are summed.
 template <int K>
 __global__ void __launch_bounds__(kBThreads) k_b_update(float* __restrict__ r, const float* __restrict__ q,
                                                         const uint8_t* __restrict__ mask, const float* __restrict__ P,
-                                                        int64_t nnodes, const double* __restrict__ rz,
-                                                        const double* __restrict__ pq, const int* __restrict__ active,
-                                                        double* part_rz, double* part_rr, FinSpec fin) {
+                                                        int64_t nnodes, double* scal, const double* __restrict__ part_pq, int npart,
+                                                        const int* __restrict__ active, double* part_rz, double* part_rr) {
+    __shared__ double sh[kBThreads / 32][K];
     const int k = threadIdx.x % K;  // blockDim and the grid stride are multiples of K
-    const float alpha = active[k] ? safe_step_f32(rz[k], pq[k]) : 0.0f;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    float r0[3], q0[3], p0[9];
+    auto load = [&] {
+        if (t >= nnodes * K) return;
+        const int64_t nd = t / K;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            r0[c] = r[(3 * nd + c) * K + k];
+            q0[c] = mask[3 * nd + c] ? 0.0f : q[(3 * nd + c) * K + k];
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) p0[c] = P[9 * nd + c];
+    };
+    load();
+    const double rz = scal[k], pq = npart ? sum_partials<K>(part_pq, npart, sh) : scal[2 * K + k];
+    if (blockIdx.x == 0 && threadIdx.x < K) {
+        scal[K + k] = rz;
+        if (npart) scal[2 * K + k] = pq;
+    }
+    const float alpha = active[k] ? safe_step_f32(rz, pq) : 0.0f;
     double srz = 0.0, srr = 0.0;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nnodes * K; t += (int64_t)gridDim.x * blockDim.x) {
+    for (; t < nnodes * K; t += stride, load()) {
         const int64_t nd = t / K;
         float rn[3], zz[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int64_t i = (3 * nd + c) * K + k;
-            const float r0 = r[i], q0 = q[i];
-            rn[c] = mask[3 * nd + c] ? r0 : r0 + alpha * q0;
-        }
-        pinv_local(P, nd, rn, zz);
+        for (int c = 0; c < 3; ++c) rn[c] = r0[c] + alpha * q0[c];
+        mat3_apply(p0, rn, zz);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             r[(3 * nd + c) * K + k] = rn[c];
@@ -945,7 +960,6 @@ __global__ void __launch_bounds__(kBThreads) k_b_update(float* __restrict__ r, c
         }
     }
     block_sum2_by_rhs<K>(srz, srr, part_rz, part_rr);
-    if (fin.counter && take_last_ticket(fin.counter)) sum2_partials_last_block<K>(part_rz, part_rr, fin);
 }
 
 // x += alpha p (free DOFs; alpha_k = rz_old_k / pq_k, the step of this iteration, whose r.z is
@@ -974,32 +988,51 @@ __global__ void k_b_pupdate(float* x, float* p, const float* z, const uint8_t* m
 }
 
 // k_b_pupdate for the point-block Jacobi preconditioner, forming z = P r from r (one thread per
-// (node, rhs)) instead of reading a stored z; it also clears q for the next operator application.
+// (node, rhs)) instead of reading a stored z; it also clears q for the next operator application. rz is
+// the sum of k_b_update's npart partials; block 0 stores it and rr in scal (as k_b_update: no block
+// reads them here).
 template <int K>
 __global__ void __launch_bounds__(kBThreads) k_b_pupdate_jacobi(float* __restrict__ x, float* __restrict__ p,
                                                                 const float* __restrict__ r, float* __restrict__ q,
                                                                 const uint8_t* __restrict__ mask, const float* __restrict__ P,
-                                                                int64_t nnodes,
-                                                                const double* rz, const double* rz_old,
-                                                                const double* pq, const int* active) {
+                                                                int64_t nnodes, double* scal, const double* __restrict__ part_rz,
+                                                                const double* __restrict__ part_rr, int npart,
+                                                                const int* __restrict__ active) {
+    __shared__ double sh[2][kBThreads / 32][K];
     const int k = threadIdx.x % K;  // blockDim and the grid stride are multiples of K
-    const float alpha = active[k] ? safe_step_f32(rz_old[k], pq[k]) : 0.0f;
-    const float beta = (active[k] && rz_old[k] != 0.0) ? (float)(rz[k] / rz_old[k]) : 0.0f;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nnodes * K; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    float rv[3], pv[3], xv[3], pm[3], p0[9];  // pm: p on free DOFs
+    auto load = [&] {
+        if (t >= nnodes * K) return;
         const int64_t nd = t / K;
-        float rv[3], pv[3], xv[3], zz[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int64_t i = (3 * nd + c) * K + k;
             rv[c] = r[i];
             pv[c] = p[i];
-            xv[c] = mask[3 * nd + c] ? x[i] : x[i] + alpha * pv[c];
+            xv[c] = x[i];
+            pm[c] = mask[3 * nd + c] ? 0.0f : pv[c];
         }
-        pinv_local(P, nd, rv, zz);
+#pragma unroll
+        for (int c = 0; c < 9; ++c) p0[c] = P[9 * nd + c];
+    };
+    load();
+    const double rz = sum_partials<K>(part_rz, npart, sh[0]), rz_old = scal[K + k], pq = scal[2 * K + k];
+    if (blockIdx.x == 0) {
+        const double rr = sum_partials<K>(part_rr, npart, sh[1]);
+        if (threadIdx.x < K) scal[k] = rz, scal[3 * K + k] = rr;
+    }
+    const float alpha = active[k] ? safe_step_f32(rz_old, pq) : 0.0f;
+    const float beta = (active[k] && rz_old != 0.0) ? (float)(rz / rz_old) : 0.0f;
+    for (; t < nnodes * K; t += stride, load()) {
+        const int64_t nd = t / K;
+        float zz[3];
+        mat3_apply(p0, rv, zz);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int64_t i = (3 * nd + c) * K + k;
-            x[i] = xv[c];
+            x[i] = xv[c] + alpha * pm[c];
             p[i] = zz[c] + beta * pv[c];
             q[i] = 0.0f;
         }
@@ -1243,12 +1276,17 @@ __global__ void __launch_bounds__(kBThreads) k_b_cols_prec(const float* __restri
 }
 
 // Blocks of the vector kernels whose partial sums are counted by gridDim.x: two items per thread, at
-// most kBBlocks. Small tiles are then not dominated by blocks that only take a ticket (18,270 nodes x
-// 8: 14.1 us per update with 1,184 blocks and two passes over their partial sums one load at a time,
-// 5.7 us now; one or four items per thread are 1 to 2 % slower per solve).
+// most kBBlocks. Small tiles are then not dominated by blocks that only write a partial sum (18,270
+// nodes x 8: 14.1 us per update with 1,184 blocks, two passes over their partial sums one load at a time
+// and a last block; 3.9 us now. One or four items per thread are 1 to 2 % slower per solve).
 static int vec_blocks(int64_t items) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((items + 2 * kBThreads - 1) / (2 * kBThreads), kBBlocks));
 }
+
+// The same for the two vector kernels of the point-Jacobi PCG, whose blocks each read all partial sums:
+// four per SM (1,179,648 cells x 8: update 15.0, pupdate 21.7 us; with two 22.7 and 23.4, with eight 18.4
+// and 24.1; with 1,184 blocks and last-block sums 21.7 and 21.5).
+static int pcg_blocks(int64_t items) { return std::min(vec_blocks(items), 4 * sm_count()); }
 
 static int bgrid(int64_t n) { return (int)std::min<int64_t>((n + 255) / 256, 148 * 8); }
 
@@ -1265,6 +1303,7 @@ struct pl_batch_solver_s {
     int* active = nullptr;
     double* part_a = nullptr;
     double* part_b = nullptr;
+    double* part_c = nullptr;
     unsigned int* ticket = nullptr;  // last-block counter of the fused reductions (zero between kernels)
     double* jx64 = nullptr;   // single-RHS FP64 action
     cudaGraphExec_t graph = nullptr;
@@ -1320,10 +1359,10 @@ bool fuses_energies(pl_batch_solver B) {
 
 // out = J v for the tile's K vectors; with pq (single-integrator operators only, see
 // fuses_energies), the energies v.(A v) are summed by the same launch into pq[K] (scaled by the
-// tile's current r.z, B->scal[0..K)).
+// tile's current r.z, B->scal[0..K)); with npart, only their partials, *npart rows of `part`.
 template <int K>
 int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq, unsigned int* ticket, double* part,
-                  const double* scal, bool cleared = false) {
+                  const double* scal, bool cleared = false, int* npart = nullptr) {
     pl_mesh m = S->mesh;
     cudaStream_t s = m->ctx->stream;
     if (pq && S->ops.size() != 1) return fail(PL_ERR_UNSUPPORTED, "fused energies need a single integrator");
@@ -1347,16 +1386,16 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
         if (m->cell_type != PL_CELL_TET4 || ig->j3 != K_ILE_JF3VU || ig->subset)
             return fail(PL_ERR_UNSUPPORTED, "batched solves support P1 tetrahedra with isotropic linear elasticity");
         FinSpec fin;
-        if (pq) {
+        if (pq && !npart) {
             fin.counter = ticket;
             fin.out_a = pq;
         }
         if (pairs) {
             const PairArrays A = pair_arrays_of(*m->pair, nullptr, reduced);
             if (m->pair->ld == kPairSmallLd)
-                launch_pair_multi<K, kPairSmallLd>(pp, A, v, out, first, pq ? part : nullptr, scal, fin, s);
+                launch_pair_multi<K, kPairSmallLd>(pp, A, v, out, first, pq ? part : nullptr, scal, fin, npart, s);
             else
-                launch_pair_multi<K, kPairMaxNodes>(pp, A, v, out, first, pq ? part : nullptr, scal, fin, s);
+                launch_pair_multi<K, kPairMaxNodes>(pp, A, v, out, first, pq ? part : nullptr, scal, fin, npart, s);
             first = false;
             continue;
         }
@@ -1376,6 +1415,7 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
             per_sm_smem = smem;
         }
         const int grid = (int)std::min<int64_t>(L.num_blocks, (int64_t)sm_count() * per_sm);
+        if (npart) *npart = grid;
         k_tet_blocked_jv32_multi<K><<<grid, kMultiBlockCells, smem, s>>>(
             pp, L.d_cell_begin, L.d_block_node_begin, reduced ? L.d_slot_node_red : L.d_slot_node,
             (const ushort4*)L.d_local_cells, L.d_inc_off, L.d_inc,
@@ -1391,8 +1431,8 @@ int jv32_multi_on(pl_solver S, int64_t n, const float* v, float* out, double* pq
 }
 
 template <int K>
-int jv32_multi(pl_batch_solver B, const float* v, float* out, double* pq = nullptr, bool cleared = false) {
-    return jv32_multi_on<K>(B->base, B->n, v, out, pq, B->ticket, B->part_a, B->scal, cleared);
+int jv32_multi(pl_batch_solver B, const float* v, float* out, double* pq = nullptr, bool cleared = false, int* npart = nullptr) {
+    return jv32_multi_on<K>(B->base, B->n, v, out, pq, B->ticket, B->part_a, B->scal, cleared, npart);
 }
 
 // z = q(P A) P r with the Chebyshev coefficients of the solver; partial r.z into part_a (and,
@@ -1714,9 +1754,12 @@ int pcg_iteration(pl_batch_solver B, bool first) {
     double* rz_old = B->scal + K;
     double* pq = B->scal + 2 * K;
     double* rr = B->scal + 3 * K;
-    // the final sums are formed by the last block of each reduction kernel (no k_b_finish launches)
+    // the final sums are formed by the last block of each reduction kernel, or (point Jacobi) by the
+    // kernel that uses them (no k_b_finish launches)
     const bool fused = fuses_energies(B);
-    int rc = jv32_multi<K>(B, B->p, B->q, fused ? pq : nullptr, !first && !tile_preconditioned(B));
+    int npq = 0;
+    int rc = jv32_multi<K>(B, B->p, B->q, fused ? pq : nullptr, !first && !tile_preconditioned(B),
+                           fused && !tile_preconditioned(B) ? &npq : nullptr);
     if (rc) return rc;
     if (!fused) {
         FinSpec fpq;
@@ -1740,18 +1783,13 @@ int pcg_iteration(pl_batch_solver B, bool first) {
         rc = precond_apply<K>(B, frz);
         if (rc) return rc;
     } else {
-        FinSpec fu;
-        fu.counter = B->ticket;
-        fu.out_a = rz;
-        fu.prev_a = rz_old;
-        fu.out_b = rr;
         // z = P r is not stored: k_b_pupdate_jacobi forms it again from r
-        k_b_update<K><<<vec_blocks(B->nnodes * K), kBThreads, 0, s>>>(B->r, B->q, S->d_mask, S->d_pinv32, B->nnodes, rz, pq,
-                                                                      B->active, B->part_a, B->part_b, fu);
-        count_launch();
-        k_b_pupdate_jacobi<K><<<vec_blocks(B->nnodes * K), kBThreads, 0, s>>>(
-            B->x, B->p, B->r, B->q, S->d_mask, S->d_pinv32, B->nnodes, rz, rz_old, pq, B->active);
-        count_launch();
+        const int g = pcg_blocks(B->nnodes * K);
+        k_b_update<K><<<g, kBThreads, 0, s>>>(B->r, B->q, S->d_mask, S->d_pinv32, B->nnodes, B->scal, B->part_a, npq, B->active,
+                                              B->part_b, B->part_c);
+        k_b_pupdate_jacobi<K><<<g, kBThreads, 0, s>>>(B->x, B->p, B->r, B->q, S->d_mask, S->d_pinv32, B->nnodes, B->scal,
+                                                      B->part_b, B->part_c, g, B->active);
+        count_launch(2);
         return PL_OK;
     }
     k_b_pupdate<K><<<kBBlocks, kBThreads, 0, s>>>(B->x, B->p, B->z, S->d_mask, B->n, rz, rz_old, pq, B->active,
@@ -2192,6 +2230,7 @@ int pl_batch_solver_create(pl_solver base, int tile, pl_batch_solver* out) {
     A(&B->active, kMaxTile);
     A(&B->part_a, (size_t)kBBlocks * kMaxTile);
     A(&B->part_b, (size_t)kBBlocks * kMaxTile);
+    A(&B->part_c, (size_t)kBBlocks * kMaxTile);
     A(&B->ticket, 1);
     if (e == cudaSuccess) e = cudaMemset(B->ticket, 0, sizeof(unsigned int));
     A(&B->jx64, B->n);
@@ -2398,7 +2437,7 @@ int pl_batch_solver_destroy(pl_batch_solver B) {
     if (B->ev_in) cudaEventDestroy(B->ev_in);
     if (B->ev_out) cudaEventDestroy(B->ev_out);
     if (B->stream) cudaStreamDestroy(B->stream);
-    void* ptrs[] = {B->r, B->z, B->p, B->q, B->x, B->scal, B->active, B->part_a, B->part_b, B->jx64, B->res, B->d, B->ticket};
+    void* ptrs[] = {B->r, B->z, B->p, B->q, B->x, B->scal, B->active, B->part_a, B->part_b, B->part_c, B->jx64, B->res, B->d, B->ticket};
     for (void* p : ptrs) dev_free(p, m->ctx->stream);
     pl_solver base = B->base;
     delete B;
