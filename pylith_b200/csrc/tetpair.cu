@@ -9,11 +9,12 @@
 // cross product are formed once. The host matches the cells of a block into pairs (98 % of them on
 // Delaunay and structured meshes); a cell left over takes a thread by itself.
 // Measured on B200 (L2 warm), residual or action against the one-cell-per-thread kernel k_tet_pad2:
-// 1,296,000 structured cells FP64 53.8 -> 45.4 us and FP32 45.8 -> 35.5; 54,737 Delaunay cells FP64
-// 9.5 -> 8.7, FP32 9.9 -> 8.7; 3,072 cells FP64 8.5 -> 6.7. What bounds it now: shared memory still
-// (reads of random nodes conflict about twofold after the numbering of bankplan.hpp), then HBM.
+// 1,296,000 structured cells FP64 53.8 -> 43.3 us and FP32 45.8 -> 33.3 (45.4 and 34.9 with whole warps
+// planned for the banks, kPlanSteps); 54,737 Delaunay cells FP64 9.5 -> 8.9, FP32 9.9 -> 8.7; 3,072 cells
+// FP64 8.5 -> 6.8. What bounds it now: shared memory still, then HBM.
 // Block size: 240 cells in 128 items with 4 CTAs per SM (FP64, at most 128 registers) measured best
-// (two launches on 1,179,648 cells 80 us); 5 and 6 CTAs 80-92 (spills), 64, 96, 192 and 256 threads
+// (two launches on 1,179,648 cells 80 us, 75 with the banks planned by halves); 5 and 6 CTAs 80-92
+// (spills), 64, 96, 192 and 256 threads
 // 82-98, two lanes per node in the sums 89. FP32: 4, 5 and 6 CTAs 45.6, 40.1, 38.6 us.
 #include <algorithm>
 #include <atomic>
@@ -350,6 +351,11 @@ __global__ void k_pair_fixup(double* __restrict__ out, const double* __restrict_
 // ---- host: layout ------------------------------------------------------------------------------
 namespace {
 
+constexpr int kHalf = 16;       // lanes whose 64-bit reads go through together (bankplan.hpp)
+// Steps of the numbering's search: 4,000 leave 2.7 cycles per gather of a warp (ideal 2; 3.7 when whole
+// warps are planned), 16,000 leave 2.4: 43.3 and 42.3 us on 1,296,000 cells, first call 350 and 799 ms.
+constexpr int kPlanSteps = 4000;
+
 struct PairPlan {
     std::vector<int32_t> loc;       // global ids of the local nodes, by local index
     // {n0 | n1 << 16, n2 | n3 << 16, n4 | (B - A + kCellBias) << 16, A}: local node indices, cells A and
@@ -469,12 +475,12 @@ bool plan_pair_block(const int32_t* bc, int64_t c0, int ncell, PairPlan& P) {
     std::vector<int> deg(nloc, 0);
     for (int i = 0; i < ni; ++i)
         for (int k = 0; k < (items[i].b < 0 ? 4 : 5); ++k) {
-            const int l = items[i].n[k], g = i / kWarp * 5 + k;
+            const int l = items[i].n[k], g = i / kHalf * 5 + k;
             deg[l]++;
             if (groups[l].empty() || std::find(groups[l].begin(), groups[l].end(), g) == groups[l].end()) groups[l].push_back(g);
         }
     std::vector<int32_t> perm;
-    spread_nodes(groups, (ni + kWarp - 1) / kWarp * 5, deg, (uint64_t)c0, 8000, perm);
+    spread_nodes(groups, (ni + kHalf - 1) / kHalf * 5, deg, (uint64_t)c0, kPlanSteps, perm);
     P.loc.resize(nloc);
     for (int l = 0; l < nloc; ++l) P.loc[perm[l]] = sorted[l];
     std::vector<std::vector<int>> lists(nloc);
@@ -488,7 +494,7 @@ bool plan_pair_block(const int32_t* bc, int64_t c0, int ncell, PairPlan& P) {
         const uint32_t db = items[i].b < 0 ? 0u : (uint32_t)(items[i].b - items[i].a + kCellBias);
         for (uint32_t w : {n[0] | n[1] << 16, n[2] | n[3] << 16, n[4] | db << 16, (uint32_t)(c0 + items[i].a)}) P.items.push_back(w);
     }
-    const auto ordered = order_for_banks(lists, (nloc + kWarp - 1) / kWarp, [](int k) { return k / kWarp; }, 3);
+    const auto ordered = order_for_banks(lists, (nloc + kWarp - 1) / kWarp, [](int k) { return k / kWarp; }, 3, kHalf);
     P.off.assign(1, 0);
     P.inc.clear();
     for (int k = 0; k < nloc; ++k) {
