@@ -937,7 +937,9 @@ int pl_compute_lhs_residual(pl_integrator ig, double t, double dt, const double*
         return PL_OK;
     }
     if (rc) return rc;
-    if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(r, 0, pl_mesh_num_dof(m) * sizeof(double), s));
+    p.after_zeros = mode == PL_INSERT && rheo != RHEO_GENMAXWELL;  // see zero_output
+    if (p.after_zeros) zero_output(r, pl_mesh_num_dof(m), m->cell_type != PL_CELL_HEX8, s);
+    else if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(r, 0, pl_mesh_num_dof(m) * sizeof(double), s));
     if (ig->scatter == PL_SCATTER_ATOMIC ||
         !launch_domain_apply_hexgroup(p, m->cell_type, rheo, bf, OP_RESIDUAL, s))
         launch_domain_apply_atomic(p, m->cell_type, rheo, bf, OP_RESIDUAL, s);
@@ -984,7 +986,8 @@ int pl_compute_lhs_jacobian_action(pl_integrator ig, double t, double dt, double
         return PL_OK;
     }
     if (rc) return rc;
-    if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(jv, 0, pl_mesh_num_dof(m) * sizeof(double), s));
+    p.after_zeros = mode == PL_INSERT;
+    if (p.after_zeros) zero_output(jv, pl_mesh_num_dof(m), m->cell_type != PL_CELL_HEX8, s);
     if (ig->scatter == PL_SCATTER_ATOMIC ||
         !launch_domain_apply_hexgroup(p, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, s))
         launch_domain_apply_atomic(p, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, s);
@@ -997,7 +1000,7 @@ int pl_compute_lhs_jacobian_action_f32(pl_integrator ig, double t, double dt, co
     pl_mesh m = ig->mesh;
     cudaStream_t s = m->ctx->stream;
     PLB_CUDA(cudaSetDevice(m->ctx->device));
-    if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(jv, 0, pl_mesh_num_dof(m) * sizeof(float), s));
+    if (mode == PL_INSERT) zero_output(jv, pl_mesh_num_dof(m), m->cell_type != PL_CELL_HEX8, s);
     if (ig->is_interface) {
         CohesiveParams p;
         int rc = bind_cohesive(ig, &p);
@@ -1018,6 +1021,7 @@ int pl_compute_lhs_jacobian_action_f32(pl_integrator ig, double t, double dt, co
     p.out32 = jv;
     p.t = t;
     p.dt = dt;
+    p.after_zeros = mode == PL_INSERT;
     if ((m->cell_type == PL_CELL_HEX8 || m->cell_type == PL_CELL_TET4) && ig->lm32_valid && ig->lm32_t == t &&
         ig->lm32_dt == dt)
         p.lm32 = ig->d_lm32;

@@ -32,6 +32,10 @@ PL_D float safe_step_f32(double rz, double pq) {
     return isfinite(a) ? a : 0.0f;
 }
 
+// Waits for the kernel before this one where the launch let this one start early (launch_domain), and
+// for nothing otherwise.
+PL_D void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 PL_D void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr)); }
 
 PL_D void red_add(double* p, double v) { atomicAdd(p, v); }

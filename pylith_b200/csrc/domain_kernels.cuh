@@ -40,6 +40,7 @@ struct DomainParams {
     unsigned int* err;
     const float* lm32;  // FP32 Jacobian action (hexahedra, tetrahedra): per-cell (lambda, mu) of the
                         // isotropic tangent at (t, dt), or NULL to evaluate the tangent per point
+    int after_zeros;    // the launch before this one is zero_output's (launch_domain)
 };
 
 // ---- elements --------------------------------------------------------------------------

@@ -344,6 +344,7 @@ __global__ void __launch_bounds__(q2::WARPS * 32, RHEO == RHEO_ILE ? 5 : 4) k_he
             __syncwarp();
         }
     }
+    wait_for_previous();
 #pragma unroll 1
     for (int i0 = lane; i0 < ENTRIES; i0 += 32 * BATCH) {
         uint32_t e[BATCH];
@@ -367,8 +368,7 @@ static void launch_t(const DomainParams& p, cudaStream_t s) {
     auto kern = k_hex27_planes<RHEO, BF, OP>;
     ensure_kernel_smem((const void*)kern, q2::smem_bytes());
     const int64_t per = q2::WARPS * q2::CELLS;
-    kern<<<(unsigned)((p.ncells + per - 1) / per), q2::WARPS * 32, q2::smem_bytes(), s>>>(p);
-    count_launch();
+    launch_domain(kern, (p.ncells + per - 1) / per, q2::WARPS * 32, q2::smem_bytes(), s, p);
 }
 
 template <int RHEO>

@@ -72,8 +72,7 @@ static void launch_t(const DomainParams& p, cudaStream_t s) {
     auto kern = k_hex8<RHEO, BF, OP, T>;
     const size_t smem = RHEO == RHEO_GENMAXWELL && OP == OP_RESIDUAL ? hex8_state_bytes(th) : 0;
     if (smem) ensure_kernel_smem((const void*)kern, smem);
-    kern<<<(unsigned)((p.ncells + th - 1) / th), th, smem, s>>>(p);
-    count_launch();
+    launch_domain(kern, (p.ncells + th - 1) / th, th, smem, s, p);
 }
 
 void launch_hex8_update_state(const DomainParams& p, cudaStream_t s) {

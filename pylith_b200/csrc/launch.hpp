@@ -23,6 +23,28 @@ void count_launch(int n = 1);
 void ensure_kernel_smem(const void* kernel, size_t bytes);
 // Multiprocessor count of the current device (queried once per device).
 int sm_count();
+// An output's n zeros for an INSERT, by a kernel that lets the next one start at once (launch_domain).
+// shared: the next kernel works from shared memory (see zero_output in domain.cu).
+void zero_output(double* out, int64_t n, bool shared, cudaStream_t s);
+void zero_output(float* out, int64_t n, bool shared, cudaStream_t s);
+// Launches kern(p, rest...). After zero_output (after_zeros) its blocks start while the zeros are still
+// being written: kern must call wait_for_previous() before it writes or reads the output. Nothing else
+// it reads is in flight then, because zero_output's kernel itself waits for all earlier work.
+template <typename P, typename... R, typename... A>
+void launch_domain(void (*kern)(P, R...), int64_t grid, int threads, size_t smem, cudaStream_t s, const P& p, const A&... rest) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &early;
+    c.numAttrs = p.after_zeros ? 1 : 0;
+    cudaLaunchKernelEx(&c, kern, p, rest...);
+    count_launch();
+}
 bool launch_tangent_lm32(const DomainParams& p, int rheo, float* out, cudaStream_t s);
 
 void launch_domain_apply_atomic(const DomainParams& p, int cell, int rheo, bool bf, int op,

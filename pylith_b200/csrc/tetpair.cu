@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas) k_tet_pair(DomainPara
         pair_load_cells<L>(p, item, aA, aB);
         pair_prefetch_cells<BF>(p, item_next);
         __syncthreads();
+        wait_for_previous();
         const auto& M = S.meta[it & 1];
         for (int k = threadIdx.x; k < ns; k += kPairThreads) {
             const uint32_t id = M.ids[k];
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(kPairThreads, kPairCtas32) k_tet_pair_jv32(Dom
         pair_load_tangents<CACHED>(p, item, lm);
         if (CACHED && item_next.w != kNoItem) prefetch_l2(&p.lm32[2 * (int64_t)item_next.w]);
         __syncthreads();
+        wait_for_previous();
         const auto& M = S.meta[it & 1];
         for (int k = threadIdx.x; k < ns; k += kPairThreads) {
             const uint32_t id = M.ids[k];
@@ -622,8 +624,7 @@ template <typename T, int LD, typename Kernel>
 void launch_pairs(Kernel kern, const DomainParams& p, const PairArrays& A, cudaStream_t s) {
     constexpr size_t smem = sizeof(PairSmem<T, LD>);
     ensure_kernel_smem((const void*)kern, smem);
-    kern<<<(unsigned)std::min<int64_t>(A.nblocks, (int64_t)sm_count() * (sizeof(T) == 4 ? kPairCtas32 : kPairCtas)), kPairThreads, smem, s>>>(p, A);
-    count_launch();
+    launch_domain(kern, std::min<int64_t>(A.nblocks, (int64_t)sm_count() * (sizeof(T) == 4 ? kPairCtas32 : kPairCtas)), kPairThreads, smem, s, p, A);
 }
 
 template <bool BF, int OP, bool INSERT, bool DET>
@@ -727,11 +728,12 @@ bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rh
                               double* partial, cudaStream_t s, bool reduced) {
     if (rheo != RHEO_ILE || L.num_blocks == 0 || (reduced && (insert || partial || !L.d_ids_red))) return false;
     // INSERT without partial sums: shared nodes are reduced into zeros
-    if (insert && !partial && L.num_fix > 0)
-        if (cudaMemsetAsync(p.out, 0, 3 * nnodes * sizeof(double), s) != cudaSuccess) return false;
-    if (op != OP_RESIDUAL) launch_op<false, OP_JACOBIAN_ACTION>(p, L, insert, partial, reduced, s);
-    else if (bf) launch_op<true, OP_RESIDUAL>(p, L, insert, partial, reduced, s);
-    else launch_op<false, OP_RESIDUAL>(p, L, insert, partial, reduced, s);
+    DomainParams q = p;
+    q.after_zeros = insert && !partial && L.num_fix > 0;
+    if (q.after_zeros) zero_output(p.out, 3 * nnodes, true, s);
+    if (op != OP_RESIDUAL) launch_op<false, OP_JACOBIAN_ACTION>(q, L, insert, partial, reduced, s);
+    else if (bf) launch_op<true, OP_RESIDUAL>(q, L, insert, partial, reduced, s);
+    else launch_op<false, OP_RESIDUAL>(q, L, insert, partial, reduced, s);
     return true;
 }
 

@@ -802,3 +802,60 @@ def test_tet_pair_kernel_sizes(oracle_lib, torch_cuda, ctx, nc, window):
     ig.compute_lhs_residual(0.0, 0.0, du, dr, mode=FA.ADD)
     ctx.synchronize()
     assert rel_l2(dr.cpu().numpy(), 2 * r_ref) <= TOL64
+
+
+# the smallest output, one block of the zeroing kernel and several; small and large cell grids
+@pytest.mark.parametrize("kind,n", [("tet4", (1, 1, 1)), ("tet4", (9, 8, 7)), ("hex8", (1, 1, 1)), ("hex8", (13, 11, 9)),
+                                    ("hex27", (1, 1, 1)), ("hex27", (7, 5, 3))])
+def test_insert_zeroes_stale_output(oracle_lib, torch_cuda, kind, n):
+    """INSERT over stale outputs, issued back to back and replayed from a CUDA graph: the cell kernels
+    start while the zeros are being written and read the output only after them; each application
+    reads the one before it (v = J u, w = J v)."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh = {"tet4": M.box_tet_kuhn, "hex8": M.box_hex, "hex27": M.box_hex27}[kind](*n)
+    mat = elastic_setup(mesh, seed=31)
+    aux = oracle_aux(O, mat)
+    u = np.random.default_rng(32).standard_normal(mesh.num_nodes * 3)
+    v_ref = O.jacobian_action(mesh, u, aux, g3=JF3_ILE)
+    w_ref = O.jacobian_action(mesh, v_ref, aux, g3=JF3_ILE)
+    ctx = FA.Context(0)
+    ig = mat.create_integrator(FA.DeviceMesh(ctx, mesh))
+    du = dev(torch, u)
+    u32 = du.float()
+    v, w, r, v32 = (torch.empty_like(x) for x in (du, du, du, u32))
+
+    def spoil():
+        for x in (v, w, r, v32):
+            x.fill_(np.nan)
+
+    def apply():
+        ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, du, v)
+        ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, v, w)
+        ig.compute_lhs_residual(0.0, 0.0, v, r)
+        ig.compute_lhs_jacobian_action_f32(0.0, 0.0, u32, v32)
+
+    def check():
+        torch.cuda.synchronize()
+        assert rel_l2(v.cpu().numpy(), v_ref) <= TOL64
+        assert rel_l2(w.cpu().numpy(), w_ref) <= TOL64
+        assert rel_l2(r.cpu().numpy(), w_ref) <= TOL64  # linear elasticity: F(v) = J v
+        assert rel_l2(v32.double().cpu().numpy(), v_ref) <= 1e-5
+
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        spoil()
+        for _ in range(3):
+            apply()
+        check()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            apply()
+        for _ in range(2):
+            spoil()
+            graph.replay()
+            check()
+    del graph
