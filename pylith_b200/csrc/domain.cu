@@ -237,55 +237,96 @@ __global__ void __launch_bounds__(128) k_domain_update_state(DomainParams p) {
 // cauchy_strain, DerivedSubfieldsElasticity.py:42-44): each registered project kernel evaluated
 // at the cell centroid, out[c][6 * k + i] for kernel k. A generalized-Maxwell stress reads the
 // state of the cell's single quadrature point (P1 tetrahedra only).
+//
+// Bound: L2, at first by the stores: a thread's six values per kernel lie in a row of its own, so a
+// warp's store touched 32 sectors. Rows are staged in shared memory and a warp stores its cells' rows
+// with consecutive lanes on consecutive doubles; node ids, coordinates and field are read before
+// they are used: stress and strain of 100,345 Q1 hexahedra 12.9 -> 8.2 us.
+constexpr int kDerivedThreads = 128;
+constexpr int kDerivedRow = 6 * 4 + 1;  // values of a cell at most; odd, so a warp's accesses spread over the banks
 template <int CELL, int RHEO>
-__global__ void __launch_bounds__(128) k_domain_derived(DomainParams p, DerivedSpec spec) {
+__global__ void __launch_bounds__(kDerivedThreads) k_domain_derived(DomainParams p, DerivedSpec spec) {
     using E = Elem<CELL>;
     using L = AuxLayout<RHEO, false>;
+    constexpr int AHEAD = E::nen <= 8 ? E::nen : 1;  // nodes held in registers
+    __shared__ double rows[kDerivedThreads * kDerivedRow];
     const AuxOffsets<RHEO, false> aoff;
-    const int nout = 6 * spec.n;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < p.ncells;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t mc = p.cell_ids ? p.cell_ids[c] : c;
-        const int32_t* cn = p.cells + mc * E::nen;
-        double X[E::ngeom][3];
+    const int nout = 6 * spec.n, lane = threadIdx.x & 31;
+    double* const wrow = rows + (threadIdx.x - lane) * kDerivedRow;  // the warp's rows
+    for (int64_t c0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; c0 < p.ncells;
+         c0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t c = c0 + lane;
+        if (c < p.ncells) {
+            const int64_t mc = p.cell_ids ? p.cell_ids[c] : c;
+            const int32_t* cn = p.cells + mc * E::nen;
+            int nd[AHEAD];
+            double U[AHEAD][3];
+            if (E::nen <= 8) {
 #pragma unroll
-        for (int k = 0; k < E::ngeom; ++k)
+                for (int n = 0; n < AHEAD; ++n) nd[n] = cn[n];
 #pragma unroll
-            for (int i = 0; i < 3; ++i) X[k][i] = p.coords[3 * (int64_t)cn[E::corner(k)] + i];
-        Geom g;
-        E::centre_geom(X, &g);
-        if (!(g.detJ > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
-        double s_x[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        for (int n = 0; n < E::nen; ++n) {
-            double gr[3];
-            E::centre_grad(g, n, gr);
-            const double* un = p.u + 3 * (int64_t)cn[n];
+                for (int n = 0; n < AHEAD; ++n)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                s_x[0 + d] += un[0] * gr[d];
-                s_x[3 + d] += un[1] * gr[d];
-                s_x[6 + d] += un[2] * gr[d];
+                    for (int i = 0; i < 3; ++i) U[n][i] = p.u[3 * (int64_t)nd[n] + i];
+            }
+            double X[E::ngeom][3];
+#pragma unroll
+            for (int k = 0; k < E::ngeom; ++k) {
+                const int64_t node = E::nen <= 8 ? nd[k < AHEAD ? k : 0] : cn[E::corner(k)];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) X[k][i] = p.coords[3 * node + i];
+            }
+            double a[L::size] = {};
+            L::load_cell(p, c, a);
+            L::load_qp(p, c, 0, E::nq, a);
+            Geom g;
+            E::centre_geom(X, &g);
+            if (!(g.detJ > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
+            double s_x[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+            auto add = [&](int n, const double* un) {
+                double gr[3];
+                E::centre_grad(g, n, gr);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    s_x[0 + d] += un[0] * gr[d];
+                    s_x[3 + d] += un[1] * gr[d];
+                    s_x[6 + d] += un[2] * gr[d];
+                }
+            };
+            if (E::nen <= 8) {
+#pragma unroll
+                for (int n = 0; n < AHEAD; ++n) add(n, U[n]);
+            } else {
+                for (int n = 0; n < E::nen; ++n) add(n, p.u + 3 * (int64_t)cn[n]);
+            }
+            const int sOff[1] = {0}, sOff_x[1] = {0};
+            double x[3] = {0, 0, 0};
+            for (int k = 0; k < spec.n; ++k) {
+                double o[6] = {0, 0, 0, 0, 0, 0};
+                if (spec.kind[k] == K_EL_STRAIN_VECTOR)
+                    pw::el3d_strain_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
+                                                   nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
+                else if (RHEO == RHEO_ILE && spec.kind[k] == K_ILE_STRESS_VECTOR)
+                    pw::ile3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
+                                                    nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
+                else if (RHEO == RHEO_GENMAXWELL && spec.kind[k] == K_GM_STRESS_VECTOR)
+                    pw::gm3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
+                                                   nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
+#pragma unroll
+                for (int i = 0; i < 6; ++i) wrow[lane * kDerivedRow + 6 * k + i] = o[i];
             }
         }
-        double a[L::size] = {};
-        L::load_cell(p, c, a);
-        L::load_qp(p, c, 0, E::nq, a);
-        const int sOff[1] = {0}, sOff_x[1] = {0};
-        double x[3] = {0, 0, 0};
-        for (int k = 0; k < spec.n; ++k) {
-            double o[6] = {0, 0, 0, 0, 0, 0};
-            if (spec.kind[k] == K_EL_STRAIN_VECTOR)
-                pw::el3d_strain_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
-                                               nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
-            else if (RHEO == RHEO_ILE && spec.kind[k] == K_ILE_STRESS_VECTOR)
-                pw::ile3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
-                                                nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
-            else if (RHEO == RHEO_GENMAXWELL && spec.kind[k] == K_GM_STRESS_VECTOR)
-                pw::gm3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
-                                               nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
-#pragma unroll
-            for (int i = 0; i < 6; ++i) p.out[c * nout + 6 * k + i] = o[i];
+        __syncwarp();
+        const int count = (int)min((int64_t)32, p.ncells - c0) * nout;
+        double* out = p.out + c0 * nout;
+        int row = lane / nout, col = lane - row * nout;  // of entry e
+        const int drow = 32 / nout, dcol = 32 - drow * nout;
+        for (int e = lane; e < count; e += 32) {
+            out[e] = wrow[row * kDerivedRow + col];
+            row += drow, col += dcol;
+            if (col >= nout) ++row, col -= nout;
         }
+        __syncwarp();
     }
 }
 
@@ -386,7 +427,7 @@ void launch_domain_update_state(const DomainParams& p, int cell, cudaStream_t s)
 
 void launch_domain_derived(const DomainParams& p, int cell, int rheo, const DerivedSpec& spec, cudaStream_t s) {
     if (p.ncells == 0) return;
-    const int th = 128;
+    const int th = kDerivedThreads;
     const int gr = grid_for(p.ncells, th);
     if (rheo == RHEO_GENMAXWELL) {
         if (cell == TET4) k_domain_derived<TET4, RHEO_GENMAXWELL><<<gr, th, 0, s>>>(p, spec);
