@@ -859,3 +859,36 @@ def test_insert_zeroes_stale_output(oracle_lib, torch_cuda, kind, n):
             graph.replay()
             check()
     del graph
+
+
+# one to four kernels (6 to 24 values per cell) on one cell, one less than, exactly and one more than a
+# warp's and a block's cells, and several blocks
+@pytest.mark.parametrize("num", [1, 2, 3, 4])
+@pytest.mark.parametrize("nc", [1, 31, 32, 33, 127, 128, 129, 1000])
+def test_derived_rows(oracle_lib, torch_cuda, ctx, nc, num):
+    """The rows of pl_compute_derived_field for every number of kernels and at warp and block edges;
+    nothing is written past the last row."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh = M.box_hex(10, 10, 10)
+    mesh.cells = mesh.cells[:nc].copy()
+    mat = elastic_setup(mesh, seed=41)
+    stress = "IsotropicLinearElasticity3D::cauchyStress_infinitesimalStrain_asVector"
+    strain = "Elasticity3D::infinitesimalStrain_asVector"
+    names = [stress, strain, strain, stress][:num]
+    k = FA.fekernels
+    fn = {stress: k.IsotropicLinearElasticity3D.cauchyStress_infinitesimalStrain_asVector,
+          strain: k.Elasticity3D.infinitesimalStrain_asVector}
+    u = np.random.default_rng(42).standard_normal(mesh.num_dof)
+    ref = np.concatenate(O.project_centroid(mesh, u, oracle_aux(O, mat), names, [6] * num), axis=1)
+    ig = mat.create_integrator(FA.DeviceMesh(ctx, mesh))
+    ig.set_kernels_derived_field([FA.ProjectKernels(f"field_{i}", fn[n]) for i, n in enumerate(names)])
+    out = torch.full((nc + 1, 6 * num), np.nan, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ig.compute_derived_field(0.0, 0.0, dev(torch, u), out)
+    ctx.synchronize()
+    got = out.cpu().numpy()
+    assert np.isnan(got[nc]).all()
+    for i in range(num):
+        assert rel_l2(got[:nc, 6 * i:6 * i + 6], ref[:, 6 * i:6 * i + 6]) <= TOL64
