@@ -13,7 +13,7 @@
 // planned for the banks, kPlanSteps); 54,737 Delaunay cells FP64 9.5 -> 8.9, FP32 9.9 -> 8.7; 3,072 cells
 // FP64 8.5 -> 6.8. What bounds it now: shared memory still, then HBM.
 // Block size: 240 cells in 128 items with 4 CTAs per SM (FP64, at most 128 registers) measured best
-// (two launches on 1,179,648 cells 80 us, 75 with the banks planned by halves); 5 and 6 CTAs 80-92
+// (two launches on 1,179,648 cells 80 us, 75 with the banks planned by halves, 70.5 with zero_output); 5 and 6 CTAs 80-92
 // (spills), 64, 96, 192 and 256 threads
 // 82-98, two lanes per node in the sums 89. FP32: 4, 5 and 6 CTAs 45.6, 40.1, 38.6 us.
 #include <algorithm>
