@@ -790,6 +790,9 @@ static bool apply_cells_f32(pl_integrator ig, const DomainParams& p, int rheo, b
     return launch_domain_jv32_blocked(p, *m->blocked, m->cell_type, rheo, m->nnodes, s, reduced);
 }
 
+// The mesh's layout for the cell-block kernels.
+static int prepare_layout(pl_mesh m) { return m->cell_type == PL_CELL_TET4 ? prepare_tet_layout(m) : ensure_blocked_layout(m); }
+
 // The reduced fault space's connectivity (each positive-side node replaced by its negative-side
 // partner) and node map. Refused (PL_ERR_UNSUPPORTED) when a pair's two nodes do not coincide:
 // the kernels then read the partner's coordinates in place of the node's own.
@@ -878,7 +881,7 @@ int jacobian_action_reduced_f32(pl_integrator_s* ig, double t, double dt, const 
         p.lm32 = ig->d_lm32;
     if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(jv, 0, pl_mesh_num_dof(m) * sizeof(float), s));
     if (use_blocked(ig) && m->cell_type == PL_CELL_TET4) {
-        if ((rc = prepare_blocked(ig)) != PL_OK || (rc = ensure_cell_ids_reduced(m)) != PL_OK) return rc;
+        if ((rc = prepare_layout(m)) != PL_OK || (rc = ensure_cell_ids_reduced(m)) != PL_OK) return rc;
         if (!apply_cells_f32(ig, p, rheo, true)) return PL_ERR_UNSUPPORTED;
     } else if (ig->scatter == PL_SCATTER_ATOMIC || !launch_domain_jv32_hexgroup(p, m->cell_type, rheo, s)) {
         launch_domain_jv_f32_atomic(p, m->cell_type, rheo, s);
@@ -887,9 +890,11 @@ int jacobian_action_reduced_f32(pl_integrator_s* ig, double t, double dt, const 
     return PL_OK;
 }
 
+// The layout, and the FP64 partial sums of the deterministic mode (the FP32 action has none: it
+// prepares the layout alone, so that it never allocates once the layout is there).
 int prepare_blocked(pl_integrator_s* ig) {
     pl_mesh m = ig->mesh;
-    const int rc = m->cell_type == PL_CELL_TET4 ? prepare_tet_layout(m) : ensure_blocked_layout(m);
+    const int rc = prepare_layout(m);
     if (rc) return rc;
     const int64_t slots = uses_pairs(m) ? m->pair->num_slots : m->blocked->num_slots;
     if (ig->scatter == PL_SCATTER_DETERMINISTIC && !ig->d_block_partial && slots > 0)
@@ -1025,7 +1030,7 @@ int pl_compute_lhs_jacobian_action_f32(pl_integrator ig, double t, double dt, co
     if ((m->cell_type == PL_CELL_HEX8 || m->cell_type == PL_CELL_TET4) && ig->lm32_valid && ig->lm32_t == t &&
         ig->lm32_dt == dt)
         p.lm32 = ig->d_lm32;
-    if (use_blocked(ig) && (rc = prepare_blocked(ig)) == PL_OK && apply_cells_f32(ig, p, rheo)) {
+    if (use_blocked(ig) && (rc = prepare_layout(m)) == PL_OK && apply_cells_f32(ig, p, rheo)) {
         PLB_CUDA(cudaGetLastError());
         return PL_OK;
     }

@@ -892,3 +892,37 @@ def test_derived_rows(oracle_lib, torch_cuda, ctx, nc, num):
     assert np.isnan(got[nc]).all()
     for i in range(num):
         assert rel_l2(got[:nc, 6 * i:6 * i + 6], ref[:, 6 * i:6 * i + 6]) <= TOL64
+
+
+def test_fp32_action_allocates_nothing_once_the_layout_is_there():
+    """The FP32 action of integrators in the deterministic mode, whose FP64 partial sums it does not
+    use: after the first call has built the mesh's layout, free device memory stays as it is. (A
+    process of its own, whose memory pool holds nothing to hand out again; 6 integrators would take
+    17 MB each.)"""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from pylith_b200 import feassemble as FA, materials as MAT, meshing as M
+mesh = M.box_tet_kuhn(64, 64, 48)
+ctx = FA.Context(0)
+dm = FA.DeviceMesh(ctx, mesh)
+mat = MAT.IsotropicLinearElasticity(*MAT.lognormal_elastic(mesh.num_cells, seed=1))
+igs = [mat.create_integrator(dm) for _ in range(6)]
+v = torch.ones(mesh.num_dof, dtype=torch.float32, device="cuda")
+out = torch.empty_like(v)
+igs[0].compute_lhs_jacobian_action_f32(0.0, 0.0, v, out)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+for ig in igs:
+    ig.set_scatter(FA.SCATTER_DETERMINISTIC)
+    ig.compute_lhs_jacobian_action_f32(0.0, 0.0, v, out)
+torch.cuda.synchronize()
+print("taken", free - torch.cuda.mem_get_info()[0])
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert int(r.stdout.split()[-1]) == 0, r.stdout
