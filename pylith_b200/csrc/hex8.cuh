@@ -332,7 +332,7 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
             for (int d = 0; d < 3; ++d) g[n][d] *= T(0.125);
     }
     __syncwarp();
-    if constexpr (!(RHEO == RHEO_GENMAXWELL && OP == OP_RESIDUAL)) wait_for_previous();  // see zero_output
+    wait_for_previous();  // see zero_output
     if constexpr (F32) hex8_scatter<T>(nodes, g, p.out32);
     else hex8_scatter<T>(nodes, g, p.out);
 }

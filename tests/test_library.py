@@ -177,3 +177,16 @@ def test_registration_accepts_the_reference_build_and_refuses_other_functions():
     with pytest.raises(_lib.PylithB200Error) as e:
         FA.register_fekernel("IsotropicLinearElasticity3D::f1v_infinitesimalStrain_refState", addr)
     assert e.value.code == -2
+
+
+def test_kernels_that_may_start_early_always_wait():
+    """Kernels launched by launch_domain may start while their output is being zeroed: each waits before
+    it touches the output, in every instantiation (the wait stands by itself, under no condition)."""
+    import glob
+
+    text = {os.path.basename(f): open(f).read() for f in glob.glob(os.path.join(ROOT, "pylith_b200", "csrc", "*.cu*"))}
+    calls = [f for f in text if "launch_domain(" in text[f]]
+    waits = {f: re.findall(r"^(.*)wait_for_previous\(\);", text[f], re.M) for f in text if f != "common.cuh"}
+    assert calls and all(not before.strip() for lines in waits.values() for before in lines), waits
+    for f in calls:
+        assert waits[f] or any(waits.get(h) for h in re.findall(r'#include "(\w+\.cuh)"', text[f])), f
