@@ -332,6 +332,7 @@ __global__ void __launch_bounds__(q2::WARPS * 32, RHEO == RHEO_ILE ? 5 : 4) k_he
                 rev_d_add(R[9 + i], R[12 + i], R[15 + i], nb[i]);
                 rev_b(R[18 + i], R[21 + i], R[24 + i], nd[i]);
             }
+            __syncwarp();  // lanes without a plane have read lane 0's: it is overwritten only now
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
                 double n[3];
@@ -341,8 +342,8 @@ __global__ void __launch_bounds__(q2::WARPS * 32, RHEO == RHEO_ILE ? 5 : 4) k_he
                 if (take[b]) n[0] += prev;
                 if (live) R[3 * b] = n[0], R[3 * b + 1] = n[1], R[3 * b + 2] = n[2];
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
     wait_for_previous();
 #pragma unroll 1
