@@ -299,7 +299,13 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
                     for (int e = 0; e < 3; ++e)
                         s_x[f * 3 + e] = G[f][0] * C[0][e] + G[f][1] * C[1][e] + G[f][2] * C[2][e];
                 if constexpr (OP == OP_JACOBIAN_ACTION) {
-                    isotropic_contract<T>(lam * rdet, mu * rdet, s_x, f1);  // linear in the gradient
+                    // The flux is linear in the gradient: the division by det is applied to the moduli, in
+                    // FP32 to the six fluxes (modulus / det leaves its range where a cell is smaller than
+                    // about 1e-9 m with moduli in Pa; a static solve takes 1 % longer with it).
+                    isotropic_contract<T>(F32 ? lam : lam * rdet, F32 ? mu : mu * rdet, s_x, f1);
+                    if constexpr (F32)
+#pragma unroll
+                        for (int f = 0; f < 9; ++f) f1[f] *= rdet;
                 } else {
 #pragma unroll
                     for (int f = 0; f < 9; ++f) s_x[f] *= rdet;

@@ -926,3 +926,22 @@ print("taken", free - torch.cuda.mem_get_info()[0])
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root)
     assert r.returncode == 0, r.stderr[-2000:]
     assert int(r.stdout.split()[-1]) == 0, r.stdout
+
+
+@pytest.mark.parametrize("kind", ["tet4", "hex8", "hex27"])
+@pytest.mark.parametrize("scale", [1e-13, 1e-7, 1.0, 1e7])
+def test_fp32_action_over_length_scales(torch_cuda, ctx, kind, scale):
+    """The FP32 action on boxes from nanometres to astronomic sizes with moduli in Pa: it agrees with the
+    FP64 action to 1e-5 as at the usual size (no factor of a cell leaves FP32's range)."""
+    from pylith_b200 import feassemble as FA
+
+    torch = torch_cuda
+    mesh = {"tet4": M.box_tet_kuhn, "hex8": M.box_hex, "hex27": M.box_hex27}[kind](4, 4, 3)
+    mesh.coords *= scale
+    ig = elastic_setup(mesh, seed=51).create_integrator(FA.DeviceMesh(ctx, mesh))
+    v = torch.from_numpy(np.random.default_rng(52).standard_normal(mesh.num_dof)).cuda().float()
+    d64, d32 = torch.empty_like(v.double()), torch.empty_like(v)
+    ig.compute_lhs_jacobian_action(0.0, 0.0, 0.0, None, v.double(), d64)
+    ig.compute_lhs_jacobian_action_f32(0.0, 0.0, v, d32)
+    ctx.synchronize()
+    assert rel_l2(d32.double().cpu().numpy(), d64.cpu().numpy()) <= 1e-5
