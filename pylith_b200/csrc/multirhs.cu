@@ -531,8 +531,9 @@ __global__ void __launch_bounds__(kMultiBlockCells, 3) k_tet_blocked_jv32_multi(
 
 // The same on the pairs of tetpair.cu, one CTA per (block, KC right-hand sides): blockIdx.y is the
 // chunk. A thread forms the element vectors of two tetrahedra that share a face (15 entries for the
-// pair instead of 24); with cf = cofactors / 6 and lambda, mu times 6 / det one set of factors serves
-// both the gradient and the test functions. In the sums a thread takes a node's three components (one
+// pair instead of 24); with cf = cofactors / sqrt(6 det) one set of factors serves both the gradient and
+// the test functions, and no factor leaves FP32's range at any cell size (cofactors / 6 with the moduli
+// times 6 / det did below about 1e-9 m with moduli in Pa). In the sums a thread takes a node's three components (one
 // component per thread: 16.3 us for 15.5). Measured with 94,080 cells and K = 8, in the PCG on B200:
 // 18.1 -> 15.5 us against k_tet_blocked_jv32_multi, 13.6 with the energies' partials summed by the kernel
 // that uses them; bound by issue and shared memory in about equal parts. 3 CTAs per SM are as fast, 5
@@ -606,18 +607,18 @@ __global__ void __launch_bounds__(kPairThreads, kPairMultiCtas<LD>)
                     const double det = e0[0] * c0[0] + e0[1] * c0[1] + e0[2] * c0[2];
                     const bool on = t == 0 || !pair_single(item);
                     if (on && !(det > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
-                    const double r6 = on ? 6.0 / det : 0.0, sg = t ? -1.0 / 6.0 : 1.0 / 6.0;
-                    lam[t] = (float)(lm[t].x * r6);
-                    mu[t] = (float)(lm[t].y * r6);
+                    const double sc = rsqrt(6.0 * fabs(det));
+                    lam[t] = on ? (det < 0.0 ? -lm[t].x : lm[t].x) : 0.f;
+                    mu[t] = on ? (det < 0.0 ? -lm[t].y : lm[t].y) : 0.f;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
-                        cf[t][0][d] = on ? (float)(c0[d] * (1.0 / 6.0)) : 0.f;
-                        cf[t][1][d] = on ? (float)(c1[d] * (1.0 / 6.0)) : 0.f;
-                        cf[t][2][d] = on ? (float)(n12[d] * sg) : 0.f;
+                        cf[t][0][d] = on ? (float)(c0[d] * sc) : 0.f;
+                        cf[t][1][d] = on ? (float)(c1[d] * sc) : 0.f;
+                        cf[t][2][d] = on ? (float)(n12[d] * (t ? -sc : sc)) : 0.f;
                     }
                 }
             }
-            // gradients of the two cells times their volumes
+            // gradients of the two cells times the square roots of their volumes
             float s[2][KC][3][3];
 #pragma unroll
             for (int cc = 0; cc < 3; ++cc) {

@@ -341,6 +341,35 @@ def test_batched_operator_cell_orders(ctx, window, tile, integrators):
         assert torch.linalg.norm(x - ref) <= 1e-8 * torch.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("scale", [1e-13, 1.0, 1e5])
+@pytest.mark.parametrize("tile", [1, 2, 8])
+def test_batched_operator_over_length_scales(ctx, scale, tile):
+    """Batched solves on boxes from nanometres up with moduli in Pa match FP64 solves of one right-hand
+    side at a time to <= 1e-8 (no factor of a cell leaves FP32's range)."""
+    import torch
+    from pylith_b200 import feassemble as FA
+
+    mesh = M.box_tet_kuhn(5, 4, 4)
+    cons = np.zeros((mesh.num_nodes, 3), dtype=bool)
+    cons[M.boundary_mask(mesh, 0, "neg")] = True
+    mesh.coords *= scale
+    dm = FA.DeviceMesh(ctx, mesh)
+    ig = MAT.IsotropicLinearElasticity(*MAT.lognormal_elastic(mesh.num_cells, seed=52)).create_integrator(dm)
+    rng = np.random.default_rng(53)
+    bs = [torch.from_numpy(rng.standard_normal(mesh.num_dof)).cuda() for _ in range(tile)]
+    refined = FA.Solver(dm, cons.ravel(), [ig], rtol=1e-11, precision=FA.Solver.FP32_REFINED, inner_rtol=1e-4)
+    refined.setup()
+    xs = [torch.zeros_like(b) for b in bs]
+    FA.BatchSolver(refined, tile).solve(bs, xs)
+    S = FA.Solver(dm, cons.ravel(), [ig], rtol=1e-11)
+    S.setup()
+    for b, x in zip(bs, xs):
+        ref = torch.zeros_like(b)
+        S.solve(b, ref)
+        ctx.synchronize()
+        assert torch.linalg.norm(x - ref) <= 1e-8 * torch.linalg.norm(ref)
+
+
 # fewer right-hand sides than columns; more, with zero ones in the first tile, in a refill and last; all zero
 @pytest.mark.parametrize("zero", [(0, 1, 0), (1, 0, 1, 1, 0, 0, 1, 0, 1, 0, 1), (1,) * 6])
 @pytest.mark.parametrize("reliable", [True, False])
