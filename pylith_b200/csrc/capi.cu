@@ -773,6 +773,9 @@ static bool use_blocked(pl_integrator ig) {
     return m->cell_type == PL_CELL_TET4 || ig->scatter == PL_SCATTER_BLOCKED || ig->scatter == PL_SCATTER_DETERMINISTIC;
 }
 
+// Whether the kernel outside the cell-block ones starts under its output's zeroing (launch_domain).
+static bool starts_early(pl_integrator ig) { return ig->mesh->cell_type != PL_CELL_TET4 && ig->scatter != PL_SCATTER_ATOMIC; }
+
 // The FP64 cell-block kernels (after prepare_blocked); false when they do not support the configuration.
 static bool apply_cells(pl_integrator ig, const DomainParams& p, int rheo, bool bf, int op, bool insert, bool reduced = false) {
     pl_mesh m = ig->mesh;
@@ -942,9 +945,8 @@ int pl_compute_lhs_residual(pl_integrator ig, double t, double dt, const double*
         return PL_OK;
     }
     if (rc) return rc;
-    p.after_zeros = mode == PL_INSERT && rheo != RHEO_GENMAXWELL;  // see zero_output
-    if (p.after_zeros) zero_output(r, pl_mesh_num_dof(m), m->cell_type != PL_CELL_HEX8, s);
-    else if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(r, 0, pl_mesh_num_dof(m) * sizeof(double), s));
+    if (mode == PL_INSERT)  // (generalized Maxwell: see zero_output)
+        p.after_zeros = zero_output(r, pl_mesh_num_dof(m), starts_early(ig) && rheo != RHEO_GENMAXWELL, m->cell_type != PL_CELL_HEX8, s);
     if (ig->scatter == PL_SCATTER_ATOMIC ||
         !launch_domain_apply_hexgroup(p, m->cell_type, rheo, bf, OP_RESIDUAL, s))
         launch_domain_apply_atomic(p, m->cell_type, rheo, bf, OP_RESIDUAL, s);
@@ -991,8 +993,8 @@ int pl_compute_lhs_jacobian_action(pl_integrator ig, double t, double dt, double
         return PL_OK;
     }
     if (rc) return rc;
-    p.after_zeros = mode == PL_INSERT;
-    if (p.after_zeros) zero_output(jv, pl_mesh_num_dof(m), m->cell_type != PL_CELL_HEX8, s);
+    if (mode == PL_INSERT)
+        p.after_zeros = zero_output(jv, pl_mesh_num_dof(m), starts_early(ig), m->cell_type != PL_CELL_HEX8, s);
     if (ig->scatter == PL_SCATTER_ATOMIC ||
         !launch_domain_apply_hexgroup(p, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, s))
         launch_domain_apply_atomic(p, m->cell_type, rheo, false, OP_JACOBIAN_ACTION, s);
@@ -1005,8 +1007,9 @@ int pl_compute_lhs_jacobian_action_f32(pl_integrator ig, double t, double dt, co
     pl_mesh m = ig->mesh;
     cudaStream_t s = m->ctx->stream;
     PLB_CUDA(cudaSetDevice(m->ctx->device));
-    if (mode == PL_INSERT) zero_output(jv, pl_mesh_num_dof(m), m->cell_type != PL_CELL_HEX8, s);
+    const int64_t n = pl_mesh_num_dof(m);
     if (ig->is_interface) {
+        if (mode == PL_INSERT) PLB_CUDA(cudaMemsetAsync(jv, 0, n * sizeof(float), s));
         CohesiveParams p;
         int rc = bind_cohesive(ig, &p);
         if (rc) return rc;
@@ -1026,15 +1029,18 @@ int pl_compute_lhs_jacobian_action_f32(pl_integrator ig, double t, double dt, co
     p.out32 = jv;
     p.t = t;
     p.dt = dt;
-    p.after_zeros = mode == PL_INSERT;
     if ((m->cell_type == PL_CELL_HEX8 || m->cell_type == PL_CELL_TET4) && ig->lm32_valid && ig->lm32_t == t &&
         ig->lm32_dt == dt)
         p.lm32 = ig->d_lm32;
-    if (use_blocked(ig) && (rc = prepare_layout(m)) == PL_OK && apply_cells_f32(ig, p, rheo)) {
+    const bool cells = use_blocked(ig);
+    if (cells && (rc = prepare_layout(m)) != PL_OK) return rc;
+    const bool early = m->cell_type == PL_CELL_TET4 ? cells && uses_pairs(m) && (p.lm32 || rheo == RHEO_ILE)
+                                                     : m->cell_type == PL_CELL_HEX8 && starts_early(ig);
+    if (mode == PL_INSERT) p.after_zeros = zero_output(jv, n, early, m->cell_type != PL_CELL_HEX8, s);
+    if (cells && apply_cells_f32(ig, p, rheo)) {
         PLB_CUDA(cudaGetLastError());
         return PL_OK;
     }
-    if (rc) return rc;
     if (ig->scatter == PL_SCATTER_ATOMIC || !launch_domain_jv32_hexgroup(p, m->cell_type, rheo, s))
         launch_domain_jv_f32_atomic(p, m->cell_type, rheo, s);
     PLB_CUDA(cudaGetLastError());

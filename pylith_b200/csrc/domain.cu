@@ -371,7 +371,6 @@ static __global__ void k_zero_output(T* __restrict__ out, int64_t n) {
 }
 template <typename T, bool SHARED>
 static void zero_output_t(T* out, int64_t n, cudaStream_t s) {
-    if (n == 0) return;
     if (SHARED) {  // once per device (a 64-bit word holds them all)
         static std::atomic<uint64_t> done{0};
         int dev = 0;
@@ -385,12 +384,20 @@ static void zero_output_t(T* out, int64_t n, cudaStream_t s) {
     k_zero_output<T, SHARED><<<(unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count() * 8), 256, 0, s>>>(out, n);
     count_launch();
 }
-void zero_output(double* out, int64_t n, bool shared, cudaStream_t s) {
-    shared ? zero_output_t<double, true>(out, n, s) : zero_output_t<double, false>(out, n, s);
+template <typename T>
+static bool zero_any(T* out, int64_t n, bool early, bool shared, cudaStream_t s) {
+    // A memset where nothing starts under it (a launch of its own then costs 0.5 to 1 us more: atomic
+    // scatter on 2,652 tetrahedra 6.6 and 7.2 us, FP32 action of 1,188 Q2 hexahedra 12.4 and 13.4) and
+    // for outputs of one block, ready before the next launch either way (FP32 action of 6 tetrahedra 6.3
+    // and 6.8 us; of 750, 648 values, 8.2 and 6.6).
+    early = early && n > 256;
+    if (!early) cudaMemsetAsync(out, 0, n * sizeof(T), s);
+    else if (shared) zero_output_t<T, true>(out, n, s);
+    else zero_output_t<T, false>(out, n, s);
+    return early;
 }
-void zero_output(float* out, int64_t n, bool shared, cudaStream_t s) {
-    shared ? zero_output_t<float, true>(out, n, s) : zero_output_t<float, false>(out, n, s);
-}
+bool zero_output(double* out, int64_t n, bool early, bool shared, cudaStream_t s) { return zero_any(out, n, early, shared, s); }
+bool zero_output(float* out, int64_t n, bool early, bool shared, cudaStream_t s) { return zero_any(out, n, early, shared, s); }
 
 void launch_domain_apply_atomic(const DomainParams& p, int cell, int rheo, bool bf, int op,
                                 cudaStream_t s) {

@@ -23,10 +23,11 @@ void count_launch(int n = 1);
 void ensure_kernel_smem(const void* kernel, size_t bytes);
 // Multiprocessor count of the current device (queried once per device).
 int sm_count();
-// An output's n zeros for an INSERT, by a kernel that lets the next one start at once (launch_domain).
-// shared: the next kernel works from shared memory (see zero_output in domain.cu).
-void zero_output(double* out, int64_t n, bool shared, cudaStream_t s);
-void zero_output(float* out, int64_t n, bool shared, cudaStream_t s);
+// An output's n zeros for an INSERT. early: the next kernel is one of launch_domain's; the zeros are then
+// written by a kernel that lets it start at once, and true is returned (its after_zeros), unless the
+// output is tiny. shared: the next kernel works from shared memory (see zero_output in domain.cu).
+bool zero_output(double* out, int64_t n, bool early, bool shared, cudaStream_t s);
+bool zero_output(float* out, int64_t n, bool early, bool shared, cudaStream_t s);
 // Launches kern(p, rest...). After zero_output (after_zeros) its blocks start while the zeros are still
 // being written: kern must call wait_for_previous() before it writes or reads the output. Nothing else
 // it reads is in flight then, because zero_output's kernel itself waits for all earlier work.

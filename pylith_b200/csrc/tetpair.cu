@@ -729,8 +729,7 @@ bool launch_domain_apply_pair(const DomainParams& p, const PairLayout& L, int rh
     if (rheo != RHEO_ILE || L.num_blocks == 0 || (reduced && (insert || partial || !L.d_ids_red))) return false;
     // INSERT without partial sums: shared nodes are reduced into zeros
     DomainParams q = p;
-    q.after_zeros = insert && !partial && L.num_fix > 0;
-    if (q.after_zeros) zero_output(p.out, 3 * nnodes, true, s);
+    q.after_zeros = insert && !partial && L.num_fix > 0 && zero_output(p.out, 3 * nnodes, true, true, s);
     if (op != OP_RESIDUAL) launch_op<false, OP_JACOBIAN_ACTION>(q, L, insert, partial, reduced, s);
     else if (bf) launch_op<true, OP_RESIDUAL>(q, L, insert, partial, reduced, s);
     else launch_op<false, OP_RESIDUAL>(q, L, insert, partial, reduced, s);

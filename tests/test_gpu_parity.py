@@ -945,3 +945,56 @@ def test_fp32_action_over_length_scales(torch_cuda, ctx, kind, scale):
     ig.compute_lhs_jacobian_action_f32(0.0, 0.0, v, d32)
     ctx.synchronize()
     assert rel_l2(d32.double().cpu().numpy(), d64.cpu().numpy()) <= 1e-5
+
+
+# calls whose kernel is launched behind the zeroing, not under it, and outputs of a few values
+ONE_LAUNCH = {
+    "tet4_atomic": (lambda: M.box_tet_kuhn(6, 5, 4), "atomic", "rjf"),
+    "tet4_subset": (lambda: M.box_tet_kuhn(6, 5, 4), "subset", "rjf"),
+    "tet4_genmaxwell": (lambda: M.box_tet_kuhn(6, 5, 4), "genmaxwell", "rjf"),
+    "tet4_scattered": (lambda: M.box_tet_kuhn(9, 9, 9, reorder=False), "scattered", "f"),
+    "hex8_atomic": (lambda: M.box_hex(6, 5, 4), "atomic", "rjf"),
+    "hex8_genmaxwell": (lambda: M.box_hex(6, 5, 4), "genmaxwell", "r"),
+    "hex8_few": (lambda: M.box_hex(2, 2, 2), "", "rjf"),
+    "hex27": (lambda: M.box_hex27(3, 3, 3), "", "f"),
+    "tet4_few": (lambda: M.box_tet_kuhn(1, 1, 1), "", "rjf"),
+}
+
+
+@pytest.mark.parametrize("case", list(ONE_LAUNCH))
+def test_insert_takes_one_launch_where_nothing_starts_early(torch_cuda, ctx, case):
+    """INSERT zeroes by a memset wherever no kernel starts under the zeroing (one launch per call), and
+    gives what ADD into zeros gives."""
+    from pylith_b200 import _lib
+    from pylith_b200 import feassemble as FA
+
+    torch = torch_cuda
+    make, form, calls = ONE_LAUNCH[case]
+    mesh = make()
+    if form == "scattered":
+        np.random.default_rng(60).shuffle(mesh.cells)
+    dm = FA.DeviceMesh(ctx, mesh)
+    if form == "genmaxwell":
+        ig = genmaxwell_setup(mesh, seed=61).create_integrator(dm, MAT.YEAR)
+    elif form == "subset":
+        ids = np.arange(0, mesh.num_cells, 2, dtype=np.int32)
+        mat = elastic_setup(mesh, seed=61)
+        ig = MAT.IsotropicLinearElasticity(mat.density[ids], mat.shear_modulus[ids], mat.bulk_modulus[ids]).create_integrator(dm, ids)
+    else:
+        ig = elastic_setup(mesh, seed=61).create_integrator(dm)
+    if form == "atomic":
+        ig.set_scatter(FA.SCATTER_ATOMIC)
+    u = torch.from_numpy(np.random.default_rng(62).standard_normal(mesh.num_dof)).cuda()
+    run = {"r": lambda o, m: ig.compute_lhs_residual(0.0, MAT.YEAR, u, o, mode=m),
+           "j": lambda o, m: ig.compute_lhs_jacobian_action(0.0, MAT.YEAR, 0.0, None, u, o, mode=m),
+           "f": lambda o, m: ig.compute_lhs_jacobian_action_f32(0.0, MAT.YEAR, u.float(), o, mode=m)}
+    for c in calls:
+        ref = torch.zeros_like(u.float() if c == "f" else u)
+        out = torch.full_like(ref, np.nan)
+        run[c](ref, FA.ADD)  # (builds the layout)
+        ctx.synchronize()
+        n0 = _lib.lib().pl_kernel_launches()
+        run[c](out, FA.INSERT)
+        ctx.synchronize()
+        assert _lib.lib().pl_kernel_launches() - n0 == 1, c
+        assert rel_l2(out.double().cpu().numpy(), ref.double().cpu().numpy()) <= (1e-6 if c == "f" else TOL64)
