@@ -1,5 +1,5 @@
 // Q2 hexahedra (27 nodes, 3x3x3 Gauss points) by sum factorisation with a plane of nodes per lane:
-// FP64 residual and Jacobian action.
+// FP64 residual and Jacobian action (small meshes: hex27lines.cu).
 //
 // Three lanes share a cell, ten cells a warp. The Q2 basis is a tensor product of the 1-D quadratic
 // basis, so the reference gradient at the points is three 1-D contractions. Lane m takes the nodes

@@ -292,9 +292,20 @@ static void launch_group_t(const DomainParams& p, cudaStream_t s) {
     count_launch();
 }
 
+// Q2 hexahedra: a line of points per lane (hex27lines.cu) while the mesh is a wave or so of its blocks,
+// a plane of nodes per lane (hex27.cu) beyond. Cells per multiprocessor at which they cross, with the
+// two measured below and above (us, ADD): isotropic 10.4 and 12.4 at 2,912 cells, 14.5 and 12.5 at 5,508;
+// generalized-Maxwell residual 20.7 and 22.7 at 5,202, 26.9 and 22.7 at 6,000; its action 14.5 and 17.0
+// at 5,184, 20.6 and 19.6 at 7,200. One cell to a few hundred: 6.3 and 10.4, residual 8.4 and 18.6.
+static bool hex27_by_lines(const DomainParams& p, int rheo, int op) {
+    const int per_sm = rheo != RHEO_GENMAXWELL ? 26 : (op == OP_RESIDUAL ? 36 : 44);
+    return p.ncells <= per_sm * (int64_t)sm_count();
+}
+
 bool launch_domain_apply_hexgroup(const DomainParams& p, int cell, int rheo, bool bf, int op, cudaStream_t s) {
     if (p.ncells == 0) return true;
     if (cell == HEX8) launch_hex8(p, rheo, bf, op, s);
+    else if (cell == HEX27 && hex27_by_lines(p, rheo, op)) launch_hex27_lines(p, rheo, bf, op, s);
     else if (cell == HEX27) launch_hex27(p, rheo, bf, op, s);
     else return false;
     return true;

@@ -60,6 +60,8 @@ void launch_hex8_jv32(const DomainParams& p, int rheo, cudaStream_t s);
 void launch_hex8_update_state(const DomainParams& p, cudaStream_t s);
 // Q2 hexahedra, a plane of nodes per lane (hex27.cu).
 void launch_hex27(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
+// The same with a line of points per lane, for small meshes (hex27lines.cu).
+void launch_hex27_lines(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
 // FP32 Jacobian action of hexahedra with a group of lanes per cell (FP64 geometry and tangent).
 bool launch_domain_jv32_hexgroup(const DomainParams& p, int cell, int rheo, cudaStream_t s);
 void launch_domain_jacobian(const DomainParams& p, int cell, int rheo, const int32_t* pos,

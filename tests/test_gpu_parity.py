@@ -998,3 +998,42 @@ def test_insert_takes_one_launch_where_nothing_starts_early(torch_cuda, ctx, cas
         ctx.synchronize()
         assert _lib.lib().pl_kernel_launches() - n0 == 1, c
         assert rel_l2(out.double().cpu().numpy(), ref.double().cpu().numpy()) <= (1e-6 if c == "f" else TOL64)
+
+
+# Q2: the last size by lines and the first by planes of each rheology and call (26, 36 and 44 cells per
+# multiprocessor), a part of a line warp's three cells, and one cell more than a block's six
+@pytest.mark.parametrize("genmaxwell", [False, True])
+@pytest.mark.parametrize("per_sm,extra", [(0, 2), (0, 7), (26, 0), (26, 1), (36, 0), (36, 1), (44, 0), (44, 1)])
+def test_q2_kernels_on_both_sides_of_their_rules(torch_cuda, ctx, genmaxwell, per_sm, extra):
+    """Residual (body force; INSERT and ADD) and action of Q2 hexahedra where the kernel changes, against
+    the thread-per-cell kernels."""
+    from pylith_b200 import feassemble as FA
+
+    torch = torch_cuda
+    nc = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    n = max(2, int(np.ceil(nc ** (1 / 3))))
+    mesh = M.box_hex27(n, n, n)
+    mesh.cells = mesh.cells[:nc].copy()
+    rng = np.random.default_rng(71)
+    dm = FA.DeviceMesh(ctx, mesh)
+    if genmaxwell:
+        ig = genmaxwell_setup(mesh, seed=72).create_integrator(dm, MAT.YEAR)
+    else:
+        ig = elastic_setup(mesh, seed=72, body_force=True).create_integrator(dm)
+    u = torch.from_numpy(rng.standard_normal(mesh.num_dof)).cuda()
+    calls = [lambda o, m: ig.compute_lhs_residual(0.0, MAT.YEAR, u, o, mode=m),
+             lambda o, m: ig.compute_lhs_jacobian_action(0.0, MAT.YEAR, 0.0, None, u, o, mode=m)]
+    refs = []
+    ig.set_scatter(FA.SCATTER_ATOMIC)
+    for call in calls:
+        refs.append(torch.zeros_like(u))
+        call(refs[-1], FA.ADD)
+    ig.set_scatter(FA.SCATTER_AUTO)
+    for call, ref in zip(calls, refs):
+        out = torch.full_like(u, np.nan)
+        call(out, FA.INSERT)
+        ctx.synchronize()
+        assert rel_l2(out.cpu().numpy(), ref.cpu().numpy()) <= TOL64
+        call(out, FA.ADD)
+        ctx.synchronize()
+        assert rel_l2(out.cpu().numpy(), 2 * ref.cpu().numpy()) <= TOL64
