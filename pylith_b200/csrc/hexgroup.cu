@@ -1,17 +1,16 @@
-// Hexahedral cells with a group of lanes per cell: the residual and Jacobian action of Q2
-// hexahedra (27 quadrature points), and the dispatch of all hexahedral kernels (Q1: hex8.cu).
+// Hexahedral cells with a group of lanes per cell: the generalized-Maxwell residual of small Q1 meshes and
+// the FP32 action of Q2; and the dispatch of all hexahedral kernels (Q1: hex8.cu, Q2 in FP64: hex27.cu,
+// hex27lines.cu).
 //
-// The thread-per-cell kernel (domain.cu) keeps a whole Q2 cell in one thread (81 accumulators,
-// 27 quadrature points in a loop) and spills. Here a warp shares one cell (27 lanes busy). Lane q
-// owns quadrature point q: it forms the trilinear geometry, the solution gradient from the cell's
-// node values staged in shared memory, calls the registered pointwise kernel and stages its
-// test-function weights wdetJ f1 J^{-T} (and wdetJ f0). Lane n then owns node n: it contracts the
-// staged weights with the reference basis gradients of node n over all quadrature points and adds
-// the result into the output (FP64 reductions; nodes are shared with neighbouring cells). The
-// reference basis tables (gradients and values at the quadrature points, and the trilinear
-// geometry gradients) are built once per block in shared memory. The FP32 variant (inner
-// iterations of the refined solver) keeps the geometry and the tangent in FP64 and stages the
-// field, the weights and the sums in FP32.
+// A warp shares one Q2 cell (27 lanes busy) or four Q1 cells (8 lanes each). Lane q owns quadrature
+// point q: it forms the trilinear geometry, the solution gradient from the cell's node values staged in
+// shared memory, calls the registered pointwise kernel and stages its test-function weights
+// wdetJ f1 J^{-T} (and wdetJ f0). Lane n then owns node n: it contracts the staged weights with the
+// reference basis gradients of node n over all quadrature points and adds the result into the output
+// (reductions; nodes are shared with neighbouring cells). The reference basis tables (gradients and
+// values at the quadrature points, and the trilinear geometry gradients) are built once per block in
+// shared memory. The FP32 action (inner iterations of the refined solver) keeps the geometry and the
+// tangent in FP64 and stages the field, the weights and the sums in FP32.
 #include "domain_kernels.cuh"
 #include "internal.hpp"
 #include "launch.hpp"
@@ -52,11 +51,15 @@ PL_D void fill_tables(double* t64, T* tt) {
     for (int i = threadIdx.x; i < H::NQ * H::NEN; i += blockDim.x) {
         const int q = i / H::NEN, n = i % H::NEN;
         double d[3];
-        const double x = gauss3_x(q % 3), y = gauss3_x((q / 3) % 3), z = gauss3_x(q / 9);
-        const int a = n % 3, b = (n / 3) % 3, c = n / 9;
-        d[0] = quad_d(a, x) * quad_v(b, y) * quad_v(c, z);
-        d[1] = quad_v(a, x) * quad_d(b, y) * quad_v(c, z);
-        d[2] = quad_v(a, x) * quad_v(b, y) * quad_d(c, z);
+        if (CELL == HEX8) {
+            hex_corner_dN<2>(n, q & 1, (q >> 1) & 1, q >> 2, d);
+        } else {
+            const double x = gauss3_x(q % 3), y = gauss3_x((q / 3) % 3), z = gauss3_x(q / 9);
+            const int a = n % 3, b = (n / 3) % 3, c = n / 9;
+            d[0] = quad_d(a, x) * quad_v(b, y) * quad_v(c, z);
+            d[1] = quad_v(a, x) * quad_d(b, y) * quad_v(c, z);
+            d[2] = quad_v(a, x) * quad_v(b, y) * quad_d(c, z);
+        }
 #pragma unroll
         for (int k = 0; k < 3; ++k) tt[q * H::LDB + n * 3 + k] = (T)d[k];
         tt[H::T_PHI + q * H::NEN + n] = (T)Elem<CELL>::phi(q, n);
@@ -64,12 +67,13 @@ PL_D void fill_tables(double* t64, T* tt) {
     for (int i = threadIdx.x; i < H::NQ * 8; i += blockDim.x) {
         const int q = i / 8, c = i % 8;
         double d[3];
-        hex_corner_dN<3>(c, q % 3, (q / 3) % 3, q / 9, d);
+        if (CELL == HEX8) hex_corner_dN<2>(c, q & 1, (q >> 1) & 1, q >> 2, d);
+        else hex_corner_dN<3>(c, q % 3, (q / 3) % 3, q / 9, d);
 #pragma unroll
         for (int k = 0; k < 3; ++k) t64[q * 25 + c * 3 + k] = d[k];
     }
     for (int q = threadIdx.x; q < H::NQ; q += blockDim.x)
-        t64[H::T_W + q] = gauss3_w(q % 3) * gauss3_w((q / 3) % 3) * gauss3_w(q / 9);
+        t64[H::T_W + q] = CELL == HEX8 ? 1.0 : gauss3_w(q % 3) * gauss3_w((q / 3) % 3) * gauss3_w(q / 9);
 }
 
 // Per-block tables and per-group staging of the group-of-lanes hexahedral kernels.
@@ -302,9 +306,20 @@ static bool hex27_by_lines(const DomainParams& p, int rheo, int op) {
     return p.ncells <= per_sm * (int64_t)sm_count();
 }
 
+// Generalized-Maxwell residual of Q1: a lane per point (this file) while that is at most one block of 32
+// cells per multiprocessor, a thread per cell (hex8.cu) beyond: the points' exponentials and state, one
+// after the other, are a longer chain. ADD: 8.4 and 10.4 us at 336 to 2,912 cells, 8.3 and 10.6 at 3,978,
+// 12.5 and 10.4 at 5,760.
+static bool hex8_by_points(const DomainParams& p, int rheo, int op) {
+    return rheo == RHEO_GENMAXWELL && op == OP_RESIDUAL && p.ncells <= 32 * (int64_t)sm_count();
+}
+
 bool launch_domain_apply_hexgroup(const DomainParams& p, int cell, int rheo, bool bf, int op, cudaStream_t s) {
     if (p.ncells == 0) return true;
-    if (cell == HEX8) launch_hex8(p, rheo, bf, op, s);
+    if (cell == HEX8 && hex8_by_points(p, rheo, op)) {
+        if (bf) launch_group_t<HEX8, RHEO_GENMAXWELL, true, OP_RESIDUAL>(p, s);
+        else launch_group_t<HEX8, RHEO_GENMAXWELL, false, OP_RESIDUAL>(p, s);
+    } else if (cell == HEX8) launch_hex8(p, rheo, bf, op, s);
     else if (cell == HEX27 && hex27_by_lines(p, rheo, op)) launch_hex27_lines(p, rheo, bf, op, s);
     else if (cell == HEX27) launch_hex27(p, rheo, bf, op, s);
     else return false;

@@ -1037,3 +1037,41 @@ def test_q2_kernels_on_both_sides_of_their_rules(torch_cuda, ctx, genmaxwell, pe
         call(out, FA.ADD)
         ctx.synchronize()
         assert rel_l2(out.cpu().numpy(), 2 * ref.cpu().numpy()) <= TOL64
+
+
+# a part of a warp's four cells and of a block's 32; the last size with a lane per point and the next
+@pytest.mark.parametrize("per_sm,extra", [(0, 3), (0, 33), (32, 0), (32, 1)])
+@pytest.mark.parametrize("body_force", [False, True])
+def test_genmaxwell_hex8_residual_on_both_sides_of_its_rule(oracle_lib, torch_cuda, ctx, per_sm, extra, body_force):
+    """The generalized-Maxwell residual of Q1 hexahedra (INSERT and ADD, with and without a body force)
+    where the kernel changes, against the oracle."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    nc = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    n = max(2, int(np.ceil(nc ** (1 / 3))))
+    mesh = M.box_hex(n, n, n)
+    mesh.cells = mesh.cells[:nc].copy()
+    g = genmaxwell_setup(mesh, seed=73)
+    aux = genmaxwell_oracle_aux(O, g)
+    u = np.random.default_rng(74).standard_normal(mesh.num_dof) * 1e-2
+    ig = g.create_integrator(FA.DeviceMesh(ctx, mesh), MAT.YEAR)
+    ref = O.residual(mesh, u, aux, f1=F1_GM, constants=[MAT.YEAR])
+    if body_force:
+        b = np.random.default_rng(75).standard_normal((nc, 3)) * 1e3
+        ig.set_aux("body_force", FA.PER_CELL, b)
+        k = FA.fekernels
+        ig.set_kernels_residual([FA.ResidualKernels("displacement", FA.LHS, k.Elasticity.g0v_bodyforce,
+                                                    k.IsotropicLinearGenMaxwell3D.f1v_infinitesimalStrain)])
+        plain = elastic_setup(mesh, seed=73)
+        with_b = O.AuxFields([(plain.density[:, None], "cell"), (b, "cell"), (plain.shear_modulus[:, None], "cell"),
+                              (plain.bulk_modulus[:, None], "cell")])
+        ref = ref + O.residual(mesh, 0 * u, with_b, f0="Elasticity::g0v_bodyforce", f1=F1_ILE)
+    du = dev(torch, u)
+    dr = torch.full_like(du, np.nan)
+    ig.compute_lhs_residual(0.0, MAT.YEAR, du, dr)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), ref) <= TOL64
+    ig.compute_lhs_residual(0.0, MAT.YEAR, du, dr, mode=FA.ADD)
+    ctx.synchronize()
+    assert rel_l2(dr.cpu().numpy(), 2 * ref) <= TOL64
