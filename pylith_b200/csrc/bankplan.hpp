@@ -34,14 +34,14 @@ inline void spread_nodes(const std::vector<std::vector<int>>& node_groups, int n
     const int nloc = (int)node_groups.size();
     perm.resize(nloc);
     for (int l = 0; l < nloc; ++l) perm[l] = l;
-    std::vector<uint8_t> cnt((size_t)ng * R, 0);  // (a group holds at most 32 distinct nodes)
+    std::vector<int> cnt((size_t)ng * R, 0);
     for (int l = 0; l < nloc; ++l)
         for (int g : node_groups[l]) cnt[(size_t)g * R + (perm[l] & (R - 1))]++;
     auto gmax = [&](int g) {
-        const uint8_t* c = &cnt[(size_t)g * R];
-        uint8_t m = 0;
+        const int* c = &cnt[(size_t)g * R];
+        int m = 0;
         for (int r = 0; r < R; ++r) m = m > c[r] ? m : c[r];
-        return (int)m;
+        return m;
     };
     auto move = [&](int l, int from, int to) {
         for (int g : node_groups[l]) {
@@ -88,65 +88,97 @@ inline void spread_nodes(const std::vector<std::vector<int>>& node_groups, int n
 // the least used bank. The warp of node k is group(k) and its lanes run the group's nodes in increasing
 // k. Returns the per-node ordered lists. Any fixed order keeps the sums identical from run to run.
 template <typename Group>
-std::vector<std::vector<int>> order_for_banks(std::vector<std::vector<int>> lists, int ngroups, Group group, int shift = 2,
+std::vector<std::vector<int>> order_for_banks(const std::vector<std::vector<int>>& lists, int ngroups, Group group, int shift = 2,
                                               int lanes_per_read = kWarp) {
-    constexpr int R = kBankPairs;
+    constexpr int R = kBankPairs, H = 2;  // a warp's reads go through in H groups of lanes at most
     const int nloc = (int)lists.size();
     std::vector<std::vector<int>> members(ngroups), ordered(nloc);
     for (int k = 0; k < nloc; ++k) members[group(k)].push_back(k);
+    // a lane's entries by bank: those of bank r that are left are entries[at[r]] .. entries[end[r]]
+    struct Lane {
+        int at[R], end[R], left;
+        uint32_t banks;  // with entries left
+    };
+    std::vector<int> entries, lanes, take, first;
+    std::vector<Lane> lane;
     for (const std::vector<int>& mem : members) {
         const int nl = (int)mem.size();
         if (nl == 0) continue;
-        int left[kWarp][R] = {};
-        for (int i = 0; i < nl; ++i)
-            for (int e : lists[mem[i]]) left[i % kWarp / lanes_per_read][(e >> shift) & (R - 1)]++;
-        std::vector<int> lanes(nl);
+        int left[H][R] = {};  // entries left of all lanes
+        lane.resize(nl);
+        entries.clear();
         int depth = 0;
-        for (int k : mem) depth = std::max(depth, (int)lists[k].size());
+        for (int i = 0; i < nl; ++i) {
+            Lane& L = lane[i];
+            const std::vector<int>& list = lists[mem[i]];
+            L.left = (int)list.size();
+            L.banks = 0;
+            depth = std::max(depth, L.left);
+            int n[R] = {}, at = (int)entries.size();
+            for (int e : list) n[(e >> shift) & (R - 1)]++;
+            for (int r = 0; r < R; ++r) {
+                L.at[r] = L.end[r] = at;
+                at += n[r];
+                L.banks |= (uint32_t)(n[r] > 0) << r;
+                left[i % kWarp / lanes_per_read][r] += n[r];
+            }
+            entries.resize(at);
+            for (int e : list) entries[L.end[(e >> shift) & (R - 1)]++] = e;
+            ordered[mem[i]].reserve(list.size());
+        }
+        lanes.resize(nl);
+        take.resize(nl);
+        first.resize(depth + 2);
         for (int j = 0; j < depth; ++j) {
-            int count[kWarp][R] = {};
-            for (int i = 0; i < nl; ++i) lanes[i] = i;
-            std::stable_sort(lanes.begin(), lanes.end(),
-                             [&](int x, int y) { return lists[mem[x]].size() > lists[mem[y]].size(); });
+            // lanes with the longest lists first
+            std::fill(first.begin(), first.end(), 0);
+            for (int i = 0; i < nl; ++i) first[depth - lane[i].left + 1]++, take[i] = -1;
+            for (int d = 0; d < depth; ++d) first[d + 1] += first[d];
+            for (int i = 0; i < nl; ++i) lanes[first[depth - lane[i].left]++] = i;
             // augmenting paths, longest lists first, the banks with the most entries left first
-            int owner[kWarp][R], take[kWarp];
-            std::fill(&owner[0][0], &owner[0][0] + kWarp * R, -1);
-            bool seen[R];
-            auto bank = [&](int e) { return (e >> shift) & (R - 1); };
+            int owner[H][R], count[H][R] = {};
+            std::fill(&owner[0][0], &owner[0][0] + H * R, -1);
+            uint32_t seen;
             auto augment = [&](auto&& self, int i) -> bool {
                 const int h = i % kWarp / lanes_per_read;
-                std::vector<int>& L = lists[mem[i]];
-                for (;;) {
-                    int best = -1;
-                    for (int t = 0; t < (int)L.size(); ++t)
-                        if (!seen[bank(L[t])] && (best < 0 || left[h][bank(L[t])] > left[h][bank(L[best])])) best = t;
-                    if (best < 0) return false;
-                    const int r = bank(L[best]), before = owner[h][r];
-                    seen[r] = true;
+                while (const uint32_t open = lane[i].banks & ~seen) {
+                    int best = __builtin_ctz(open);
+                    for (uint32_t o = open & (open - 1); o; o &= o - 1)
+                        if (left[h][__builtin_ctz(o)] > left[h][best]) best = __builtin_ctz(o);
+                    seen |= 1u << best;
+                    const int before = owner[h][best];
                     if (before >= 0 && !self(self, before)) continue;
-                    owner[h][r] = i;
-                    take[i] = L[best];
+                    owner[h][best] = i;
+                    take[i] = best;
                     return true;
                 }
+                return false;
             };
+            int unowned[H] = {};  // banks with entries left and no owner
+            for (int h = 0; h < H; ++h)
+                for (int r = 0; r < R; ++r) unowned[h] += left[h][r] > 0;
             for (int i : lanes) {
-                take[i] = -1;
-                std::fill(seen, seen + R, false);
-                augment(augment, i);
+                const int h = i % kWarp / lanes_per_read;
+                if (lane[i].left == 0) break;
+                seen = 0;
+                if (unowned[h] > 0 && augment(augment, i)) unowned[h]--;
             }
             for (int i : lanes)
-                if (take[i] >= 0) count[i % kWarp / lanes_per_read][bank(take[i])]++;
+                if (take[i] >= 0) count[i % kWarp / lanes_per_read][take[i]]++;
             for (int i : lanes) {
-                std::vector<int>& L = lists[mem[i]];
-                if (L.empty()) continue;
+                Lane& L = lane[i];
+                if (L.left == 0) break;
                 const int h = i % kWarp / lanes_per_read;
                 if (take[i] < 0) {
-                    take[i] = *std::min_element(L.begin(), L.end(), [&](int x, int y) { return count[h][bank(x)] < count[h][bank(y)]; });
-                    count[h][bank(take[i])]++;
+                    for (int r = 0; r < R; ++r)
+                        if (L.banks >> r & 1 && (take[i] < 0 || count[h][r] < count[h][take[i]])) take[i] = r;
+                    count[h][take[i]]++;
                 }
-                left[h][bank(take[i])]--;
-                ordered[mem[i]].push_back(take[i]);
-                L.erase(std::find(L.begin(), L.end(), take[i]));
+                const int r = take[i];
+                left[h][r]--;
+                L.left--;
+                ordered[mem[i]].push_back(entries[L.at[r]++]);
+                if (L.at[r] == L.end[r]) L.banks &= ~(1u << r);
             }
         }
     }

@@ -355,7 +355,7 @@ namespace {
 
 constexpr int kHalf = 16;       // lanes whose 64-bit reads go through together (bankplan.hpp)
 // Steps of the numbering's search: 4,000 leave 2.7 cycles per gather of a warp (ideal 2; 3.7 when whole
-// warps are planned), 16,000 leave 2.4: 43.3 and 42.3 us on 1,296,000 cells, first call 350 and 799 ms.
+// warps are planned), 16,000 leave 2.4 and plan more than twice as long: 43.3 and 42.3 us on 1,296,000 cells.
 constexpr int kPlanSteps = 4000;
 
 struct PairPlan {
@@ -384,32 +384,38 @@ void apex_last(const int* v, int k, int32_t (&out)[4]) {
 // cells with the fewest free neighbours first. Pairs whose orientations do not fit (cells that are
 // not consistently oriented across the face) stay single.
 std::vector<Item> match_cells(const std::vector<int>& lc, int ncell) {
-    struct Face {
-        uint64_t key;
-        int cell, k;
-    };
-    std::vector<Face> faces;
+    static_assert(kPairMaxNodes <= 256 && kPairCells <= 256, "a face (three local nodes), its cell and corner in one word");
+    std::vector<uint64_t> faces;
     faces.reserve(4 * (size_t)ncell);
     for (int c = 0; c < ncell; ++c)
         for (int k = 0; k < 4; ++k) {
             int f[3], m = 0;
             for (int i = 0; i < 4; ++i)
                 if (i != k) f[m++] = lc[4 * c + i];
-            std::sort(f, f + 3);
-            faces.push_back({(uint64_t)f[0] << 40 | (uint64_t)f[1] << 20 | (uint64_t)f[2], c, k});
+            if (f[0] > f[1]) std::swap(f[0], f[1]);
+            if (f[1] > f[2]) std::swap(f[1], f[2]);
+            if (f[0] > f[1]) std::swap(f[0], f[1]);
+            faces.push_back((uint64_t)f[0] << 32 | (uint64_t)f[1] << 24 | (uint64_t)f[2] << 16 | (uint64_t)c << 2 | (uint64_t)k);
         }
-    std::sort(faces.begin(), faces.end(), [](const Face& x, const Face& y) {
-        return x.key != y.key ? x.key < y.key : (x.cell != y.cell ? x.cell < y.cell : x.k < y.k);
-    });
+    std::sort(faces.begin(), faces.end());
     struct Edge {
         int cell, k, k2;  // neighbour, this cell's and its corner off the face
     };
-    std::vector<std::vector<Edge>> adj(ncell);
-    for (size_t i = 0; i + 1 < faces.size(); ++i)
-        if (faces[i].key == faces[i + 1].key && faces[i].cell != faces[i + 1].cell) {
-            adj[faces[i].cell].push_back({faces[i + 1].cell, faces[i].k, faces[i + 1].k});
-            adj[faces[i + 1].cell].push_back({faces[i].cell, faces[i + 1].k, faces[i].k});
-        }
+    struct Edges {
+        int count = 0;
+        Edge e[8];  // (a face that more than two cells share gives a cell two)
+        const Edge* begin() const { return e; }
+        const Edge* end() const { return e + count; }
+        int size() const { return count; }
+        void push_back(const Edge& x) { e[count++] = x; }
+    };
+    std::vector<Edges> adj(ncell);
+    for (size_t i = 0; i + 1 < faces.size(); ++i) {
+        const int c = (int)(faces[i] >> 2 & 0x3fff), d = (int)(faces[i + 1] >> 2 & 0x3fff);
+        if (faces[i] >> 16 != faces[i + 1] >> 16 || c == d) continue;
+        adj[c].push_back({d, (int)(faces[i] & 3), (int)(faces[i + 1] & 3)});
+        adj[d].push_back({c, (int)(faces[i + 1] & 3), (int)(faces[i] & 3)});
+    }
     std::vector<int> deg(ncell);
     std::vector<char> used(ncell, 0);
     using Q = std::pair<int, int>;
@@ -461,18 +467,55 @@ std::vector<Item> match_cells(const std::vector<int>& lc, int ncell) {
     return items;
 }
 
-// Plans one block of the cells c0 .. c0 + ncell - 1 (connectivity bc[ncell][4]); false when they need more items or nodes than a block has.
-bool plan_pair_block(const int32_t* bc, int64_t c0, int ncell, PairPlan& P) {
-    std::vector<int32_t> sorted(bc, bc + 4 * (size_t)ncell);
-    std::sort(sorted.begin(), sorted.end());
-    sorted.erase(std::unique(sorted.begin(), sorted.end()), sorted.end());
-    const int nloc = (int)sorted.size();
-    if (nloc > kPairMaxNodes) return false;
+// A block: its cell count, its nodes in increasing order, and its items (local nodes: indices into them).
+struct PairCut {
+    int ncell;
+    std::vector<int32_t> nodes;
+    std::vector<Item> items;
+};
+
+// The block of the ncell cells bc[ncell][4]; returns 0, or where they need more items or nodes than a block
+// has, how many cells fewer it must be at least (a cell less saves an item or four nodes at most).
+int cut_pair_block(const int32_t* bc, int ncell, PairCut& cut) {
+    cut.ncell = ncell;
+    std::vector<uint64_t> at(4 * (size_t)ncell);  // (node, corner)
+    for (int i = 0; i < 4 * ncell; ++i) at[i] = (uint64_t)bc[i] << 32 | (uint32_t)i;
+    std::sort(at.begin(), at.end());
+    cut.nodes.clear();
     std::vector<int> lc(4 * (size_t)ncell);
-    for (int i = 0; i < 4 * ncell; ++i) lc[i] = (int)(std::lower_bound(sorted.begin(), sorted.end(), bc[i]) - sorted.begin());
-    const std::vector<Item> items = match_cells(lc, ncell);
-    const int ni = (int)items.size();
-    if (ni > kPairThreads) return false;
+    for (uint64_t x : at) {
+        const int32_t v = (int32_t)(x >> 32);
+        if (cut.nodes.empty() || cut.nodes.back() != v) cut.nodes.push_back(v);
+        lc[(uint32_t)x] = (int)cut.nodes.size() - 1;
+    }
+    const int nodes = (int)cut.nodes.size();
+    if (nodes > kPairMaxNodes) return (nodes - kPairMaxNodes + 3) / 4;
+    cut.items = match_cells(lc, ncell);
+    return std::max(0, (int)cut.items.size() - kPairThreads);
+}
+
+// Blocks of the cells [begin, end): as even as kPairCells allows, a block that does not fit shrunk; false
+// for scattered cells (see ensure_pair_layout). A few per cent of the planning: all of a mesh is cut
+// before any of it is planned.
+bool cut_pair_range(const int32_t* cells, int64_t begin, int64_t end, std::vector<PairCut>& out) {
+    for (int64_t c = begin; c < end;) {
+        const int64_t left = end - c, nb = (left + kPairCells - 1) / kPairCells;
+        int n = (int)((left + nb - 1) / nb);
+        PairCut cut;
+        for (int fewer; (fewer = cut_pair_block(cells + 4 * c, n, cut)) > 0;) {
+            for (const int most = n - fewer; n > most; n -= std::max(2, n / 16))
+                if (n <= kPairCells / 2) return false;
+        }
+        out.push_back(std::move(cut));
+        c += n;
+    }
+    return true;
+}
+
+// Numbers the nodes and orders the incidences of the block that starts at cell c0.
+void plan_pair_block(int64_t c0, const PairCut& cut, PairPlan& P) {
+    const std::vector<Item>& items = cut.items;
+    const int nloc = (int)cut.nodes.size(), ni = (int)items.size();
     std::vector<std::vector<int>> groups(nloc);
     std::vector<int> deg(nloc, 0);
     for (int i = 0; i < ni; ++i)
@@ -484,7 +527,7 @@ bool plan_pair_block(const int32_t* bc, int64_t c0, int ncell, PairPlan& P) {
     std::vector<int32_t> perm;
     spread_nodes(groups, (ni + kHalf - 1) / kHalf * 5, deg, (uint64_t)c0, kPlanSteps, perm);
     P.loc.resize(nloc);
-    for (int l = 0; l < nloc; ++l) P.loc[perm[l]] = sorted[l];
+    for (int l = 0; l < nloc; ++l) P.loc[perm[l]] = cut.nodes[l];
     std::vector<std::vector<int>> lists(nloc);
     P.items.clear();
     for (int i = 0; i < ni; ++i) {
@@ -503,23 +546,6 @@ bool plan_pair_block(const int32_t* bc, int64_t c0, int ncell, PairPlan& P) {
         for (int e : ordered[k]) P.inc.push_back((uint16_t)((e & 7) * 3 * kPairThreads + (e >> 3)));
         P.off.push_back((uint16_t)P.inc.size());
     }
-    return true;
-}
-
-// Blocks of the cells [begin, end): as even as kPairCells allows, a block that does not fit shrunk.
-bool plan_pair_range(const int32_t* cells, int64_t begin, int64_t end, std::vector<PairPlan>& out) {
-    for (int64_t c = begin; c < end;) {
-        const int64_t left = end - c, nb = (left + kPairCells - 1) / kPairCells;
-        int n = (int)((left + nb - 1) / nb);
-        PairPlan P;
-        while (!plan_pair_block(cells + 4 * c, c, n, P)) {
-            if (n <= kPairCells / 2) return false;  // scattered cells: see ensure_pair_layout
-            n -= std::max(2, n / 16);
-        }
-        out.push_back(std::move(P));
-        c += n;
-    }
-    return true;
 }
 
 int build_pair_layout(pl_mesh_s* m) {
@@ -532,24 +558,37 @@ int build_pair_layout(pl_mesh_s* m) {
     const int64_t nc = m->ncells, want = (nc + kPairCells - 1) / kPairCells;
     const int64_t per = std::max<int64_t>(1, std::min<int64_t>(16, want / 64)), nr = (want + per - 1) / per;
     std::vector<std::vector<PairPlan>> plans(nr);
-    std::atomic<int64_t> next{0};
     std::atomic<bool> failed{false}, refused{false};
-    auto work = [&]() noexcept {
+    auto all_ranges = [&](auto&& range) {  // range(r, first cell, last): false where the mesh is refused
+        std::atomic<int64_t> next{0};
+        auto work = [&]() noexcept {
+            try {
+                for (int64_t r; !failed.load() && !refused.load() && (r = next.fetch_add(1)) < nr;)
+                    if (!range(r, r * nc / nr, (r + 1) * nc / nr)) refused.store(true);
+            } catch (...) {
+                failed.store(true);
+            }
+        };
+        const int nth = (int)std::min<int64_t>(std::min(15u, std::thread::hardware_concurrency()), nr);
+        std::vector<std::thread> th;
         try {
-            for (int64_t r; !failed.load() && !refused.load() && (r = next.fetch_add(1)) < nr;)
-                if (!plan_pair_range(m->h_cells.data(), r * nc / nr, (r + 1) * nc / nr, plans[r])) refused.store(true);
+            for (int t = 1; t < nth; ++t) th.emplace_back(work);
         } catch (...) {
-            failed.store(true);
         }
+        work();
+        for (std::thread& x : th) x.join();
     };
-    const int nth = (int)std::min<int64_t>(std::min(15u, std::thread::hardware_concurrency()), nr);
-    std::vector<std::thread> th;
-    try {
-        for (int t = 1; t < nth; ++t) th.emplace_back(work);
-    } catch (...) {
-    }
-    work();
-    for (std::thread& x : th) x.join();
+    std::vector<std::vector<PairCut>> cuts(nr);
+    all_ranges([&](int64_t r, int64_t c0, int64_t c1) { return cut_pair_range(m->h_cells.data(), c0, c1, cuts[r]); });
+    if (!refused.load()) all_ranges([&](int64_t r, int64_t c, int64_t) {
+        for (PairCut& cut : cuts[r]) {
+            plans[r].emplace_back();
+            plan_pair_block(c, cut, plans[r].back());
+            c += cut.ncell;
+            cut = PairCut();
+        }
+        return true;
+    });
     if (failed.load()) return fail(PL_ERR_OUT_OF_MEMORY, "cell-pair layout planning ran out of host memory");
     if (refused.load()) return PL_OK;
     int maxloc = 0;
@@ -667,9 +706,15 @@ static bool tet_pairs_selected() {
 }
 
 // The mesh's pair layout (num_blocks 0: not usable). Meshes whose consecutive cells are scattered, so
-// that a block of kPairCells / 2 of them does not fit, keep the layout of single cells: 384,000 cells
-// shuffled throughout run 48.0 us there and 52.2 here (first call 252 and 386 ms); in their own order
-// 27.6 and 23.5 (235 and 132 ms).
+// that a block of kPairCells / 2 of them does not fit, keep the layout of single cells; the blocks are cut
+// before any is planned, so that such a mesh pays little for the attempt. Residual here and there, first
+// call in brackets, in us (ms):
+//   1,179,648 structured cells along a Morton curve 35.0 and 48.4 (253 and 597), in grid order, with
+//     kPairMaxNodes slots per block, 35.1 and 47.4 (198 and 432)
+//   394,718 Delaunay cells along a Morton curve 16.5 and 21.7 (90 and 210), in Qhull's order 18.7 and 31.9
+//     (89 and 186)
+//   384,000 cells shuffled within windows of 480 21.5 and 29.8 (121 to 170 and 231); of 10,000, refused,
+//     44.4 either way (207 and 202 without the attempt); shuffled throughout, if forced, 52.2 and 48.0
 int ensure_pair_layout(pl_mesh_s* m) {
     if (m->pair) return PL_OK;
     int rc;

@@ -10,7 +10,8 @@ namespace plb {
 constexpr int kPairThreads = 128;    // items (pairs or single cells) of a block at most
 constexpr int kPairCells = 240;      // cells of a block at most: about 122 items
 constexpr int kPairMaxNodes = 2 * kPairThreads;  // nodes of a block at most (two per thread)
-constexpr int kPairSmallLd = 144;    // slots per block where all of a mesh's blocks fit (compact ones do)
+constexpr int kPairSmallLd = 144;    // slots per block where all of a mesh's blocks fit (compact ones do; else
+                                     // kPairMaxNodes: 35.0 and 35.1 us, see ensure_pair_layout in tetpair.cu)
 constexpr uint32_t kPairShared = 0x80000000u;
 constexpr uint32_t kNoNode = 0xffffffffu, kNoItem = 0xffffffffu;
 constexpr int kCellBias = 0x8000;
