@@ -1075,3 +1075,24 @@ def test_genmaxwell_hex8_residual_on_both_sides_of_its_rule(oracle_lib, torch_cu
     ig.compute_lhs_residual(0.0, MAT.YEAR, du, dr, mode=FA.ADD)
     ctx.synchronize()
     assert rel_l2(dr.cpu().numpy(), 2 * ref) <= TOL64
+
+
+# the last size whose state fits 128 MB and the first that does not
+@pytest.mark.parametrize("nc", [87381, 87382])
+def test_genmaxwell_hex8_state_update_on_both_sides_of_its_rule(oracle_lib, torch_cuda, ctx, nc):
+    """The state update of Q1 hexahedra where the kernel changes, against the oracle."""
+    from pylith_b200 import feassemble as FA
+
+    O, torch = oracle_lib, torch_cuda
+    mesh = M.box_hex(45, 45, 44)
+    mesh.cells = mesh.cells[:nc].copy()
+    g = genmaxwell_setup(mesh, seed=76)
+    u = np.random.default_rng(77).standard_normal(mesh.num_dof) * 1e-2
+    visc, total = O.project_qp(
+        mesh, u, genmaxwell_oracle_aux(O, g), ["IsotropicLinearGenMaxwell3D::viscousStrain_infinitesimalStrain_asVector",
+                                               "Elasticity3D::infinitesimalStrain_asVector"], [18, 6], constants=[MAT.YEAR])
+    ig = g.create_integrator(FA.DeviceMesh(ctx, mesh), MAT.YEAR)
+    ig.update_state_vars(0.0, MAT.YEAR, dev(torch, u))
+    ctx.synchronize()
+    assert rel_l2(ig.get_aux("viscous_strain", (nc, 8, 18)), visc) <= TOL64
+    assert rel_l2(ig.get_aux("total_strain", (nc, 8, 6)), total) <= TOL64
