@@ -232,6 +232,24 @@ __global__ void __launch_bounds__(128) k_domain_update_state(DomainParams p) {
     }
 }
 
+// One project kernel at a point with gradient s_x and aux a.
+template <int RHEO>
+PL_D void derived_point(const DomainParams& p, int kind, const double* s_x, const double* a, double (&o)[6]) {
+    using L = AuxLayout<RHEO, false>;
+    const AuxOffsets<RHEO, false> aoff;
+    const int sOff[1] = {0}, sOff_x[1] = {0};
+    double x[3] = {0, 0, 0};
+    if (kind == K_EL_STRAIN_VECTOR)
+        pw::el3d_strain_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a, nullptr, nullptr, p.t,
+                                       x, p.num_constants, p.constants, o);
+    else if (RHEO == RHEO_ILE && kind == K_ILE_STRESS_VECTOR)
+        pw::ile3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a, nullptr, nullptr, p.t,
+                                        x, p.num_constants, p.constants, o);
+    else if (RHEO == RHEO_GENMAXWELL && kind == K_GM_STRESS_VECTOR)
+        pw::gm3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a, nullptr, nullptr, p.t,
+                                       x, p.num_constants, p.constants, o);
+}
+
 // Derived fields of basis order 0 (IntegratorDomain::_computeDerivedField,
 // IntegratorDomain.cc:596-630, with PyLith's default basis order 0 for cauchy_stress and
 // cauchy_strain, DerivedSubfieldsElasticity.py:42-44): each registered project kernel evaluated
@@ -241,7 +259,8 @@ __global__ void __launch_bounds__(128) k_domain_update_state(DomainParams p) {
 // Bound: L2, at first by the stores: a thread's six values per kernel lie in a row of its own, so a
 // warp's store touched 32 sectors. Rows are staged in shared memory and a warp stores its cells' rows
 // with consecutive lanes on consecutive doubles; node ids, coordinates and field are read before
-// they are used: stress and strain of 100,345 Q1 hexahedra 12.9 -> 8.2 us.
+// they are used: stress and strain of 100,345 Q1 hexahedra 12.9 -> 8.2 us with the nodes in L2; with L2
+// cold 36,720 cells 11.5 -> 9.9, 196,608 24.6 -> 18.4.
 constexpr int kDerivedThreads = 128;
 constexpr int kDerivedRow = 6 * 4 + 1;  // values of a cell at most; odd, so a warp's accesses spread over the banks
 template <int CELL, int RHEO>
@@ -250,7 +269,6 @@ __global__ void __launch_bounds__(kDerivedThreads) k_domain_derived(DomainParams
     using L = AuxLayout<RHEO, false>;
     constexpr int AHEAD = E::nen <= 8 ? E::nen : 1;  // nodes held in registers
     __shared__ double rows[kDerivedThreads * kDerivedRow];
-    const AuxOffsets<RHEO, false> aoff;
     const int nout = 6 * spec.n, lane = threadIdx.x & 31;
     double* const wrow = rows + (threadIdx.x - lane) * kDerivedRow;  // the warp's rows
     for (int64_t c0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane; c0 < p.ncells;
@@ -299,19 +317,9 @@ __global__ void __launch_bounds__(kDerivedThreads) k_domain_derived(DomainParams
             } else {
                 for (int n = 0; n < E::nen; ++n) add(n, p.u + 3 * (int64_t)cn[n]);
             }
-            const int sOff[1] = {0}, sOff_x[1] = {0};
-            double x[3] = {0, 0, 0};
             for (int k = 0; k < spec.n; ++k) {
                 double o[6] = {0, 0, 0, 0, 0, 0};
-                if (spec.kind[k] == K_EL_STRAIN_VECTOR)
-                    pw::el3d_strain_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
-                                                   nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
-                else if (RHEO == RHEO_ILE && spec.kind[k] == K_ILE_STRESS_VECTOR)
-                    pw::ile3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
-                                                    nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
-                else if (RHEO == RHEO_GENMAXWELL && spec.kind[k] == K_GM_STRESS_VECTOR)
-                    pw::gm3d_stress_vector<double>(3, 1, L::numA, sOff, sOff_x, nullptr, nullptr, s_x, aoff.v, nullptr, a,
-                                                   nullptr, nullptr, p.t, x, p.num_constants, p.constants, o);
+                derived_point<RHEO>(p, spec.kind[k], s_x, a, o);
 #pragma unroll
                 for (int i = 0; i < 6; ++i) wrow[lane * kDerivedRow + 6 * k + i] = o[i];
             }
@@ -327,6 +335,48 @@ __global__ void __launch_bounds__(kDerivedThreads) k_domain_derived(DomainParams
             if (col >= nout) ++row, col -= nout;
         }
         __syncwarp();
+    }
+}
+
+// The same without staging, for Q2 meshes of up to a block per multiprocessor, where the row stores do not
+// count and the shorter code does: 384 to 11,520 cells, L2 cold, 12.3 us and 14.3 staged; 24,576 cells and
+// four kernels 10.5 us and 8.3 staged.
+template <int CELL, int RHEO>
+__global__ void __launch_bounds__(kDerivedThreads) k_domain_derived_direct(DomainParams p, DerivedSpec spec) {
+    using E = Elem<CELL>;
+    using L = AuxLayout<RHEO, false>;
+    const int nout = 6 * spec.n;
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= p.ncells) return;
+    const int32_t* cn = p.cells + (p.cell_ids ? p.cell_ids[c] : c) * E::nen;
+    double X[E::ngeom][3];
+#pragma unroll
+    for (int k = 0; k < E::ngeom; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) X[k][i] = p.coords[3 * (int64_t)cn[E::corner(k)] + i];
+    Geom g;
+    E::centre_geom(X, &g);
+    if (!(g.detJ > 0.0)) flag_error(p.err, CHECK_NONPOSITIVE_DETJ);
+    double s_x[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int n = 0; n < E::nen; ++n) {
+        double gr[3];
+        E::centre_grad(g, n, gr);
+        const double* un = p.u + 3 * (int64_t)cn[n];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            s_x[0 + d] += un[0] * gr[d];
+            s_x[3 + d] += un[1] * gr[d];
+            s_x[6 + d] += un[2] * gr[d];
+        }
+    }
+    double a[L::size] = {};
+    L::load_cell(p, c, a);
+    L::load_qp(p, c, 0, E::nq, a);
+    for (int k = 0; k < spec.n; ++k) {
+        double o[6] = {0, 0, 0, 0, 0, 0};
+        derived_point<RHEO>(p, spec.kind[k], s_x, a, o);
+#pragma unroll
+        for (int i = 0; i < 6; ++i) p.out[c * nout + 6 * k + i] = o[i];
     }
 }
 
@@ -441,7 +491,11 @@ void launch_domain_derived(const DomainParams& p, int cell, int rheo, const Deri
     if (p.ncells == 0) return;
     const int th = kDerivedThreads;
     const int gr = grid_for(p.ncells, th);
-    if (rheo == RHEO_GENMAXWELL) {
+    if (cell == HEX27 && p.ncells <= (int64_t)th * sm_count()) {
+        const int blocks = (int)((p.ncells + th - 1) / th);
+        if (rheo == RHEO_GENMAXWELL) k_domain_derived_direct<HEX27, RHEO_GENMAXWELL><<<blocks, th, 0, s>>>(p, spec);
+        else k_domain_derived_direct<HEX27, RHEO_ILE><<<blocks, th, 0, s>>>(p, spec);
+    } else if (rheo == RHEO_GENMAXWELL) {
         if (cell == TET4) k_domain_derived<TET4, RHEO_GENMAXWELL><<<gr, th, 0, s>>>(p, spec);
         else if (cell == HEX8) k_domain_derived<HEX8, RHEO_GENMAXWELL><<<gr, th, 0, s>>>(p, spec);
         else k_domain_derived<HEX27, RHEO_GENMAXWELL><<<gr, th, 0, s>>>(p, spec);

@@ -1096,3 +1096,39 @@ def test_genmaxwell_hex8_state_update_on_both_sides_of_its_rule(oracle_lib, torc
     ctx.synchronize()
     assert rel_l2(ig.get_aux("viscous_strain", (nc, 8, 18)), visc) <= TOL64
     assert rel_l2(ig.get_aux("total_strain", (nc, 8, 6)), total) <= TOL64
+
+
+# Q2: one cell, a warp and a block and one more of each; the last size without staged rows and the next
+@pytest.mark.parametrize("per_sm,extra", [(0, 1), (0, 33), (0, 129), (128, 0), (128, 1)])
+@pytest.mark.parametrize("num", [2, 4])
+def test_derived_rows_of_q2(torch_cuda, ctx, per_sm, extra, num):
+    """Derived fields of Q2 hexahedra where the kernel changes, for a displacement of constant gradient:
+    every cell's strain is that gradient's, its stress follows, and nothing is written past the last row."""
+    from pylith_b200 import feassemble as FA
+
+    torch = torch_cuda
+    nc = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    n = max(2, int(np.ceil(nc ** (1 / 3))))
+    mesh = M.box_hex27(n, n, n)
+    mesh.cells = mesh.cells[:nc].copy()
+    mat = elastic_setup(mesh, seed=95)
+    G = np.random.default_rng(96).standard_normal((3, 3)) * 1e-3
+    e = 0.5 * (G + G.T)
+    strain = np.tile(e[[0, 1, 2, 0, 1, 0], [0, 1, 2, 1, 2, 2]], (nc, 1))
+    lam = mat.bulk_modulus - 2.0 / 3.0 * mat.shear_modulus
+    stress = 2.0 * mat.shear_modulus[:, None] * strain
+    stress[:, :3] += (lam * np.trace(e))[:, None]
+    k = FA.fekernels
+    f_stress = k.IsotropicLinearElasticity3D.cauchyStress_infinitesimalStrain_asVector
+    f_strain = k.Elasticity3D.infinitesimalStrain_asVector
+    ig = mat.create_integrator(FA.DeviceMesh(ctx, mesh))
+    ig.set_kernels_derived_field([FA.ProjectKernels(f"field_{i}", f_strain if i % 2 else f_stress) for i in range(num)])
+    out = torch.full((nc + 1, 6 * num), np.nan, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ig.compute_derived_field(0.0, 0.0, dev(torch, (mesh.coords @ G.T).ravel()), out)
+    ctx.synchronize()
+    got = out.cpu().numpy()
+    assert np.isnan(got[nc]).all()
+    # (differences of displacements of up to 20 m over cells of 400 m and more, u and x rounded: 1e-11)
+    for i in range(num):
+        assert rel_l2(got[:nc, 6 * i:6 * i + 6], strain if i % 2 else stress) <= 1e-10
