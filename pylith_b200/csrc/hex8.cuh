@@ -285,6 +285,15 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
                 mu = (T)(-Jf3[((0 * 3 + 1) * 3 + 1) * 3 + 0]);
             }
         }
+        T scale = T(0.125);
+        if constexpr (F32) {
+            // the moduli as multiples of a power of two, applied to the node sums: modulus / det would leave
+            // FP32's range where a cell is smaller than about 1e-9 m with moduli in Pa
+            const unsigned e = min(max(__float_as_uint(lam + 2.0f * mu) >> 23 & 0xffu, 1u), 253u);
+            const float to_one = __uint_as_float((254u - e) << 23);
+            lam *= to_one, mu *= to_one;
+            scale *= __uint_as_float(e << 23);
+        }
         [[maybe_unused]] pw::MaxwellFactors<double> mf;
         // once per cell: evaluated at each point, the exponentials made the unrolled code overflow the
         // instruction cache (69 us against 44 for the residual of 48x48x36 cells)
@@ -299,13 +308,7 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
                     for (int e = 0; e < 3; ++e)
                         s_x[f * 3 + e] = G[f][0] * C[0][e] + G[f][1] * C[1][e] + G[f][2] * C[2][e];
                 if constexpr (OP == OP_JACOBIAN_ACTION) {
-                    // The flux is linear in the gradient: the division by det is applied to the moduli, in
-                    // FP32 to the six fluxes (modulus / det leaves its range where a cell is smaller than
-                    // about 1e-9 m with moduli in Pa; a static solve takes 1 % longer with it).
-                    isotropic_contract<T>(F32 ? lam : lam * rdet, F32 ? mu : mu * rdet, s_x, f1);
-                    if constexpr (F32)
-#pragma unroll
-                        for (int f = 0; f < 9; ++f) f1[f] *= rdet;
+                    isotropic_contract<T>(lam * rdet, mu * rdet, s_x, f1);  // linear in the gradient
                 } else {
 #pragma unroll
                     for (int f = 0; f < 9; ++f) s_x[f] *= rdet;
@@ -335,7 +338,7 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) g[n][d] *= T(0.125);
+            for (int d = 0; d < 3; ++d) g[n][d] *= scale;
     }
     __syncwarp();
     wait_for_previous();  // see zero_output
