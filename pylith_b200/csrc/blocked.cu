@@ -1026,9 +1026,11 @@ static void launch_pipe_t(const DomainParams& p, const BlockedLayout& b, bool in
     }
 }
 
-// Which FP64 kernel of this file runs, read once per process from PYLITH_B200_TET_KERNEL: "pad2" (also
-// where the variable is unset and the pairs of tetpair.cu do not serve the mesh: two barriers per block over the padded layout), "pipe" (one barrier per block over the
-// padded layout) or "twophase" (two barriers per block, per-thread 8-byte gathers of all node data).
+// Which FP64 kernel of this file runs, read once per process from PYLITH_B200_TET_KERNEL: "pad2" (two
+// barriers per block over the padded layout), "pipe" (one barrier per block over the padded layout) or
+// "twophase" (two barriers per block, per-thread 8-byte gathers of all node data). Unset, on meshes that the
+// pairs of tetpair.cu refuse: pad2 where its shared memory holds the largest block (about 256 nodes, which
+// such meshes exceed), else twophase.
 enum TetKernel { TK_PAD2, TK_PIPE, TK_TWOPHASE };
 static TetKernel tet_kernel_choice() {
     static const TetKernel k = [] {

@@ -3,12 +3,12 @@
 // Bound: FP64 arithmetic, about 1,350 operations per cell (65 % of the FP64 pipe busy at 8 warps per
 // multiprocessor, DRAM 13 %); FP32, instruction issue and latency. One thread per cell takes the
 // whole sweep into registers (254 in FP64), where 8 lanes per cell staged every contraction through
-// shared memory: on the 96x96x72 box (663,552 cells) the FP64 residual went from 293 to 84 us, the
-// FP64 action from 277 to 79 us and the FP32 action from 207 to 55 us. The reductions alone, 16 M
+// shared memory: on the 96x96x72 box (663,552 cells), numbered along x, the FP64 residual went from 275
+// to 78 us, the FP64 action from 275 to 74 us and the FP32 action from 192 to 45 us; numbered along a
+// Morton curve 264, 264, 185 -> 94, 90, 60; shuffled 293, 293, 212 -> 131, 127, 115. The reductions alone, 16 M
 // on that box, take 58 us in FP64 when each cell adds its own 24 sums and 31 us when consecutive
 // cells hand on their shared face (hex8_scatter). FP32 with 6 blocks of 64 threads per
-// multiprocessor (145 registers, no spills) measured 62 us against 55 us with 8 (128 registers, 36
-// bytes spilled).
+// multiprocessor (145 registers) was slower than with 8 (128): 62 against 55 us when measured.
 #include <algorithm>
 
 #include "hex8.cuh"

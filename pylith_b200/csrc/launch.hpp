@@ -51,8 +51,8 @@ bool launch_tangent_lm32(const DomainParams& p, int rheo, float* out, cudaStream
 void launch_domain_apply_atomic(const DomainParams& p, int cell, int rheo, bool bf, int op,
                                 cudaStream_t s);
 void launch_domain_jv_f32_atomic(const DomainParams& p, int cell, int rheo, cudaStream_t s);
-// Hexahedra (Q1, Q2) with a group of lanes per cell (FP64 residual / Jacobian action, FP64
-// reductions into the output); returns false for other cell types.
+// FP64 residual / Jacobian action of hexahedra (Q1, Q2; FP64 reductions into the output), by the kernel
+// that suits the size (hexgroup.cu); returns false for other cell types.
 bool launch_domain_apply_hexgroup(const DomainParams& p, int cell, int rheo, bool bf, int op, cudaStream_t s);
 // Q1 hexahedra, one thread per cell (hex8.cu).
 void launch_hex8(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
@@ -62,7 +62,8 @@ void launch_hex8_update_state(const DomainParams& p, cudaStream_t s);
 void launch_hex27(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
 // The same with a line of points per lane, for small meshes (hex27lines.cu).
 void launch_hex27_lines(const DomainParams& p, int rheo, bool bf, int op, cudaStream_t s);
-// FP32 Jacobian action of hexahedra with a group of lanes per cell (FP64 geometry and tangent).
+// FP32 Jacobian action of hexahedra: Q1 with a thread per cell (hex8.cu; FP32 geometry from coordinates
+// differenced in FP64), Q2 with a group of lanes per cell (FP64 geometry and tangent).
 bool launch_domain_jv32_hexgroup(const DomainParams& p, int cell, int rheo, cudaStream_t s);
 void launch_domain_jacobian(const DomainParams& p, int cell, int rheo, const int32_t* pos,
                             double* vals, cudaStream_t s);

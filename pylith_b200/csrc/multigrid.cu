@@ -114,8 +114,8 @@ int mg_red_grid(int64_t n) {
 
 // The vector kernels of a cycle run between level operators q = J v that add into q, so each kernel
 // that reads q clears it for the next one, and the residual in + q (= in - A z) is formed where it is
-// used instead of in a pass of its own: nine launches per level and cycle, four of them operators
-// (18 with separate residuals, additions and clearing).
+// used instead of in a pass of its own: ten launches per level and cycle at the smoother degree 2, four of
+// them operators (18 with separate residuals, additions and clearing).
 
 // First Chebyshev step from a zero guess: d = D^{-1} rhs / theta. RES: rhs = in + q on free DOFs, 0
 // elsewhere, kept in t, and q is cleared; else rhs = in. out (may be NULL): out = d, or out += d.

@@ -5,7 +5,7 @@
 // libsrc/pylith/problems/GreensFns.cc:291-337, and one PyLith process per forward problem). A
 // serving loop on one GPU has many small problems at once, each too small to fill the device:
 // here every PCG iteration of every active problem runs in the same eight launches -- fault
-// unfold, the FP32 Q1 Jacobian action over all members' cells (k_hex8_jv32_ragged, hexgroup.cu),
+// unfold, the FP32 Q1 Jacobian action over all members' cells (k_hex8_jv32_ragged, hex8.cu),
 // fault fold, p.Ap, its per-member sum, the x/r/z update with its r.z and r.r, their per-member
 // sums, and the search-direction update -- with every dot product and step length kept per member
 // (each member runs exactly its own PCG). Members join and leave between iterations; the

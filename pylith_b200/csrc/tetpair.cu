@@ -8,14 +8,16 @@
 // values, 15 entries, five incidences for the pair, 60 % of the traffic, and the shared edges and
 // cross product are formed once. The host matches the cells of a block into pairs (98 % of them on
 // Delaunay and structured meshes); a cell left over takes a thread by itself.
-// Measured on B200 (L2 warm), residual or action against the one-cell-per-thread kernel k_tet_pad2:
-// 1,296,000 structured cells FP64 53.8 -> 43.3 us and FP32 45.8 -> 33.3 (45.4 and 34.9 with whole warps
-// planned for the banks, kPlanSteps); 54,737 Delaunay cells FP64 9.5 -> 8.9, FP32 9.9 -> 8.7; 3,072 cells
-// FP64 8.5 -> 6.8. What bounds it now: shared memory still, then HBM.
-// Block size: 240 cells in 128 items with 4 CTAs per SM (FP64, at most 128 registers) measured best
-// (two launches on 1,179,648 cells 80 us, 75 with the banks planned by halves, 70.5 with zero_output); 5 and 6 CTAs 80-92
-// (spills), 64, 96, 192 and 256 threads
-// 82-98, two lanes per node in the sums 89. FP32: 4, 5 and 6 CTAs 45.6, 40.1, 38.6 us.
+//
+// Bound: shared memory still (79 % of its pipe on 1,218,746 cells), then HBM. Measured on B200 against the
+// one-cell-per-thread kernel k_tet_pad2, residual or action, L2 warm: 1,296,000 structured cells FP64 53.8 ->
+// 42.3 us and FP32 45.8 -> 33.3; 54,737 Delaunay cells FP64 9.5 -> 8.9, FP32 9.9 -> 8.7; 3,072 cells FP64 8.5
+// -> 6.8. INSERT applications also start under their output's zeroing (zero_output).
+//
+// Sizes of a block: 240 cells in 128 items (threads), 4 CTAs per SM in FP64 (at most 128 registers), 6 in
+// FP32. Others, residual and action of 1,179,648 cells, 80 us this way before the banks were planned by
+// half-warps: 5 and 6 CTAs 80 to 92 (spills); 64, 96, 192 and 256 threads 82 to 98; two lanes per node in the
+// sums 89. FP32 with 4, 5 and 6 CTAs: 45.6, 40.1 and 38.6 us.
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
