@@ -289,7 +289,7 @@ PL_D void hex8_cell(const DomainParams& p, int64_t c, double* stage = nullptr) {
         if constexpr (F32) {
             // the moduli as multiples of a power of two, applied to the node sums: modulus / det would leave
             // FP32's range where a cell is smaller than about 1e-9 m with moduli in Pa
-            const unsigned e = min(max(__float_as_uint(lam + 2.0f * mu) >> 23 & 0xffu, 1u), 253u);
+            const unsigned e = min(max(__float_as_uint(fabsf(lam) + 2.0f * fabsf(mu)) >> 23 & 0xffu, 1u), 253u);
             const float to_one = __uint_as_float((254u - e) << 23);
             lam *= to_one, mu *= to_one;
             scale *= __uint_as_float(e << 23);
