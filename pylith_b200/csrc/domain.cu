@@ -196,6 +196,17 @@ __global__ void __launch_bounds__(128) k_domain_update_state(DomainParams p) {
         for (int k = 0; k < E::ngeom; ++k)
 #pragma unroll
             for (int i = 0; i < 3; ++i) X[k][i] = p.coords[3 * (int64_t)nodes[E::corner(k)] + i];
+        // Q1: coordinates and field relative to the first corner, as in hex8.cu (the basis gradients sum to
+        // zero), so that no large coordinates or displacements cancel
+        double u0[3] = {0, 0, 0};
+        if (CELL == HEX8) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                u0[i] = p.u[3 * (int64_t)nodes[0] + i];
+#pragma unroll
+                for (int k = E::ngeom - 1; k >= 0; --k) X[k][i] -= X[0][i];
+            }
+        }
         double a[L::size] = {};
         L::load_cell(p, c, a);
 #pragma unroll 1
@@ -207,11 +218,12 @@ __global__ void __launch_bounds__(128) k_domain_update_state(DomainParams p) {
                 double gr[3];
                 E::grad(g, q, n, gr);
                 const double* un = p.u + 3 * (int64_t)nodes[n];
+                const double u[3] = {un[0] - u0[0], un[1] - u0[1], un[2] - u0[2]};
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    s_x[0 + d] += un[0] * gr[d];
-                    s_x[3 + d] += un[1] * gr[d];
-                    s_x[6 + d] += un[2] * gr[d];
+                    s_x[0 + d] += u[0] * gr[d];
+                    s_x[3 + d] += u[1] * gr[d];
+                    s_x[6 + d] += u[2] * gr[d];
                 }
             }
             L::load_qp(p, c, q, E::nq, a);

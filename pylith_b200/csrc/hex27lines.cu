@@ -76,9 +76,10 @@ __global__ void __launch_bounds__(Lines::WARPS * 32) k_hex27_lines(DomainParams 
                 for (int cc = 0; cc < 3; ++cc) u[a][cc] = field[3 * (int64_t)nodes[a] + cc];
             }
             if (l < 8) {
-                const int cn = p.cells[mc * 27 + Elem<HEX27>::corner(l)];
+                // relative to the first corner (the basis gradients sum to zero): large coordinates do not cancel
+                const int cn = p.cells[mc * 27 + Elem<HEX27>::corner(l)], c0n = p.cells[mc * 27];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) sX[l * 3 + k] = p.coords[3 * (int64_t)cn + k];
+                for (int k = 0; k < 3; ++k) sX[l * 3 + k] = p.coords[3 * (int64_t)cn + k] - p.coords[3 * (int64_t)c0n + k];
             }
             // forward x: B u and D u along the line
 #pragma unroll

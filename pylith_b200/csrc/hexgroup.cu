@@ -128,13 +128,24 @@ PL_D void hex_group_cells(const DomainParams& p, int64_t base, const HexGroupSme
     T* sF = g.sF;
     T* sF0 = g.sF0;
     const int grp = g.grp, l = g.l;
-    const bool f32 = sizeof(T) == 4;
+    constexpr bool f32 = sizeof(T) == 4;
     {
         const int64_t c = base + grp;
         const bool live = c < p.ncells;
         const int64_t mc = live ? (p.cell_ids ? p.cell_ids[c] : c) : 0;
         int node = 0;
-        if (live && l < H::NEN) {
+        if (CELL == HEX8 && live) {
+            // field and coordinates relative to the first corner (the basis gradients sum to zero), so that no
+            // large coordinates or displacements cancel
+            static_assert(CELL != HEX8 || (!f32 && OP == OP_RESIDUAL), "the Q1 instantiation is the FP64 residual's");
+            node = p.cells[mc * 8 + l];
+            const int64_t first = p.cells[mc * 8];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                su[l * 3 + k] = p.u[3 * (int64_t)node + k] - p.u[3 * first + k];
+                sX[l * 3 + k] = p.coords[3 * (int64_t)node + k] - p.coords[3 * first + k];
+            }
+        } else if (live && l < H::NEN) {
             node = p.cells[mc * H::NEN + l];
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -142,7 +153,7 @@ PL_D void hex_group_cells(const DomainParams& p, int64_t base, const HexGroupSme
                 else su[l * 3 + k] = (T)(OP == OP_RESIDUAL ? p.u : p.v)[3 * (int64_t)node + k];
             }
         }
-        if (live && l < 8) {
+        if (CELL != HEX8 && live && l < 8) {
             const int cn = p.cells[mc * H::NEN + Elem<CELL>::corner(l)];
 #pragma unroll
             for (int k = 0; k < 3; ++k) sX[l * 3 + k] = p.coords[3 * (int64_t)cn + k];

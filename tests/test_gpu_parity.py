@@ -1132,3 +1132,38 @@ def test_derived_rows_of_q2(torch_cuda, ctx, per_sm, extra, num):
     # (differences of displacements of up to 20 m over cells of 400 m and more, u and x rounded: 1e-11)
     for i in range(num):
         assert rel_l2(got[:nc, 6 * i:6 * i + 6], strain if i % 2 else stress) <= 1e-10
+
+
+@pytest.mark.parametrize("kind,n", [("hex8", (7, 6, 5)), ("hex8", (46, 45, 43)), ("hex27", (4, 3, 3)), ("hex27", (19, 17, 13))])
+@pytest.mark.parametrize("genmaxwell", [False, True])
+def test_hexahedra_far_from_the_origin(torch_cuda, ctx, kind, n, genmaxwell):
+    """The hexahedral kernels on a box 2^26 m from the origin and, Q1, displaced by 2^20 m as a whole:
+    residual, action and Q1 state update agree with those of the box at the origin to 1e-12. (Cells of 256 m
+    and displacements of whole multiples of 2^-20: all differences are exact in both, so only the kernels'
+    own rounding is left; sums of absolute coordinates would lose 2^26 / 256 times 1e-16, of displacements
+    2^20 times.)"""
+    from pylith_b200 import feassemble as FA
+
+    torch = torch_cuda
+    got = []
+    for far in (False, True):
+        mesh = (M.box_hex if kind == "hex8" else M.box_hex27)(*n, (0.0, 0.0, 0.0), tuple(256.0 * k for k in n))
+        u = np.round(np.random.default_rng(97).standard_normal((mesh.num_nodes, 3)) * 2.0**20) / 2.0**20
+        if far:
+            mesh.coords += np.array([2.0**26, -2.0**25, 2.0**24])
+            u += np.array([2.0**20, -2.0**19, 2.0**18]) * (kind == "hex8")
+        mat = genmaxwell_setup(mesh, seed=98) if genmaxwell else elastic_setup(mesh, seed=98)
+        dm = FA.DeviceMesh(ctx, mesh)
+        ig = mat.create_integrator(dm, MAT.YEAR) if genmaxwell else mat.create_integrator(dm)
+        du = dev(torch, u.ravel())
+        r, jv = torch.empty_like(du), torch.empty_like(du)
+        ig.compute_lhs_residual(0.0, MAT.YEAR, du, r)
+        ig.compute_lhs_jacobian_action(0.0, MAT.YEAR, 0.0, None, du, jv)
+        fields = [r.cpu().numpy(), jv.cpu().numpy()]
+        if genmaxwell and kind == "hex8":
+            ig.update_state_vars(0.0, MAT.YEAR, du)
+            ctx.synchronize()
+            fields += [ig.get_aux("viscous_strain", (mesh.num_cells, 8, 18)), ig.get_aux("total_strain", (mesh.num_cells, 8, 6))]
+        got.append(fields)
+    for a, b in zip(*got):
+        assert rel_l2(b, a) <= TOL64
